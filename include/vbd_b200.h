@@ -290,7 +290,15 @@ int vbd_solver_status(vbd_solver* s, int64_t* singular_skips, int32_t* nonfinite
  *   VBD_OPT_PDL:         1 = launch colour sweeps with programmatic dependent launch, so a sweep
  *                        loads its element data while the previous sweep drains
  *   VBD_OPT_BLOCK:       threads per block of the sweep kernel: 64, 128 or 256
- *   VBD_OPT_PERSISTENT:  1 = run each step / solve as one cooperative launch that walks the colours
+ *   VBD_OPT_PERSISTENT:  0 = the captured graph of per-colour launches.  Until it is set, steps, solves
+ *                        and adjoint sweeps of meshes of at least 256 free vertices run as tile walks
+ *                        instead where these apply: one cooperative launch, the free vertices cut into
+ *                        one spatial tile per SM that exchanges its border with its neighbours through
+ *                        L2 after each colour (factored records, 4, 8 or 16 lanes for every colour,
+ *                        VBD_OPT_GRAPH on, no kernel timing, the handle's stream not capturing, the
+ *                        tile's vertices within shared memory).  Same results as the graph; reads
+ *                        back as 0; VBD_ERR_TIMEOUT from vbd_solver_sync if a bounded wait gave up;
+ *                        1 = run each step / solve as one cooperative launch that walks the colours
  *                        with a grid barrier after each one (bounded wait: a barrier that gives up
  *                        makes the next vbd_solver_sync return VBD_ERR_TIMEOUT);
  *                        2 = run each sub-step / solve as ONE thread-block cluster that keeps both

@@ -60,10 +60,17 @@ void build_vertex_tets(int32_t num_verts, int32_t num_tets, const int32_t* tets,
 // M_0 . cof(M)_0; layout 4 derives it as s.w / |q_n|^2 with s = M q_n, w = cof(M) q_n and |q_n|^2 =
 // -(s_0 + s_1 + s_2), which cancels when |q_n| is small next to the other rows (anisotropic or
 // sliver tets).  The FP32 steps follow k_pack_factored and decode_fact.
-void factored_detm_error(int32_t num_tets, const float* dm_inv, double* err3, double* err4, double* frac4) {
+namespace {
+
+struct DetmError {
     double e3 = 0.0, e4 = 0.0;
     long long counted = 0, over = 0;
-    for (int64_t t = 0; t < num_tets; ++t) {
+};
+
+DetmError detm_error_of(int64_t first, int64_t last, const float* dm_inv) {
+    double e3 = 0.0, e4 = 0.0;
+    long long counted = 0, over = 0;
+    for (int64_t t = first; t < last; ++t) {
         const float* d = dm_inv + 9 * t;
         float Q[4][3];
         for (int c = 0; c < 3; ++c) {
@@ -119,9 +126,25 @@ void factored_detm_error(int32_t num_tets, const float* dm_inv, double* err3, do
             if (!(r4 <= std::max(kFactoredDetmTol, kFactoredDetmRatio * r3))) ++over;
         }
     }
-    if (err3) *err3 = e3;
-    if (err4) *err4 = e4;
-    if (frac4) *frac4 = counted ? (double)over / (double)counted : 0.0;
+    return DetmError{e3, e4, counted, over};
+}
+
+}  // namespace
+
+void factored_detm_error(int32_t num_tets, const float* dm_inv, double* err3, double* err4, double* frac4) {
+    std::vector<DetmError> part(4 * kMaxWorkers);
+    each_range(num_tets, num_tets > 20000,
+               [&](int i, long long b, long long e) { part[i] = detm_error_of(b, e, dm_inv); });
+    DetmError sum;
+    for (const DetmError& d : part) {
+        sum.e3 = std::max(sum.e3, d.e3);
+        sum.e4 = std::max(sum.e4, d.e4);
+        sum.counted += d.counted;
+        sum.over += d.over;
+    }
+    if (err3) *err3 = sum.e3;
+    if (err4) *err4 = sum.e4;
+    if (frac4) *frac4 = sum.counted ? (double)sum.over / (double)sum.counted : 0.0;
 }
 
 }  // namespace vbd

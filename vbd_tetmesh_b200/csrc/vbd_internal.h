@@ -1,9 +1,14 @@
 // Internal helpers shared by the host and device translation units of libvbd_b200.
 #pragma once
 
+#include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <string>
+#include <system_error>
+#include <thread>
+#include <vector>
 
 namespace vbd {
 
@@ -34,6 +39,31 @@ constexpr double kFactoredDegenerate = 1e-3;
 // fraction of the incidences (systematic anisotropy); a few isolated thin tets do not move the
 // positions measurably (the 512-mesh batch: 4.08e-6 against 4.15e-6 of the diagonal from FP64).
 constexpr double kFactoredLossFraction = 1e-3;
+
+// fn(worker, item) for every item in [0, items), workers in [0, kMaxWorkers), over several host threads
+// when the work is large (a set-up loop of milliseconds).  Fewer threads where none can be made.
+constexpr int kMaxWorkers = 16;
+template <class Fn> void each_item(int items, bool large, Fn fn) {
+    const int workers =
+        large ? (int)std::max(1u, std::min((unsigned)kMaxWorkers, std::thread::hardware_concurrency())) : 1;
+    std::atomic<int> next{0};
+    auto run = [&](int w) {
+        for (int i; (i = next.fetch_add(1)) < items;) fn(w, i);
+    };
+    std::vector<std::thread> ts;
+    try {
+        for (int w = 1; w < workers && w < items; ++w) ts.emplace_back(run, w);
+    } catch (const std::system_error&) {
+    }
+    run(0);
+    for (auto& t : ts) t.join();
+}
+
+// The same over ranges [b, e) of n elements.
+template <class Fn> void each_range(long long n, bool large, Fn fn) {
+    const int parts = large ? 4 * kMaxWorkers : 1;
+    each_item(parts, large, [&](int, int i) { fn(i, n * i / parts, n * (i + 1) / parts); });
+}
 
 }  // namespace vbd
 

@@ -595,9 +595,10 @@ __device__ __forceinline__ void vertex_update(const SweepParams& p, int v, int l
 // The group's reduction and the first lane's block solve, Chebyshev blend and stores (the second
 // half of vertex_update).
 // The block solve of one vertex from its reduced sums (VBD.cpp:141-152, Types.h:85-112): returns
-// the new position, or xi where |det H| <= 1e-8 (counted in status); flags a non-finite result.
-__device__ __forceinline__ float4 block_solve(const Acc& acc, float4 xi, float4 yi, float dtsr,
-                                              unsigned long long* status) {
+// the new position, or xi where |det H| <= 1e-8 (counted in status); block_solve also flags a
+// non-finite result.
+__device__ __forceinline__ float4 block_update(const Acc& acc, float4 xi, float4 yi, float dtsr,
+                                               unsigned long long* status) {
     const float cm = yi.w * dtsr;
     const float H00 = cm + acc.h00, H01 = acc.h01, H02 = acc.h02;
     const float H11 = cm + acc.h11, H12 = acc.h12, H22 = cm + acc.h22;
@@ -621,7 +622,17 @@ __device__ __forceinline__ float4 block_solve(const Acc& acc, float4 xi, float4 
     } else {
         atomicAdd(status + ST_SINGULAR, 1ull);
     }
+    return xn;
+}
+
+__device__ __forceinline__ void flag_nonfinite(float4 xn, unsigned long long* status) {
     if (!(isfinite(xn.x) && isfinite(xn.y) && isfinite(xn.z))) status[ST_NONFINITE] = 1ull;
+}
+
+__device__ __forceinline__ float4 block_solve(const Acc& acc, float4 xi, float4 yi, float dtsr,
+                                              unsigned long long* status) {
+    const float4 xn = block_update(acc, xi, yi, dtsr, status);
+    flag_nonfinite(xn, status);
     return xn;
 }
 

@@ -12,6 +12,7 @@
 #include "vbd_internal.h"
 #include "vbd_cluster.cuh"
 #include "vbd_kernels.cuh"
+#include "vbd_tile.cuh"
 
 namespace vbd {
 
@@ -114,6 +115,15 @@ template <int L> static void (*pick_cluster(int layout, bool resident))(PersistP
 
 template <int L> static void (*pick_cluster_adjoint(int layout))(AdjWalkParams) {
     return layout == 3 ? &k_cluster_adjoint<L, 3> : &k_cluster_adjoint<L, 4>;
+}
+
+// The tile walk runs lanes / 2 threads per vertex; it reads its own record chunks, packed from the
+// factored records of either layout.
+template <bool ADJ, int W> static void (*pick_tile(int lanes))(TileParams) {
+    return lanes == 4 ? &k_tile_walk<2, ADJ, W> : lanes == 8 ? &k_tile_walk<4, ADJ, W> : &k_tile_walk<8, ADJ, W>;
+}
+template <bool ADJ> static void (*pick_tile(int lanes, int warps))(TileParams) {
+    return warps == 8 ? pick_tile<ADJ, 8>(lanes) : pick_tile<ADJ, 16>(lanes);
 }
 
 template <int L> static void (*pick_persistent(int layout))(PersistParams) {
@@ -256,6 +266,23 @@ struct vbd_solver {
     vbd::DBuf<float4> live_seg;
     vbd::DBuf<float> adj_gmu, adj_glam;
     int adj_cur = 0;  // which of adj_lam / adj_lam2 holds lam
+    // the tile walk (vbd_tile.cuh): its plan for the mesh, whether it runs in place of the captured
+    // graph (chosen at init or by the autotuner, off once VBD_OPT_PERSISTENT is set), and its device data
+    vbd::TilePlan tplan;
+    int tile_walk = 0;
+    bool persistent_set = false;
+    bool tile_dirty = true;     // chunks must be packed again (new records)
+    int tile_layout = 0;        // layout the chunks were packed from
+    int tile_lanes = 0;         // lanes the device data is for
+    std::vector<int32_t> batch_mesh;  // mesh of each vertex, set by vbd_solver_init_batch for its init
+    vbd::DBuf<float4> t_chunk, t_words;  // t_words: 4 N exchanged words, then the start counter
+    vbd::DBuf<int> t_lists;              // the plan's lists, one after the other (tile_list offsets)
+    enum { TL_HEAD, TL_GROUPS, TL_WCOL, TL_WSTREAM, TL_TABLE, TL_LID, TL_GHOST, TL_VTILE, TL_VLOCAL, TL_COUNT };
+    size_t tile_list[TL_COUNT + 1] = {};
+    const int* tile_ints(int which) const { return t_lists.p + tile_list[which]; }
+    unsigned long long t_started = 0;   // CTAs of all tile launches so far
+    unsigned t_tag = 1;                 // next unused word tag
+    int sm_count = 0, smem_optin = 0;
     long long launches = 0;
     std::vector<vbd::GraphEntry> graphs;
     std::vector<double> colour_bytes;               // algorithmic bytes of one sweep of colour c
@@ -671,7 +698,7 @@ struct vbd_solver {
 
     // Set-up of the adjoint walk outside any graph capture: the sweep schedule on the device and
     // the cluster shape.
-    int prepare_adj_walk(int sweeps, float rho, void (**fn_out)(vbd::AdjWalkParams)) {
+    int upload_adj_schedule(int sweeps, float rho) {
         std::vector<float> w(std::max(sweeps, 1), 1.0f);
         float omega = 1.0f;
         for (int it = 1; it <= sweeps; ++it) {
@@ -684,6 +711,11 @@ struct vbd_solver {
             CUDA_TRY(cudaStreamSynchronize(stream));
             adj_omega_cache = w;
         }
+        return VBD_OK;
+    }
+
+    int prepare_adj_walk(int sweeps, float rho, void (**fn_out)(vbd::AdjWalkParams)) {
+        VBD_TRY(upload_adj_schedule(sweeps, rho));
         if (d_cstart.n != cstart.size()) {
             VBD_TRY(d_cstart.alloc(cstart.size()));
             CUDA_TRY(cudaMemcpy(d_cstart.p, cstart.data(), sizeof(int) * cstart.size(), cudaMemcpyHostToDevice));
@@ -849,6 +881,176 @@ struct vbd_solver {
         return launch_persistent(iters, dtsr, accel, rho, predict, finish, from_inertia, h, hg);
     }
 
+    // Chunks per warp ring of a tile launch whose CTAs hold `vectors` local vectors.
+    int tile_ring(int warps, int vectors) const {
+        const long long fixed =
+            (long long)vbd::tile_smem(warps, 0, tplan.max_local, tplan.max_ids, tplan.max_groups, C, vectors) + 10240;
+        return (int)std::min<long long>(vbd::kTileMaxRing, (smem_optin - fixed) / (warps * vbd::kTileChunkBytes));
+    }
+    // The kernel of 8 warps needs room for two groups' chunks where it can be had, for one at least; that of
+    // 16 warps for two chunks.
+    bool tile_fits(int vectors) const {
+        return tile_ring(tplan.warps, vectors) >= (tplan.warps == 8 ? tplan.max_rounds : 2);
+    }
+    // Warps of the tile CTAs for the current lanes.
+    int tile_warps() const {
+        const double groups = (double)nfree / std::max(1, C) / std::max(1, tplan.P) * lanes / vbd::kTileChunk;
+        return groups <= vbd::kTileFewGroups && (max_valence + lanes - 1) / lanes <= vbd::kTileMaxRing / 2 ? 8 : 16;
+    }
+    // Whether steps and solves run as tile walks.  Under a caller's stream capture they do not: each
+    // launch needs tags of its own, which a replayed launch would repeat.
+    bool use_tile() {
+        if (!tile_walk || tplan.P == 0 || semantics || timing || !use_graph || persistent || !colour_lanes.empty() ||
+            layout < 3 || (lanes != 4 && lanes != 8 && lanes != 16) || ninc == 0)
+            return false;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (cs != cudaStreamCaptureStatusNone) return false;
+        if (tplan.lanes != lanes) vbd::tile_groups(&tplan, lanes, tile_warps(), h_inc_off.data());
+        return tile_fits(1);
+    }
+
+    // The plan's lane-dependent part and the record chunks, made when first needed for the current lanes,
+    // layout and materials.
+    int ensure_tile() {
+        if (tile_lanes != lanes) {
+            const struct {
+                const void* p;
+                size_t ints;
+            } lists[TL_COUNT] = {
+                {tplan.head.data(), tplan.head.size() * sizeof(vbd::TileHead) / 4},
+                {tplan.groups.data(), tplan.groups.size() * sizeof(vbd::TileGroup) / 4},
+                {tplan.wcol.data(), tplan.wcol.size()},
+                {tplan.wstream.data(), tplan.wstream.size()},
+                {tplan.chunk.data(), tplan.chunk.size()},
+                {tplan.lid.data(), tplan.lid.size()},
+                {tplan.ghost.data(), tplan.ghost.size()},
+                {tplan.vtile.data(), tplan.vtile.size()},
+                {tplan.vlocal.data(), tplan.vlocal.size()},
+            };
+            for (int k = 0; k < TL_COUNT; ++k) tile_list[k + 1] = tile_list[k] + (lists[k].ints + 3) / 4 * 4;
+            std::vector<int> all(tile_list[TL_COUNT]);
+            for (int k = 0; k < TL_COUNT; ++k)
+                if (lists[k].ints) std::memcpy(all.data() + tile_list[k], lists[k].p, 4 * lists[k].ints);
+            if (t_lists.n < all.size()) VBD_TRY(t_lists.alloc(all.size()));
+            CUDA_TRY(cudaMemcpyAsync(t_lists.p, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, stream));
+            if (t_words.n != 4 * (size_t)N + 1) {
+                VBD_TRY(t_words.alloc(4 * (size_t)N + 1));
+                CUDA_TRY(cudaMemsetAsync(t_words.p, 0, sizeof(float4) * t_words.n, stream));
+                t_started = 0;
+                t_tag = 1;
+            }
+            const size_t n4 = tplan.chunk.size() / 3 * (vbd::kTileChunkBytes / 16);
+            if (t_chunk.n != n4) VBD_TRY(t_chunk.alloc(n4));
+            CUDA_TRY(cudaStreamSynchronize(stream));  // the host lists may change after this
+            tile_dirty = true;
+            tile_lanes = lanes;
+        }
+        if (tile_dirty || tile_layout != layout) {
+            const int nch = (int)(tplan.chunk.size() / 3);
+            vbd::SweepParams p{};
+            p.inc_off = inc_off.p;
+            p.crec = crec.p;
+            p.cmat = cmat.p;
+            if (nch > 0) {
+                const unsigned grid = vbd::nblk((long long)nch * 32, 256);
+                auto fn = layout == 3 ? &vbd::k_pack_tile<3> : &vbd::k_pack_tile<4>;
+                fn<<<grid, 256, 0, stream>>>(p, tile_ints(TL_TABLE), nch, lanes,
+                                             reinterpret_cast<const vbd::TileGroup*>(tile_ints(TL_GROUPS)),
+                                             reinterpret_cast<const vbd::TileHead*>(tile_ints(TL_HEAD)), tile_ints(TL_LID),
+                                             tile_ints(TL_VTILE), tile_ints(TL_VLOCAL), nfree, t_chunk.p);
+                VBD_TRY(check_launch());
+            }
+            tile_dirty = false;
+            tile_layout = layout;
+        }
+        return VBD_OK;
+    }
+
+    vbd::TileParams tile_params(int k0, int k1, float dtsr, const float* omega, bool accel, int vectors) {
+        if ((unsigned long long)t_tag + (unsigned)(k1 - k0) > 0xfffffff0ull) {  // the tags start over
+            cudaMemsetAsync(t_words.p, 0, sizeof(float4) * 4 * (size_t)N, stream);
+            t_tag = 1;
+        }
+        vbd::TileParams w{};
+        w.chunk = t_chunk.p;
+        w.head = reinterpret_cast<const vbd::TileHead*>(tile_ints(TL_HEAD));
+        w.lid = tile_ints(TL_LID);
+        w.groups = reinterpret_cast<const vbd::TileGroup*>(tile_ints(TL_GROUPS));
+        w.wcol = tile_ints(TL_WCOL);
+        w.ghost = tile_ints(TL_GHOST);
+        w.wstream = reinterpret_cast<const int2*>(tile_ints(TL_WSTREAM));
+        w.words = t_words.p;
+        w.arrived = reinterpret_cast<unsigned long long*>(t_words.p + 4 * (size_t)N);
+        w.arrived_target = (t_started += (unsigned)tplan.P);
+        w.status = status.p;
+        w.omega = omega;
+        w.tag = t_tag - (unsigned)k0;
+        t_tag += (unsigned)(k1 - k0);
+        w.n = N;
+        w.nfree = nfree;
+        w.ncol = C;
+        w.k0 = k0;
+        w.k1 = k1;
+        w.ring = tile_ring(tplan.warps, vectors);
+        w.max_local = tplan.max_local;
+        w.max_ids = tplan.max_ids;
+        w.max_groups = tplan.max_groups;
+        w.max_rounds = tplan.max_rounds;
+        w.dtsr = dtsr;
+        w.keep_pp = accel ? 1 : 0;
+        w.y = y.p;
+        return w;
+    }
+
+    int tile_launch(void (*fn)(vbd::TileParams), vbd::TileParams& w, int vectors) {
+        const size_t smem = vbd::tile_smem(tplan.warps, w.ring, w.max_local, w.max_ids, w.max_groups, C, vectors);
+        CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+        void* args[] = {&w};
+        CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(tplan.P), dim3(32 * tplan.warps), args,
+                                             smem, stream));
+        return check_launch();
+    }
+
+    // A sub-step (hg given: predictor and velocity update) or a solve as tile walks: one launch, or one
+    // per energy evaluation with an energy history (emit_iterations' schedule).
+    int launch_tile(int iters, float dtsr, bool accel, float rho, bool from_inertia, float h, const float* hg,
+                    bool record_energy) {
+        VBD_TRY(upload_schedule(iters, accel, rho));
+        VBD_TRY(ensure_tile());
+        int k0 = 0;
+        do {
+            int k1 = iters;
+            if (record_energy) k1 = std::min(iters, k0 == 0 ? 1 : k0 + energy_every);
+            // both position buffers in shared memory where that leaves the rings their depth
+            const int two = accel && tile_ring(tplan.warps, 2) >= vbd::kTileTwoRing;
+            vbd::TileParams w = tile_params(k0, k1, dtsr, d_omega.p, accel, 1 + two);
+            w.two = two;
+            w.x0 = x0.p;
+            w.x1 = x1.p;
+            w.pp = pp.p;
+            w.v = v.p;
+            w.xprev = xprev.p;
+            w.predict = hg && k0 == 0;
+            w.finish = hg && k1 == iters;
+            w.from_inertia = from_inertia && k0 == 0;
+            w.h = h;
+            if (hg) {
+                w.hgx = hg[0];
+                w.hgy = hg[1];
+                w.hgz = hg[2];
+            }
+            VBD_TRY(tile_launch(vbd::pick_tile<false>(lanes, tplan.warps), w, 1 + two));
+            if (record_energy && k1 > k0 && (k1 - 1) % energy_every == 0) VBD_TRY(emit_energy_append(x0.p));
+            k0 = k1;
+        } while (k0 < iters);
+        return VBD_OK;
+    }
+
     int snapshot(vbd::DBuf<float4>& dst) {
         const size_t b4 = sizeof(float4) * (size_t)N;
         CUDA_TRY(cudaMemcpyAsync(dst.p, x0.p, b4, cudaMemcpyDeviceToDevice, stream));
@@ -887,6 +1089,7 @@ struct vbd_solver {
         key.rho = t.rho;
         if (persistent && !timing)
             return launch_walk(t.iters, t.dtsr, t.accel != 0, t.rho, true, true, false, t.h, t.hg);
+        if (use_tile()) return launch_tile(t.iters, t.dtsr, t.accel != 0, t.rho, false, t.h, t.hg, false);
         return run(key, [&] { return emit_substep(t.h, t.dtsr, t.hg, t.iters, t.accel != 0, t.rho); });
     }
 
@@ -895,7 +1098,7 @@ struct vbd_solver {
     // getAcceleratorOmega(k, rho) (rho = 0: plain Gauss-Seidel), then the parameter gradients, the
     // pinned-vertex coupling and the step's adjoint update.
     int emit_adjoint_substep(const TapeStep& t, const float4* X, int sweeps, float rho,
-                             void (*walk)(vbd::AdjWalkParams) = nullptr) {
+                             void (*walk)(vbd::AdjWalkParams) = nullptr, bool tile = false) {
         const float c = 0.999f / t.h;
         const int L = lanes < 4 ? 4 : lanes;
         vbd::k_adj_rhs<<<vbd::nblk(std::max(nfree, 1), 256), 256, 0, stream>>>(adj_ax.p, adj_av.p, adj_G.p, c, nfree);
@@ -911,7 +1114,20 @@ struct vbd_solver {
                 if (omega > 1.0f) cur ^= 1;
             }
         }
-        for (int it = 1; it <= sweeps && !walk; ++it) {
+        if (tile) {
+            vbd::TileParams w = tile_params(0, sweeps, t.dtsr, d_adj_omega.p, accel, 2);
+            w.X = X;
+            w.G = adj_G.p;
+            w.pp = adj_lpp.p;
+            w.lam_in = cur ? adj_lam2.p : adj_lam.p;
+            for (int it = 1; it <= sweeps && accel; ++it) {
+                omega = vbd::omega_of(it, rho, omega);
+                if (omega > 1.0f) cur ^= 1;
+            }
+            w.lam_out = cur ? adj_lam2.p : adj_lam.p;
+            VBD_TRY(tile_launch(vbd::pick_tile<true>(lanes, tplan.warps), w, 2));
+        }
+        for (int it = 1; it <= sweeps && !walk && !tile; ++it) {
             bool blend = false;
             if (accel) {
                 omega = vbd::omega_of(it, rho, omega);
@@ -993,7 +1209,13 @@ struct vbd_solver {
             key.walk = 2;
             key.block = ca_ctas;
         }
-        VBD_TRY(run(key, [&] { return emit_adjoint_substep(t, X, sweeps, rho, walk); }));
+        if (!walk && !adj_alternate && use_tile() && tile_fits(2)) {
+            VBD_TRY(upload_adj_schedule(sweeps, rho));
+            VBD_TRY(ensure_tile());
+            VBD_TRY(emit_adjoint_substep(t, X, sweeps, rho, nullptr, true));
+        } else {
+            VBD_TRY(run(key, [&] { return emit_adjoint_substep(t, X, sweeps, rho, walk); }));
+        }
         float omega = 1.0f;
         for (int it = 1; it <= sweeps && rho > 0.0f; ++it) {
             omega = vbd::omega_of(it, rho, omega);
@@ -1060,6 +1282,7 @@ struct vbd_solver {
     // Captured graphs bake in buffer addresses: every (re)allocation or release of the streamed
     // record copies invalidates them.
     int repack_stream() {
+        tile_dirty = true;
         if (layout != 1 && irec.p) {
             drop_graphs();
             irec.release();
@@ -1164,6 +1387,8 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
         CUDA_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
         s->own_stream = true;
     }
+    s->sm_count = prop.multiProcessorCount;
+    s->smem_optin = (int)prop.sharedMemPerBlockOptin;
     VBD_TRY(s->status.alloc(vbd::ST_SLOTS));
     CUDA_TRY(cudaMemset(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS));
     VBD_TRY(s->scalar.alloc(1));
@@ -1232,15 +1457,59 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     s->crec.release();
     s->cmat.release();
 
-    // Internal order: free vertices colour by colour (group order), then the pinned ones.
+    // Incident tets of each vertex, ascending tet id (TetMesh::vertAdjacentTets).
+    std::vector<int32_t> voff(N + 1), vtets(4LL * T);
+    vbd::build_vertex_tets(N, T, tets, voff.data(), vtets.data());
+
+    // Tiles of the tile walk.
+    vbd::TilePlan plan;
+    std::vector<int32_t> tile;
+    std::vector<uint8_t> boundary;
+    {
+        int free_count = 0;
+        for (int i = 0; i < N; ++i) free_count += fixed[i] ? 0 : 1;
+        if (free_count >= vbd::kTileMinVertices && T > 0) {
+            plan.P = std::min(s->sm_count, free_count / vbd::kTileVertices);
+            plan.n = N;
+            plan.nfree = free_count;
+            const int32_t* mesh = (int)s->batch_mesh.size() == N ? s->batch_mesh.data() : nullptr;
+            vbd::tile_partition(N, positions, fixed, mesh, plan.P, &tile);
+            vbd::tile_boundary(N, T, tets, tile, &boundary);
+        }
+    }
+
+    // Internal order: free vertices colour by colour, then the pinned ones.  Inside a colour: group
+    // order, or with tiles tile by tile, in a tile the vertices other tiles read first, then by falling
+    // valence (the vertices a warp of the tile walk sweeps together then have about as many tets).
     std::vector<int32_t> perm;
     perm.reserve(N);
     std::vector<int> cstart(num_colours + 1, 0);
+    std::vector<std::pair<unsigned long long, int32_t>> order, keys;
+    std::vector<std::pair<int, int>> sorted_at;
     for (int c = 0; c < num_colours; ++c) {
         cstart[c] = (int)perm.size();
-        for (int k = group_offsets[c]; k < group_offsets[c + 1]; ++k)
-            if (!fixed[group_vertices[k]]) perm.push_back(group_vertices[k]);
+        if (!plan.P) {
+            for (int k = group_offsets[c]; k < group_offsets[c + 1]; ++k)
+                if (!fixed[group_vertices[k]]) perm.push_back(group_vertices[k]);
+            continue;
+        }
+        order.clear();
+        for (int k = group_offsets[c]; k < group_offsets[c + 1]; ++k) {
+            const int32_t i = group_vertices[k];
+            if (fixed[i]) continue;
+            const unsigned long long val = (unsigned)std::min(voff[i + 1] - voff[i], 0xffff);
+            order.emplace_back(((unsigned long long)tile[i] << 17) | ((boundary[i] ? 0ull : 1ull) << 16) | (0xffffull - val), i);
+        }
+        for (const auto& o : order) perm.push_back(o.second);
+        sorted_at.emplace_back(cstart[c], (int)perm.size());
+        keys.insert(keys.end(), order.begin(), order.end());
     }
+    if (plan.P)  // each colour in its own order
+        vbd::each_item((int)sorted_at.size(), N > 4000, [&](int, int c) {
+            const auto r = sorted_at[c];
+            std::sort(keys.begin() + r.first, keys.begin() + r.second);
+            for (int i = r.first; i < r.second; ++i) perm[i] = keys[i].second;
+        });
     cstart[num_colours] = (int)perm.size();
     const int nfree = (int)perm.size();
     for (int i = 0; i < N; ++i)
@@ -1248,9 +1517,6 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     std::vector<int32_t> iperm(N);
     for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
 
-    // Incident tets of each free vertex, ascending tet id (TetMesh::vertAdjacentTets).
-    std::vector<int32_t> voff(N + 1), vtets(4LL * T);
-    vbd::build_vertex_tets(N, T, tets, voff.data(), vtets.data());
     // Incident tets of every vertex (free ones first, so the sweeps' incidences are [0, ninc); the
     // pinned vertices' lists serve the adjoint's coupling term).
     std::vector<int32_t> inc_off(N + 1, 0);
@@ -1258,21 +1524,41 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     const long long ninc = inc_off[nfree];
     const long long ninc_all = inc_off[N];
     std::vector<int32_t> inc_tet(std::max<long long>(ninc_all, 1)), inc_vertex(std::max<long long>(ninc_all, 1));
-    for (int i = 0; i < N; ++i) {
-        std::copy(vtets.begin() + voff[perm[i]], vtets.begin() + voff[perm[i] + 1], inc_tet.begin() + inc_off[i]);
-        std::fill(inc_vertex.begin() + inc_off[i], inc_vertex.begin() + inc_off[i + 1], i);
-    }
+    const bool large = N > 4000;
+    vbd::each_range(N, large, [&](int, long long b, long long e) {
+        for (long long i = b; i < e; ++i) {
+            std::copy(vtets.begin() + voff[perm[i]], vtets.begin() + voff[perm[i] + 1], inc_tet.begin() + inc_off[i]);
+            std::fill(inc_vertex.begin() + inc_off[i], inc_vertex.begin() + inc_off[i + 1], (int32_t)i);
+        }
+    });
 
     std::vector<vbd::TetRec> rec(std::max(T, 1));
-    for (int t = 0; t < T; ++t) {
-        const int32_t* q = tets + 4LL * t;
-        const float* d = dm_inv + 9LL * t;
-        vbd::TetRec& r = rec[t];
-        r.ids = make_int4(iperm[q[0]], iperm[q[1]], iperm[q[2]], iperm[q[3]]);
-        r.a = make_float4(d[0], d[1], d[2], d[3]);
-        r.b = make_float4(d[4], d[5], d[6], d[7]);
-        r.c = make_float4(d[8], rest_vol[t], tet_mu ? tet_mu[t] : 0.0f, tet_lambda ? tet_lambda[t] : 0.0f);
+    vbd::each_range(T, large, [&](int, long long b, long long e) {
+        for (long long t = b; t < e; ++t) {
+            const int32_t* q = tets + 4LL * t;
+            const float* d = dm_inv + 9LL * t;
+            vbd::TetRec& r = rec[t];
+            r.ids = make_int4(iperm[q[0]], iperm[q[1]], iperm[q[2]], iperm[q[3]]);
+            r.a = make_float4(d[0], d[1], d[2], d[3]);
+            r.b = make_float4(d[4], d[5], d[6], d[7]);
+            r.c = make_float4(d[8], rest_vol[t], tet_mu ? tet_mu[t] : 0.0f, tet_lambda ? tet_lambda[t] : 0.0f);
+        }
+    });
+
+    if (plan.P) {
+        std::vector<int32_t> tile_in(N, -1);
+        std::vector<uint8_t> bnd_in(N, 0);
+        for (int i = 0; i < nfree; ++i) {
+            tile_in[i] = tile[perm[i]];
+            bnd_in[i] = boundary[perm[i]];
+        }
+        vbd::tile_lists(&plan, cstart, tile_in, bnd_in, inc_off.data(), inc_tet.data(), &rec[0].ids.x,
+                        (int)(sizeof(vbd::TetRec) / sizeof(int)));
     }
+    s->tplan = std::move(plan);
+    s->t_words.release();
+    s->tile_lanes = 0;
+    s->tile_walk = !s->persistent_set && s->tplan.P > 0 && s->tplan.max_local <= vbd::kTileMaxLocal;
 
     std::vector<float4> hx(N), hv(N), hy(N);
     for (int i = 0; i < N; ++i) {
@@ -1362,6 +1648,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     s->d_cstart.release();
     s->have_materials = tet_mu != nullptr;
     VBD_TRY(s->repack_stream());
+    if (s->use_tile()) VBD_TRY(s->ensure_tile());
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     s->ready = true;
     return VBD_OK;
@@ -1399,8 +1686,12 @@ int vbd_solver_init_batch(vbd_solver* s, int32_t M, const int32_t* voff, const i
     VBD_TRY(vbd_color_vertices(N, T, tets.data(), colour_of.data(), &nc, 0, nullptr, nullptr));
     std::vector<int32_t> offs(nc + 1), verts(N);
     VBD_TRY(vbd_color_vertices(N, T, tets.data(), colour_of.data(), &nc, nc, offs.data(), verts.data()));
-    return vbd_solver_init(s, N, T, positions, velocities, nullptr, vertex_mass, fixed, tets.data(), nc, offs.data(),
-                           verts.data(), dm_inv, rest_vol, tet_mu, tet_lambda);
+    s->batch_mesh.resize(N);
+    for (int m = 0; m < M; ++m) std::fill(s->batch_mesh.begin() + voff[m], s->batch_mesh.begin() + voff[m + 1], m);
+    const int rc = vbd_solver_init(s, N, T, positions, velocities, nullptr, vertex_mass, fixed, tets.data(), nc, offs.data(),
+                                   verts.data(), dm_inv, rest_vol, tet_mu, tet_lambda);
+    s->batch_mesh.clear();
+    return rc;
 }
 
 int vbd_solver_set_materials(vbd_solver* s, const float* tet_mu, const float* tet_lambda) {
@@ -1519,6 +1810,9 @@ int vbd_solver_solve(vbd_solver* s, int32_t iterations, float dt_sqr_reciprocal,
     if (s->persistent && !s->timing)
         return s->launch_walk(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, false, false,
                               init_mode == VBD_INIT_FROM_INERTIA, 1.0f, nullptr);
+    if (s->use_tile())
+        return s->launch_tile(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode == VBD_INIT_FROM_INERTIA,
+                              1.0f, nullptr, false);
     return s->run(key, [&] { return s->emit_solve(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode); });
 }
 
@@ -1565,6 +1859,8 @@ int vbd_solver_step(vbd_solver* s, float dt, int32_t substeps, int32_t iteration
         // separate launches
         if (s->persistent && !s->timing && nenergy == 0)
             VBD_TRY(s->launch_walk(iterations, dtsr, use_acceleration != 0, rho, true, true, false, h, hg));
+        else if (s->use_tile())
+            VBD_TRY(s->launch_tile(iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0));
         else
             VBD_TRY(s->run(key, [&] {
                 return s->emit_substep(h, dtsr, hg, iterations, use_acceleration != 0, rho, nenergy > 0);
@@ -1718,7 +2014,7 @@ int vbd_solver_sync(vbd_solver* s) {
         if (t[0] || t[1]) {
             CUDA_TRY(cudaMemset(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t)));
             if (t[0]) VBD_FAIL(VBD_ERR_TIMEOUT, "a grid barrier of the persistent kernel gave up waiting");
-            VBD_FAIL(VBD_ERR_TIMEOUT, "an mbarrier wait of the cluster walk gave up");
+            VBD_FAIL(VBD_ERR_TIMEOUT, "a wait of the cluster or tile walk gave up");
         }
     }
     return VBD_OK;
@@ -1839,6 +2135,8 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
                 if (!s->cluster_fit(&why)) VBD_FAIL(VBD_ERR_INVALID_ARG, "%s", why);
             }
             s->persistent = value;
+            s->persistent_set = true;
+            s->tile_walk = 0;
             return VBD_OK;
         case VBD_OPT_CLUSTER_CTAS:
             if (value < 0 || value > 16) VBD_FAIL(VBD_ERR_INVALID_ARG, "cluster CTAs must be 0 (automatic) to 16");
@@ -1992,6 +2290,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
         int lanes, layout, prefetch, pdl, block, persistent, cache, persist;
         std::vector<int> colour_lanes;  // empty = `lanes` for every colour
         int ctas = 0;                   // CTAs of the cluster walk (0 = automatic)
+        int tile = 0;                   // the tile walk instead of the captured graph
     };
     const float g[3] = {0.f, 0.f, 0.f};
     cudaEvent_t e0, e1;
@@ -2007,6 +2306,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
         s->persist_mb = c.persist;
         s->colour_lanes = c.colour_lanes;
         s->cluster_ctas_opt = c.ctas;
+        s->tile_walk = c.tile;
         if (s->layout != c.layout) {
             s->layout = c.layout;
             return s->repack_stream();
@@ -2038,7 +2338,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
         {8, 0, 1, 1, 128}, {4, 0, 1, 1, 128},
     };
     Cand best{s->lanes,      s->layout,       s->eff_prefetch(), s->pdl,          s->block,
-              s->persistent, s->record_cache, s->persist_mb,     s->colour_lanes, s->cluster_ctas_opt};
+              s->persistent, s->record_cache, s->persist_mb,     s->colour_lanes, s->cluster_ctas_opt, s->tile_walk};
     float best_ms = 1e30f;
     const int init_persist = s->persist_mb;  // the init-time record policy, for the factored candidates
     s->prefetch_auto = false;
@@ -2135,6 +2435,17 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
         c.persistent = 1;
         c.colour_lanes.clear();
         rc = try_cand(c);
+        // the tile walk at each lane count it runs
+        if (s->tplan.P > 0 && base.layout >= 3)
+            for (int L : {4, 8, 16}) {
+                if (rc) break;
+                Cand k = base;
+                k.persistent = 0;
+                k.lanes = L;
+                k.colour_lanes.clear();
+                k.tile = 1;
+                rc = try_cand(k);
+            }
         // the cluster walk, for a mesh whose positions fit in one CTA's shared memory: each lane count
         // with either factored layout (the stored det M of layout 3 saves a division per record,
         // which counts where the records stay in L2)
@@ -2145,6 +2456,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
                 for (int L : {4, 8, 16, 32}) {
                     Cand k = base;
                     k.persistent = 2;
+                    k.tile = 0;
                     k.lanes = L;
                     k.layout = lay;
                     k.colour_lanes.clear();

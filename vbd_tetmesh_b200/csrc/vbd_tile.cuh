@@ -1,0 +1,765 @@
+// The tile walk: all iterations of a sub-step (or of its adjoint solve) in ONE cooperative launch, for
+// meshes too large for one cluster's shared memory.
+//
+// Per-colour launches pay a kernel boundary per colour (2.3 us and up) and start each colour's
+// record stream only then.  Here the free vertices are cut into one spatial tile per CTA (one CTA per
+// SM; vbd_tile_plan.cpp) and the colours are separated by data instead of by launches:
+//   * a tile keeps the positions of its own vertices and of the neighbours it reads (its ghosts) in
+//     shared memory, so every neighbour gather is a shared-memory load;
+//   * a vertex that other tiles read is published as ONE 16-byte word, {x~, tag}, with a relaxed
+//     128-bit store (single-copy atomic); after sweeping colour c a tile polls the words of its
+//     colour-c ghosts until they carry the iteration's tag.  Data and flag travel together, so there
+//     are no fences, no flags and no grid barrier: a tile waits for its neighbours only.  One
+//     __syncthreads per colour separates the colours inside the tile;
+//   * the element records are re-ordered into the exact order each warp reads them (chunks of 64
+//     incidences, two per thread, field by field), and each warp streams its own chunks through a
+//     private shared-memory ring with asynchronous copies.  Records never change during the
+//     sweeps, so the ring runs ahead across colours and iterations: the stream does not stop while
+//     a tile waits for its neighbours.
+// Why overwriting a published word is safe: words alternate by tag parity, and the owner of v can be
+// two iterations ahead of a reader of v only if it has received, from that reader, a value computed
+// after the reader took v's word (every reader of v owns a free neighbour of v, and v's own sweep
+// gathers that neighbour).
+//
+// What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
+// one SM to another's poll, 885 on average) plus one vertex's chain per colour: 1.6 to 2 us a colour
+// against 2.3 to 2.6 us a launch.  Large tiles by issue and the chunk stream: 64^3 cube 3.4 against 4.1 ms
+// a step of 400 colours, 4.0 TB/s of DRAM reads.
+// Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
+// records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds
+// the sums of lanes t and t + L/2 (group_reduce's first addition), so a vertex takes L/2 threads:
+// half the warps' shuffles and idle solve lanes of the per-colour kernel.
+#pragma once
+
+#include "vbd_cluster.cuh"
+#include "vbd_tile_plan.h"
+
+namespace vbd {
+
+struct TileParams {
+    const float4* chunk;        // record chunks, kTileChunkBytes each
+    const TileHead* head;
+    const int* lid;
+    const TileGroup* groups;
+    const int* wcol;            // [P][warps][C + 1]: first group of each warp and colour
+    const int* ghost;           // [P][C + 1]
+    const int2* wstream;        // [P][warps]
+    float4* words;              // exchanged words: [parity][n] x~, then [parity][n] blended
+    unsigned long long* arrived;
+    unsigned long long arrived_target;  // *arrived once every CTA of this launch has started
+    unsigned long long* status;
+    const float* omega;         // Chebyshev weight of each iteration (1 = no blend)
+    unsigned tag;               // iteration k publishes tag + k; unused by any earlier launch
+    int n, nfree, ncol, k0, k1; // iterations [k0, k1) of the schedule
+    int ring, max_local, max_ids, max_groups, max_rounds;
+    int two;                    // both position buffers in shared memory
+    float dtsr;
+    int keep_pp;
+    // forward: positions start and end in x0
+    float4* x0;
+    float4* x1;
+    float4* pp;
+    float4* y;
+    float4* v;
+    float4* xprev;
+    int predict, finish, from_inertia;
+    float h, hgx, hgy, hgz;
+    // adjoint: converged positions X, right-hand side G, adjoint in / out, pre-sweep adjoint in pp
+    const float4* X;
+    const float4* G;
+    const float4* lam_in;
+    float4* lam_out;
+};
+
+// Dynamic shared memory of a CTA: the rings, the local vectors (`vectors` of them, one entry more each),
+// the groups, the internal ids of the own vertices and ghosts, the first ghost of each colour, and the
+// first group of each warp and colour.
+__host__ __device__ inline size_t tile_smem(int warps, int ring, int max_local, int max_ids, int max_groups, int ncol,
+                                            int vectors) {
+    return (size_t)warps * ring * kTileChunkBytes + 16u * (size_t)(max_local + 1) * vectors +
+           sizeof(TileGroup) * (size_t)max_groups + 4u * (size_t)max_ids + 4u * (size_t)(warps + 1) * (ncol + 1);
+}
+
+// The 128-bit words: one relaxed, single-copy-atomic access each.
+__device__ __forceinline__ void word_store(float4* p, float x, float y, float z, unsigned tag) {
+    const unsigned long long a = ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(x);
+    const unsigned long long b = ((unsigned long long)tag << 32) | __float_as_uint(z);
+    asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(a),
+                 "l"(b)
+                 : "memory");
+}
+__device__ __forceinline__ float4 word_load(const float4* p) {
+    unsigned long long a, b;
+    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+                 : "=l"(a), "=l"(b)
+                 : "l"(p)
+                 : "memory");
+    return make_float4(__uint_as_float((unsigned)a), __uint_as_float((unsigned)(a >> 32)), __uint_as_float((unsigned)b),
+                       __uint_as_float((unsigned)(b >> 32)));
+}
+
+// Gives up a wait: another wait already gave up, or this one has lasted kTileWaitNs with every CTA of
+// the launch running (a CTA that cannot start while another program's kernel holds its SM is
+// waited for up to kTileStartNs).
+constexpr unsigned long long kTileWaitNs = 2000000000ull;
+constexpr unsigned long long kTileStartNs = 60000000000ull;
+struct TileClock {
+    unsigned long long first = 0, last = 0;
+};
+__device__ __noinline__ bool tile_give_up(unsigned long long* status, unsigned long long* arrived,
+                                          unsigned long long target, TileClock& c) {
+    if (*reinterpret_cast<volatile unsigned long long*>(status + ST_WALK_TIMEOUT) != 0ull) return true;
+    const unsigned long long now = global_ns();
+    if (c.first == 0) c.first = c.last = now;
+    if (now - c.last <= kTileWaitNs) return false;
+    if (*reinterpret_cast<volatile unsigned long long*>(arrived) < target && now - c.first <= kTileStartNs) {
+        c.last = now;
+        return false;
+    }
+    atomicOr(reinterpret_cast<unsigned int*>(status + ST_WALK_TIMEOUT), 1u);
+    return true;
+}
+
+// Waits for word w to carry `tag` and stores its vector to *dst.
+__device__ __forceinline__ bool tile_spin(const TileParams& p, const float4* w, unsigned tag, float4* dst) {
+    TileClock clk;
+    for (unsigned i = 1;; ++i) {
+        const float4 v = word_load(w);
+        if (__float_as_uint(v.w) == tag) {
+            *dst = make_float4(v.x, v.y, v.z, 0.f);
+            return true;
+        }
+        if ((i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, clk)) return false;
+    }
+}
+// The same with a first look already taken.
+__device__ __forceinline__ bool tile_take(const TileParams& p, float4 v, const float4* w, unsigned tag, float4* dst) {
+    if (__float_as_uint(v.w) != tag) return tile_spin(p, w, tag, dst);
+    *dst = make_float4(v.x, v.y, v.z, 0.f);
+    return true;
+}
+
+// A warp's ring of record chunks.  W = 8 fills it by its own lanes with 16-byte asynchronous copies, one
+// commit group per chunk (empty ones once the walk's chunks are all under way).
+struct TileRing {
+    int first, end, next;  // the warp's chunks [first, end), read cyclically; next one to copy
+    int left;              // chunks still to copy
+    int slot;              // slot of the next chunk to sweep
+};
+
+__device__ __forceinline__ void ring_issue(const TileParams& p, TileRing& r, unsigned buf, int slot, int lane) {
+    if (r.left > 0) {
+        const char* src = reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kTileChunkBytes + 16 * lane;
+        const unsigned dst = buf + (unsigned)(slot * kTileChunkBytes + 16 * lane);
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512 * i), "l"(src + 512 * i) : "memory");
+        if (lane < 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 2560), "l"(src + 2560) : "memory");
+        --r.left;
+        if (++r.next == r.end) r.next = r.first;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// The same as one bulk copy, completing on the slot's mbarrier (W = 16).
+__device__ __forceinline__ void ring_issue_bulk(const TileParams& p, TileRing& r, unsigned buf, unsigned bar, int slot,
+                                                int lane) {
+    if (r.left <= 0) return;
+    if (lane == 0) {
+        mbar_expect(bar + 8u * slot, kTileChunkBytes);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         buf + (unsigned)(slot * kTileChunkBytes)),
+                     "l"(reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kTileChunkBytes),
+                     "r"((unsigned)kTileChunkBytes), "r"(bar + 8u * slot)
+                     : "memory");
+    }
+    --r.left;
+    if (++r.next == r.end) r.next = r.first;
+}
+__device__ __forceinline__ bool ring_try(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool ring_wait_bulk(const TileParams& p, unsigned bar, unsigned parity) {
+    bool done = ring_try(bar, parity);
+    if (!done) {
+        TileClock clk;
+        for (unsigned i = 1; !done; ++i) {
+            done = ring_try(bar, parity);
+            if (!done && (i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, clk)) break;
+        }
+    }
+    return __all_sync(0xffffffffu, done);
+}
+static_assert(kTileChunkBytes == 5 * 512 + 256, "ring_issue copies 176 pieces of 16 bytes");
+
+// Waits until at most `pending` of the newest commit groups are outstanding.
+template <int N> __device__ __forceinline__ void ring_wait_for() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void ring_wait(int pending) {
+    switch (pending) {
+        case 0: ring_wait_for<0>(); break;
+        case 1: ring_wait_for<1>(); break;
+        case 2: ring_wait_for<2>(); break;
+        case 3: ring_wait_for<3>(); break;
+        default: ring_wait_for<4>(); break;
+    }
+    __syncwarp();
+}
+
+// Two FP32 values in one 64-bit register pair, for the two-wide FP32 instructions (each half rounds as
+// the scalar instruction does).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(F2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float f2_hi(F2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 neg2(F2 a) { return mul2(a, f2(-1.f, -1.f)); }
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.f, -1.f), a); }
+// a0 b0 + a1 b1 + a2 b2, rounded as nvcc contracts that expression.
+__device__ __forceinline__ F2 dot2(F2 a0, F2 b0, F2 a1, F2 b1, F2 a2, F2 b2) {
+    return fma2(a2, b2, fma2(a0, b0, mul2(a1, b1)));
+}
+// a b - c d given nc = -c, rounded as nvcc contracts it.
+__device__ __forceinline__ F2 cross2(F2 a, F2 b, F2 nc, F2 d) { return fma2(a, b, mul2(nc, d)); }
+
+__device__ __forceinline__ void load_if(bool pred, const float4* p, float4& v) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+                 : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+                 : "l"(p), "r"((int)pred)
+                 : "memory");
+}
+__device__ __forceinline__ void load_if(bool pred, const float* p, float& v) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.global.f32 %0, [%1];\n}"
+                 : "+f"(v)
+                 : "l"(p), "r"((int)pred)
+                 : "memory");
+}
+
+// One thread's two records of a chunk: lanes t (first half of each pair) and t + L/2 of its vertex.  The
+// fields are read where they are used (they would hold 18 registers).
+struct TilePair {
+    const char* buf;
+    int lane;
+    __device__ __forceinline__ ulonglong2 two(int k) const { return reinterpret_cast<const ulonglong2*>(buf)[32 * k + lane]; }
+    __device__ __forceinline__ ulonglong2 s01() const { return two(0); }
+    __device__ __forceinline__ ulonglong2 s2w0() const { return two(1); }
+    __device__ __forceinline__ ulonglong2 w12() const { return two(2); }
+    __device__ __forceinline__ ulonglong2 ab() const { return two(3); }
+    // neighbours: {nb0 | nb1 << 16, nb2 | valid << 16} of the first record, then of the second
+    __device__ __forceinline__ int4 ids() const { return reinterpret_cast<const int4*>(buf)[128 + lane]; }
+    __device__ __forceinline__ F2 detm() const { return reinterpret_cast<const F2*>(buf + 160 * 16)[lane]; }
+};
+
+// Sums of two lanes of one vertex.
+struct Acc2 {
+    F2 h00, h01, h02, h11, h12, h22, g0, g1, g2;
+    __device__ __forceinline__ void zero() { h00 = h01 = h02 = h11 = h12 = h22 = g0 = g1 = g2 = 0ull; }
+    __device__ __forceinline__ Acc sum() const {
+        Acc r;
+        r.h00 = f2_lo(h00) + f2_hi(h00);
+        r.h01 = f2_lo(h01) + f2_hi(h01);
+        r.h02 = f2_lo(h02) + f2_hi(h02);
+        r.h11 = f2_lo(h11) + f2_hi(h11);
+        r.h12 = f2_lo(h12) + f2_hi(h12);
+        r.h22 = f2_lo(h22) + f2_hi(h22);
+        r.g0 = f2_lo(g0) + f2_hi(g0);
+        r.g1 = f2_lo(g1) + f2_hi(g1);
+        r.g2 = f2_lo(g2) + f2_hi(g2);
+        return r;
+    }
+};
+
+// The geometry of two records: edge vectors d_k and the columns c_k of cof(D) (c_0 = d_1 x d_2, ...).  A
+// product a b - c d needs one negated factor; those of d_1 and d_2 serve all three columns.
+struct Geom2 {
+    F2 d[3][3], c[3][3], n1[3], n2[3];
+};
+__device__ __forceinline__ void tile_edges(const int4 id, float4 xi, const float4* X, Geom2& q) {
+    const unsigned a0 = id.x, a1 = id.y, b0 = id.z, b1 = id.w;
+    const float4 pa[3] = {X[a0 & 0xffffu], X[a0 >> 16], X[a1 & 0xffffu]};
+    const float4 pb[3] = {X[b0 & 0xffffu], X[b0 >> 16], X[b1 & 0xffffu]};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        q.d[k][0] = f2(pa[k].x - xi.x, pb[k].x - xi.x);
+        q.d[k][1] = f2(pa[k].y - xi.y, pb[k].y - xi.y);
+        q.d[k][2] = f2(pa[k].z - xi.z, pb[k].z - xi.z);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        q.n1[i] = neg2(q.d[1][i]);
+        q.n2[i] = neg2(q.d[2][i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+        q.c[0][i] = cross2(q.d[1][i1], q.d[2][i2], q.n1[i2], q.d[2][i1]);
+        q.c[1][i] = cross2(q.d[2][i1], q.d[0][i2], q.n2[i2], q.d[0][i1]);
+        q.c[2][i] = cross2(q.d[0][i1], q.d[1][i2], q.d[0][i2], q.n1[i1]);
+    }
+}
+
+// fact_contrib for two records at once, operation for operation as nvcc contracts it, so that each
+// half has fact_contrib's bits.  A record that is only padding has zero fields and the vertex itself
+// as its neighbours: d = 0, and it adds zero to every sum.
+__device__ __forceinline__ void tile_contrib(const TilePair& r, const int4 id, float4 xi, const float4* X, Acc2& acc) {
+    Geom2 q;
+    tile_edges(id, xi, X, q);
+    const ulonglong2 ab = r.ab();
+    const F2 bj = mul2(ab.y, fma2(dot2(q.d[0][0], q.c[0][0], q.d[0][1], q.c[0][1], q.d[0][2], q.c[0][2]), r.detm(),
+                                  f2(-1.f, -1.f)));
+    const ulonglong2 sw = r.s2w0(), w12 = r.w12(), s01 = r.s01();
+    F2 C[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        C[i] = dot2(q.c[0][i], sw.y, q.c[1][i], w12.x, q.c[2][i], w12.y);
+        const F2 Fq = dot2(q.d[0][i], s01.x, q.d[1][i], s01.y, q.d[2][i], sw.x);
+        F2& g = i == 0 ? acc.g0 : i == 1 ? acc.g1 : acc.g2;
+        g = add2(g, fma2(ab.x, sub2(Fq, C[i]), mul2(bj, C[i])));
+    }
+    const F2 am = mul2(ab.x, neg2(add2(add2(s01.x, s01.y), sw.x)));
+    const F2 b0 = mul2(ab.y, C[0]), b1 = mul2(ab.y, C[1]), b2 = mul2(ab.y, C[2]);
+    acc.h00 = add2(acc.h00, fma2(b0, C[0], am));
+    acc.h01 = fma2(b0, C[1], acc.h01);
+    acc.h02 = fma2(b0, C[2], acc.h02);
+    acc.h11 = add2(acc.h11, fma2(b1, C[1], am));
+    acc.h12 = fma2(b1, C[2], acc.h12);
+    acc.h22 = add2(acc.h22, fma2(b2, C[2], am));
+}
+
+// fact_adjoint for two records at once.  A padding record reads the zero entry `zero` of L.
+__device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, float4 xi, const float4* X,
+                                             const float4* L, int zero, Acc2& acc) {
+    Geom2 q;
+    tile_edges(id, xi, X, q);
+    F2 m[3][3];
+    {
+        const unsigned a0 = id.x, a1 = id.y, b0 = id.z, b1 = id.w;
+        const bool va = a1 >> 16, vb = b1 >> 16;
+        const float4 la[3] = {L[va ? a0 & 0xffffu : zero], L[va ? a0 >> 16 : zero], L[va ? a1 & 0xffffu : zero]};
+        const float4 lb[3] = {L[vb ? b0 & 0xffffu : zero], L[vb ? b0 >> 16 : zero], L[vb ? b1 & 0xffffu : zero]};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            m[k][0] = f2(la[k].x, lb[k].x);
+            m[k][1] = f2(la[k].y, lb[k].y);
+            m[k][2] = f2(la[k].z, lb[k].z);
+        }
+    }
+    const F2 detm = r.detm();
+    const F2 jm1 = fma2(dot2(q.d[0][0], q.c[0][0], q.d[0][1], q.c[0][1], q.d[0][2], q.c[0][2]), detm, f2(-1.f, -1.f));
+    F2 dJ;
+    {
+        const F2 t0 = dot2(q.c[0][0], m[0][0], q.c[0][1], m[0][1], q.c[0][2], m[0][2]);
+        const F2 t1 = dot2(q.c[1][0], m[1][0], q.c[1][1], m[1][1], q.c[1][2], m[1][2]);
+        const F2 t2 = dot2(q.c[2][0], m[2][0], q.c[2][1], m[2][1], q.c[2][2], m[2][2]);
+        dJ = mul2(detm, add2(add2(t0, t1), t2));
+    }
+    const F2 n0[3] = {neg2(q.d[0][0]), neg2(q.d[0][1]), neg2(q.d[0][2])};
+    const ulonglong2 sw = r.s2w0(), w12 = r.w12(), s01 = r.s01(), ab = r.ab();
+    F2 C[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+        // lam_1 x d_2 + d_1 x lam_2 and cyclic
+        const F2 e0 = add2(cross2(m[1][i1], q.d[2][i2], m[1][i2], q.n2[i1]), cross2(q.d[1][i1], m[2][i2], q.n1[i2], m[2][i1]));
+        const F2 e1 = add2(cross2(m[2][i1], q.d[0][i2], m[2][i2], n0[i1]), cross2(q.d[2][i1], m[0][i2], q.n2[i2], m[0][i1]));
+        const F2 e2 = add2(cross2(m[0][i1], q.d[1][i2], m[0][i2], q.n1[i1]), cross2(q.d[0][i1], m[1][i2], n0[i2], m[1][i1]));
+        C[i] = dot2(q.c[0][i], sw.y, q.c[1][i], w12.x, q.c[2][i], w12.y);
+        const F2 dF = dot2(m[0][i], s01.x, m[1][i], s01.y, m[2][i], sw.x);
+        const F2 dC = dot2(e0, sw.y, e1, w12.x, e2, w12.y);
+        F2& g = i == 0 ? acc.g0 : i == 1 ? acc.g1 : acc.g2;
+        g = add2(g, fma2(ab.x, sub2(dF, dC), mul2(ab.y, fma2(dJ, C[i], mul2(jm1, dC)))));
+    }
+    const F2 am = mul2(ab.x, neg2(add2(add2(s01.x, s01.y), sw.x)));
+    const F2 b0 = mul2(ab.y, C[0]), b1 = mul2(ab.y, C[1]), b2 = mul2(ab.y, C[2]);
+    acc.h00 = add2(acc.h00, fma2(b0, C[0], am));
+    acc.h01 = fma2(b0, C[1], acc.h01);
+    acc.h02 = fma2(b0, C[2], acc.h02);
+    acc.h11 = add2(acc.h11, fma2(b1, C[1], am));
+    acc.h12 = fma2(b1, C[2], acc.h12);
+    acc.h22 = add2(acc.h22, fma2(b2, C[2], am));
+}
+
+// Record chunks from the packed incidence records (layout 3 or 4): chunk i holds round `r` of a group;
+// vertex slot k's threads t take incidences r L + t and r L + t + L/2.  Neighbour ids become local.
+template <int LAYOUT>
+__global__ void __launch_bounds__(256) k_pack_tile(SweepParams p, const int* __restrict__ table, int nchunks, int lanes,
+                                                   const TileGroup* __restrict__ groups, const TileHead* __restrict__ head,
+                                                   const int* __restrict__ lid, const int* __restrict__ vtile,
+                                                   const int* __restrict__ vlocal, int nfree, float4* __restrict__ out) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= nchunks) return;
+    const int tile = table[3 * i], round = table[3 * i + 2];
+    const TileGroup g = groups[table[3 * i + 1]];
+    const TileHead h = head[tile];
+    const int T = lanes / 2;
+    const int slot = lane / T, t = lane % T;
+    auto local = [&](int v) {
+        if (v < nfree && vtile[v] == tile) return vlocal[v];
+        const int* e = lid + h.lid + h.nown;  // ghosts and pinned neighbours, ascending ids
+        int lo = 0, hi = h.nghost + h.npinned;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (e[mid] < v) lo = mid + 1;
+            else hi = mid;
+        }
+        return h.nown + lo;
+    };
+    FactRec r[2];
+    int id0[2], id1[2];
+    const int self = g.lv + min(slot, g.count - 1);  // padding: the vertex itself
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        r[b] = FactRec{};
+        id0[b] = self | (self << 16);
+        id1[b] = self;
+        if (slot >= g.count) continue;
+        const int j = p.inc_off[g.gv + slot] + round * lanes + t + b * T;
+        if (j >= p.inc_off[g.gv + slot + 1]) continue;
+        r[b] = decode_fact(Elem<LAYOUT>::fetch(p, j));
+        id0[b] = local(r[b].nb0) | (local(r[b].nb1) << 16);
+        id1[b] = local(r[b].nb2) | (1 << 16);
+    }
+    float4* o = out + (size_t)i * (kTileChunkBytes / 16);
+    o[lane] = make_float4(r[0].s0, r[1].s0, r[0].s1, r[1].s1);
+    o[32 + lane] = make_float4(r[0].s2, r[1].s2, r[0].w0, r[1].w0);
+    o[64 + lane] = make_float4(r[0].w1, r[1].w1, r[0].w2, r[1].w2);
+    o[96 + lane] = make_float4(r[0].a, r[1].a, r[0].b, r[1].b);
+    reinterpret_cast<int4*>(o)[128 + lane] = make_int4(id0[0], id1[0], id0[1], id1[1]);
+    reinterpret_cast<float2*>(o + 160)[lane] = make_float2(r[0].detm, r[1].detm);
+}
+
+// T threads per vertex (2 T lanes' partial sums), W warps.  W = 8 is the form for tiles with little work
+// per colour, where a colour lasts as long as one vertex's dependency chain: everything that does not
+// depend on the neighbours is fetched before the barrier, and up to two ring slots are refilled only
+// after the group's results are out.  W = 16 is the form for tiles that keep an SM's issue slots and
+// memory streams busy, held to 128 registers.
+template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
+    extern __shared__ __align__(16) unsigned char tsm[];
+    constexpr int NT = W * 32;
+    constexpr bool LAT = W <= 8;
+    __shared__ __align__(8) unsigned long long bars[LAT ? 1 : W * kTileMaxRing];
+    __shared__ float4 stage[LAT ? 1 : W * 64 / T];  // W = 16: own data of each warp's next group
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.x;
+    const TileHead h = p.head[tile];
+    char* ring_buf = reinterpret_cast<char*>(tsm) + (size_t)warp * p.ring * kTileChunkBytes;
+    float4* sx = reinterpret_cast<float4*>(tsm + (size_t)W * p.ring * kTileChunkBytes);  // x (or lambda)
+    float4* sX = sx + (p.max_local + 1);                  // adjoint: X; forward: the blended buffer (p.two)
+    TileGroup* sg = reinterpret_cast<TileGroup*>(sx + (size_t)(p.max_local + 1) * (ADJ || p.two ? 2 : 1));
+    int* gid = reinterpret_cast<int*>(sg + p.max_groups);  // internal ids of own vertices and ghosts
+    int* ghost = gid + p.max_ids;
+    int* wcols = ghost + p.ncol + 1;
+
+    const unsigned ring_smem = (unsigned)__cvta_generic_to_shared(ring_buf);
+    TileRing ring;
+    {
+        const int2 ws = p.wstream[tile * W + warp];
+        ring.first = ring.next = ws.x;
+        ring.end = ws.x + ws.y;
+        ring.left = ws.y * (p.k1 - p.k0);
+        ring.slot = 0;
+    }
+    const unsigned bar = LAT ? 0u : (unsigned)__cvta_generic_to_shared(bars + warp * kTileMaxRing);
+    unsigned parity = 0;  // W = 16: of the ring's current round
+    if (!LAT) {
+        if (lane == 0) {
+            for (int i = 0; i < p.ring; ++i) mbar_init(bar + 8u * i);
+            fence_mbar_init();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncwarp();
+    }
+    for (int i = 0; i < p.ring; ++i) {
+        if (LAT) ring_issue(p, ring, ring_smem, i, lane);
+        else ring_issue_bulk(p, ring, ring_smem, bar, i, lane);
+    }
+    if (tid == 0) atomicAdd(p.arrived, 1ull);
+
+    for (int i = tid; i < h.ngroups; i += NT) sg[i] = p.groups[h.group + i];
+    for (int i = tid; i <= p.ncol; i += NT) ghost[i] = p.ghost[tile * (p.ncol + 1) + i];
+    for (int i = tid; i < W * (p.ncol + 1); i += NT) wcols[i] = p.wcol[tile * W * (p.ncol + 1) + i];
+    const int* lid = p.lid + h.lid;
+    const int nloc = h.nown + h.nghost + h.npinned;
+    for (int i = tid; i < h.nown + h.nghost; i += NT) gid[i] = lid[i];
+    if constexpr (ADJ) {
+        for (int i = tid; i < nloc; i += NT) {
+            const int g = lid[i];
+            sX[i] = __ldg(p.X + g);
+            sx[i] = p.lam_in[g];
+        }
+        if (tid == 0) sx[p.max_local] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+        // own vertices, and this CTA's share of the pinned ones
+        const int gp = p.nfree + tile * NT + tid, step = gridDim.x * NT;
+        if (p.predict) {
+            for (int i = tid; i < h.nown; i += NT)
+                predict_vertex(lid[i], p.x0, p.v, p.xprev, p.y, p.nfree, p.h, p.hgx, p.hgy, p.hgz);
+            for (int g = gp; g < p.n; g += step)
+                predict_vertex(g, p.x0, p.v, p.xprev, p.y, p.nfree, p.h, p.hgx, p.hgy, p.hgz);
+        }
+        for (int i = tid; i < nloc; i += NT) {
+            const int g = lid[i];
+            const float4 a = p.from_inertia ? p.y[g] : p.x0[g];
+            sx[i] = make_float4(a.x, a.y, a.z, 0.f);
+            if (p.two) sX[i] = make_float4(a.x, a.y, a.z, 0.f);
+        }
+        if (p.from_inertia)  // x = y for the pinned vertices too (k_copy_xyz)
+            for (int g = gp; g < p.n; g += step) {
+                const float4 a = p.y[g];
+                p.x0[g] = p.x1[g] = make_float4(a.x, a.y, a.z, 0.f);
+            }
+    }
+    __syncthreads();
+
+    // Which ghost a thread polls first: W = 8 spreads them over the warps, the last one first (a warp's
+    // poll takes as long as its slowest lane, and the first warps sweep most).
+    const int poll_at = LAT ? lane * W + (W - 1 - warp) : NT - 1 - tid;
+    const int slot = lane / T, t = lane & (T - 1);
+    const int* wcol = wcols + warp * (p.ncol + 1);
+    const int wfirst = wcol[0], wlast = wcol[p.ncol];
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    // The warp's next group and its vertices' own data, fetched before the barrier that precedes its
+    // sweep: y (adjoint: G) by thread t = 0 of a vertex, the position before the last sweep by t = 1.  W = 8
+    // holds them in registers; W = 16 has none to spare and stages them in shared memory.
+    TileGroup next_g{};
+    float4 own = zero4;
+    float mass = 0.f;
+    float4* my_stage = stage + (LAT ? 0 : warp * (64 / T) + 2 * slot);
+    auto load_group = [&](int gi) {
+        const TileGroup g = sg[gi];
+        const int gv = g.gv + slot;
+        const float4* src = (t == 0 ? (ADJ ? p.G : p.y) : p.pp) + gv;
+        if (LAT) {
+            next_g = g;
+            // predicated loads into the same registers: no instruction waits for them before the solve
+            load_if(slot < g.count && t < 2, src, own);
+            if constexpr (ADJ) load_if(slot < g.count && t == 0, &p.y[gv].w, mass);
+        } else {
+            if (slot < g.count && t < 2)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(my_stage + t)),
+                             "l"(src)
+                             : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+    };
+    bool ok = true;
+    // Chunk i is commit group i.  W = 8: a group's chunks (at most p.max_rounds) have all landed before the
+    // barrier that precedes its sweep, and its slots are refilled after its results are out.  W = 16: a
+    // chunk is waited for when it is swept and refilled right after.
+    const int pending = p.ring - p.max_rounds;
+    auto chunk_at = [&](int s) { return TilePair{ring_buf + s * kTileChunkBytes, lane}; };
+    auto next_slot = [&](int s) { return s + 1 == p.ring ? 0 : s + 1; };
+    if (p.k1 > p.k0 && wlast > wfirst) {
+        load_group(wfirst);
+        if (LAT) ring_wait(pending);
+    }
+    bool alive = true;
+    float4* xs = sx;  // x (adjoint: lambda) of this iteration
+    float4* xb = sX;  // p.two: receives the blended positions
+    for (int k = p.k0; k < p.k1 && alive; ++k) {
+        const float om = __ldg(p.omega + k);
+        const bool blend = om > 1.0f;
+        const unsigned tag = p.tag + (unsigned)k;
+        // the words of x~ and of the blended positions; W = 16 forms the addresses where it uses them
+        auto words = [&](unsigned which) {
+            unsigned at = which + (tag & 1u);
+            if (!LAT) asm volatile("" : "+r"(at));
+            return p.words + (size_t)at * p.n;
+        };
+        int gi = wfirst;
+        for (int c = 0; c < p.ncol; ++c) {
+            const int gend = wcol[c + 1];
+            int p0 = 0, p1 = 0;  // the ghosts of colour c (last threads first: the last warps sweep least)
+            if (LAT) p0 = ghost[c] + poll_at, p1 = ghost[c + 1];
+            __syncthreads();  // everything colour c reads is in shared memory
+            while (gi < gend) {
+                float4 xi = zero4;
+                int rounds;
+                {
+                    const TileGroup g = LAT ? next_g : sg[gi];
+                    if (slot < g.count) xi = (ADJ ? sX : xs)[g.lv + slot];
+                    rounds = g.rounds;
+                }
+                Acc2 acc2;
+                acc2.zero();
+                if constexpr (LAT) {
+                    // two chunks at a time: their gathers and products are independent, the sums in order
+                    int at = ring.slot, left = rounds;
+                    for (; left > 1; left -= 2) {
+                        const TilePair r0 = chunk_at(at), r1 = chunk_at(next_slot(at));
+                        at = next_slot(next_slot(at));
+                        if constexpr (ADJ) {
+                            tile_adjoint(r0, r0.ids(), xi, sX, xs, p.max_local, acc2);
+                            tile_adjoint(r1, r1.ids(), xi, sX, xs, p.max_local, acc2);
+                        } else {
+                            tile_contrib(r0, r0.ids(), xi, xs, acc2);
+                            tile_contrib(r1, r1.ids(), xi, xs, acc2);
+                        }
+                    }
+                    if (left > 0) {
+                        const TilePair r0 = chunk_at(at);
+                        if constexpr (ADJ) tile_adjoint(r0, r0.ids(), xi, sX, xs, p.max_local, acc2);
+                        else tile_contrib(r0, r0.ids(), xi, xs, acc2);
+                    }
+                } else {
+                    for (; rounds > 0 && ok; --rounds) {
+                        const int used = ring.slot;
+                        ok = ring_wait_bulk(p, bar + 8u * used, parity);
+                        ring.slot = next_slot(used);
+                        if (ring.slot == 0) parity ^= 1u;
+                        const TilePair rec = chunk_at(used);
+                        if constexpr (ADJ) tile_adjoint(rec, rec.ids(), xi, sX, xs, p.max_local, acc2);
+                        else tile_contrib(rec, rec.ids(), xi, xs, acc2);
+                        __syncwarp();  // every lane has read slot `used`
+                        ring_issue_bulk(p, ring, ring_smem, bar, used, lane);
+                    }
+                }
+                // W = 16 reads the group again instead of holding it
+                const TileGroup g = LAT ? next_g : sg[gi];
+                const bool active = slot < g.count;
+                const int lv = g.lv + slot;
+                // lanes t and t + T, then the T threads: group_reduce's order for 2 T lanes
+                Acc acc = acc2.sum();
+                group_reduce<T>(acc);
+                float4 y = own, q = own;
+                if (LAT) {
+                    if (blend) {  // the previous position, from the vertex's second thread
+                        q.x = __shfl_down_sync(0xffffffffu, own.x, 1);
+                        q.y = __shfl_down_sync(0xffffffffu, own.y, 1);
+                        q.z = __shfl_down_sync(0xffffffffu, own.z, 1);
+                    }
+                } else {
+                    ring_wait_for<0>();
+                    __syncwarp();
+                    if (active && t == 0) {
+                        y = my_stage[0];
+                        q = my_stage[1];
+                        if constexpr (ADJ) mass = __ldg(&p.y[g.gv + slot].w);
+                    }
+                }
+                if (active && t == 0) {
+                    const int gv = g.gv + slot;
+                    float4 xn, xa, old;
+                    if constexpr (ADJ) {
+                        old = xs[lv];
+                        xn = adj_block_solve(acc, mass, p.dtsr, y);
+                    } else {
+                        old = xi;
+                        xn = block_update(acc, xi, y, p.dtsr, p.status);
+                    }
+                    if (slot < g.publish) word_store(words(0u) + gv, xn.x, xn.y, xn.z, tag);
+                    if (blend) {
+                        xa = ADJ ? adj_blend(xn, q, om) : cheb_blend(xn, q, om);
+                        if (!p.two || slot < g.publish) word_store(words(2u) + gv, xa.x, xa.y, xa.z, tag);
+                        if (p.two) xb[lv] = xa;
+                    }
+                    xs[lv] = xn;
+                    if (p.keep_pp) p.pp[gv] = old;
+                    if (!ADJ) flag_nonfinite(xn, p.status);
+                }
+                __syncwarp();  // the second thread may read p.pp of the same vertex next
+                ++gi;
+                load_group(gi < wlast ? gi : wfirst);
+                if (LAT) {
+                    for (; rounds > 0; --rounds) {
+                        ring_issue(p, ring, ring_smem, ring.slot, lane);
+                        ring.slot = next_slot(ring.slot);
+                    }
+                    ring_wait(pending);
+                }
+            }
+            // Colour c of the neighbouring tiles: x~, which the next colour reads.  Nobody reads x~ of the last
+            // colour when the iteration blends.  With both buffers here the blended words are taken as
+            // well, one colour late (they have landed by then and are needed only next iteration).
+            const bool last = c == p.ncol - 1, more = k < p.k1 - 1;
+            if (!LAT) p0 = ghost[c] + poll_at, p1 = ghost[c + 1];
+            if (blend && p.two && more) {
+                const int e = last ? ghost[c + 1] : ghost[c];
+                for (int i = (c ? ghost[c - 1] : ghost[0]) + poll_at; ok && i < e; i += NT) {
+                    const float4* w = words(2u) + gid[i];
+                    ok = tile_take(p, word_load(w), w, tag, xb + i);
+                }
+            }
+            if (last ? !blend && more : true)
+                for (int i = p0; ok && i < p1; i += NT) {
+                    const float4* w = words(0u) + gid[i];
+                    ok = LAT ? tile_spin(p, w, tag, xs + i) : tile_take(p, word_load(w), w, tag, xs + i);
+                }
+        }
+        // one wait that gave up ends the walk
+        alive = __syncthreads_and(ok) != 0;
+        if (!alive || !blend) continue;
+        if (p.two) {
+            float4* s = xs;
+            xs = xb;
+            xb = s;
+            continue;
+        }
+        // the blended positions replace x~: own ones and ghosts
+        const int e = k == p.k1 - 1 ? h.nown : h.nown + h.nghost;
+        constexpr int kBatch = 6;
+        const float4* wb = words(2u);
+        for (int i0 = tid; ok && i0 < e; i0 += kBatch * NT) {
+            float4 w[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (i0 + u * NT < e) w[u] = word_load(wb + gid[i0 + u * NT]);
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const int i = i0 + u * NT;
+                if (i >= e) continue;
+                if (__float_as_uint(w[u].w) == tag) xs[i] = make_float4(w[u].x, w[u].y, w[u].z, 0.f);
+                else ok = ok && tile_spin(p, wb + gid[i], tag, xs + i);
+            }
+        }
+    }
+    ok = __syncthreads_and(alive && ok) != 0;
+    // no copy outlives the walk (one that gave up has bulk copies under way; the waits are bounded)
+    ring_wait_for<0>();
+    if (!LAT && !ok) {
+        for (int i = 0; i < p.ring; ++i) {
+            for (int n = 0; n < 100000 && !ring_try(bar + 8u * ring.slot, parity); ++n) __nanosleep(100);
+            ring.slot = next_slot(ring.slot);
+            if (ring.slot == 0) parity ^= 1u;
+        }
+    }
+    if (!ok) return;
+    for (int i = tid; i < h.nown; i += NT) {
+        const int gv = gid[i];
+        const float4 xf = xs[i];
+        if constexpr (ADJ) {
+            p.lam_out[gv] = xf;
+        } else {
+            p.x0[gv] = xf;
+            if (p.from_inertia) p.x1[gv] = xf;
+            if (p.finish) p.v[gv] = damped_velocity(xf, p.xprev[gv], p.v[gv], p.h);
+        }
+    }
+}
+
+}  // namespace vbd

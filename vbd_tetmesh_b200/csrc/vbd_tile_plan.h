@@ -1,0 +1,80 @@
+// Host plan of the tile walk (vbd_tile.cuh): which free vertices each CTA ("tile") owns, the
+// vertices it reads from other tiles, and the order its warps sweep them in.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+namespace vbd {
+
+constexpr int kTileMaxWarps = 16;           // warps of a tile's CTA: 8 or 16 (TilePlan::warps)
+constexpr int kTileChunk = 64;              // incidences per record chunk: two per thread of a warp
+constexpr int kTileChunkBytes = kTileChunk * 44;
+constexpr int kTileMaxRing = 6;             // chunks a warp's ring holds at most
+constexpr int kTileMaxLocal = 65535;        // local vertex ids are 16 bits
+// A mesh gets a plan from this many free vertices.  Microseconds per colour of a step, tile walk against
+// captured graph (cubes of n^3 cells, one B200): n = 6 (294 free vertices) 1.61 / 2.33, 8 1.77 / 2.40, 16
+// 1.91 / 2.57, 24 2.07 / 3.31, 32 2.76 / 3.53, 48 4.8 / 5.5, 64 8.4 / 10.2.  Below it one or two tiles
+// would hold the mesh.
+constexpr int kTileMinVertices = 256;
+// Free vertices per tile at least, up to one tile per SM.  32, 64 and 128 measured 0.81, 0.81 and 0.86 ms a
+// step on the 12^3 to 16^3 cubes: a colour lasts one exchange and one vertex's chain either way.
+constexpr int kTileVertices = 32;
+// Groups per colour and tile up to which 8 warps sweep them; 16 above.  Microseconds per colour with 8 / 16
+// warps: 28^3 cube (4.6 groups) 2.36 / 2.46, 32^3 (7.2) 2.99 / 2.76, 64 beams (7.7) 3.06 / 2.81, 64^3 (29)
+// 10.8 / 8.4.
+constexpr int kTileFewGroups = 6;
+// Ring depth that holding both position buffers must leave.
+constexpr int kTileTwoRing = 4;
+
+// One group of vertices a warp sweeps together: internal ids [gv, gv + count), local ids from lv;
+// `rounds` chunks hold its incidences.  The first `publish` of them are read by other tiles.
+struct alignas(16) TileGroup {
+    int gv, lv;
+    short count, publish;
+    int rounds;
+};
+
+struct TileHead {
+    int nown, nghost, npinned;  // local ids: own by colour, then ghosts by colour, then pinned vertices
+    int lid;                    // first entry in the local-to-internal id list
+    int group;                  // first group
+    int ngroups;
+};
+
+struct TilePlan {
+    int P = 0, C = 0, n = 0, nfree = 0;
+    std::vector<int32_t> vtile;    // tile of each internal free vertex
+    std::vector<int32_t> vlocal;   // its local id in that tile
+    std::vector<int32_t> cb;       // [C][P + 1]: colour c's vertices of tile t are [cb[t], cb[t + 1])
+    std::vector<int32_t> bnd;      // [C][P]: the first of them up to this id are read by other tiles
+    std::vector<TileHead> head;    // [P]
+    std::vector<int32_t> lid;      // local-to-internal ids of all tiles
+    std::vector<int32_t> ghost;    // [P][C + 1]: first ghost of each colour (local id)
+    int max_local = 0, max_ids = 0, max_groups = 0, max_rounds = 0;
+    // for `lanes` threads' worth of partial sums per vertex:
+    int lanes = 0, warps = 0;
+    std::vector<TileGroup> groups;
+    std::vector<int32_t> wcol;     // [P][warps][C + 1]: first group of each warp and colour, from the tile's first
+    std::vector<int32_t> wstream;  // [P][warps][2]: first chunk and chunks of each warp
+    std::vector<int32_t> chunk;    // [chunks][3]: tile, group, round
+};
+
+// The tile of each vertex (-1 for pinned ones): recursive bisection of the free vertices, first by
+// mesh (mesh_of may be null: one mesh), then along the longest axis of their positions.
+void tile_partition(int n, const float* positions, const uint8_t* fixed, const int32_t* mesh_of, int parts,
+                    std::vector<int32_t>* tile);
+
+// Marks the free vertices that a free vertex of another tile shares a tet with.
+void tile_boundary(int n, int ntet, const int32_t* tets, const std::vector<int32_t>& tile, std::vector<uint8_t>* boundary);
+
+// The plan's lists that do not depend on the lane count, from the internal numbering.  tets_internal[4 T]
+// holds internal ids; inc_off / inc_tet the incidences of internal vertices.
+void tile_lists(TilePlan* plan, const std::vector<int>& cstart, const std::vector<int32_t>& tile_internal,
+                const std::vector<uint8_t>& boundary_internal, const int32_t* inc_off, const int32_t* inc_tet,
+                const int32_t* tets_internal, int tet_stride);
+
+// The groups and record chunks for `lanes` partial sums per vertex (two per thread) and CTAs of `warps` warps.
+void tile_groups(TilePlan* plan, int lanes, int warps, const int32_t* inc_off);
+
+}  // namespace vbd
