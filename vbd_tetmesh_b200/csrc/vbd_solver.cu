@@ -544,6 +544,7 @@ struct vbd_solver {
         if (d_cstart.n != cstart.size()) {
             VBD_TRY(d_cstart.alloc(cstart.size()));
             CUDA_TRY(cudaMemcpy(d_cstart.p, cstart.data(), sizeof(int) * cstart.size(), cudaMemcpyHostToDevice));
+            CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));  // landed before any kernel of `stream`
         }
         std::vector<float> w = omega_schedule(iters, accel, rho);
         if (w != omega_cache) {
@@ -719,6 +720,7 @@ struct vbd_solver {
         if (d_cstart.n != cstart.size()) {
             VBD_TRY(d_cstart.alloc(cstart.size()));
             CUDA_TRY(cudaMemcpy(d_cstart.p, cstart.data(), sizeof(int) * cstart.size(), cudaMemcpyHostToDevice));
+            CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));  // landed before any kernel of `stream`
         }
         const int L = lanes < 4 ? 4 : lanes;
         void (*fn)(vbd::AdjWalkParams) = nullptr;
@@ -1390,7 +1392,7 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
     s->sm_count = prop.multiProcessorCount;
     s->smem_optin = (int)prop.sharedMemPerBlockOptin;
     VBD_TRY(s->status.alloc(vbd::ST_SLOTS));
-    CUDA_TRY(cudaMemset(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS));
+    CUDA_TRY(cudaMemsetAsync(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS, s->stream));
     VBD_TRY(s->scalar.alloc(1));
     *out = s.release();
     return VBD_OK;
@@ -1586,22 +1588,24 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     const long long max_blocks = std::max<long long>(4096, vbd::nblk((long long)N * 32, 256));
     VBD_TRY(s->partials.alloc(max_blocks));
     const size_t b4 = sizeof(float4) * (size_t)N;
-    CUDA_TRY(cudaMemcpy(s->x0.p, hx.data(), b4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->x1.p, hx.data(), b4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->xprev.p, hx.data(), b4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->pp.p, hx.data(), b4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->v.p, hv.data(), b4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->y.p, hy.data(), b4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->perm.p, perm.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->inc_off.p, inc_off.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice));
+    // on the solver's own stream: a copy from pageable memory may return before it has landed, and a
+    // non-blocking stream's kernels do not wait for the legacy stream's copies
+    CUDA_TRY(cudaMemcpyAsync(s->x0.p, hx.data(), b4, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->x1.p, hx.data(), b4, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->xprev.p, hx.data(), b4, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->pp.p, hx.data(), b4, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->v.p, hv.data(), b4, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->y.p, hy.data(), b4, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->perm.p, perm.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->inc_off.p, inc_off.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice, s->stream));
     s->h_inc_off = inc_off;  // the cluster walk's resident-record plan reads it on the host
-    CUDA_TRY(cudaMemcpy(s->inc_tet.p, inc_tet.data(), sizeof(int) * inc_tet.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->inc_vertex.p, inc_vertex.data(), sizeof(int) * inc_vertex.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->rec.p, rec.data(), sizeof(vbd::TetRec) * rec.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemset(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS));
+    CUDA_TRY(cudaMemcpyAsync(s->inc_tet.p, inc_tet.data(), sizeof(int) * inc_tet.size(), cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->inc_vertex.p, inc_vertex.data(), sizeof(int) * inc_vertex.size(), cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(s->rec.p, rec.data(), sizeof(vbd::TetRec) * rec.size(), cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS, s->stream));
     // the energy history belongs to the previous mesh
     s->ehist_queued = 0;
-    if (s->ecount.p) CUDA_TRY(cudaMemset(s->ecount.p, 0, sizeof(int)));
+    if (s->ecount.p) CUDA_TRY(cudaMemsetAsync(s->ecount.p, 0, sizeof(int), s->stream));
 
     if (s->lanes_auto) {
         int L = (nfree > 0 && (double)ninc >= 21.0 * nfree) ? 8 : 4;
@@ -2012,7 +2016,7 @@ int vbd_solver_sync(vbd_solver* s) {
         unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
         CUDA_TRY(cudaMemcpy(t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
         if (t[0] || t[1]) {
-            CUDA_TRY(cudaMemset(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t)));
+            CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
             if (t[0]) VBD_FAIL(VBD_ERR_TIMEOUT, "a grid barrier of the persistent kernel gave up waiting");
             VBD_FAIL(VBD_ERR_TIMEOUT, "a wait of the cluster or tile walk gave up");
         }
@@ -2034,7 +2038,7 @@ int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* time
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     unsigned long long t = 0;
     CUDA_TRY(cudaMemcpy(&t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemset(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t)));
+    CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
     *timed_out = t ? 1 : 0;
     return VBD_OK;
 }
