@@ -259,7 +259,19 @@ struct vbd_solver {
     };
     std::vector<TapeStep> tape;
     int ckpt_every = 0;
-    std::vector<std::unique_ptr<vbd::DBuf<float4>>> ckpts;  // 2N each: x then v
+    // 2N each: x then v.  A new recording takes the buffers of the last one (ckpt_pool) before it allocates:
+    // cudaMalloc and cudaFree in every pass of a fit cost 1.5 ms, and now and then 100 ms to a second.
+    std::vector<std::unique_ptr<vbd::DBuf<float4>>> ckpts, ckpt_pool;
+    int add_ckpt() {
+        if (ckpt_pool.empty()) {
+            ckpts.emplace_back(new vbd::DBuf<float4>());
+        } else {
+            ckpts.push_back(std::move(ckpt_pool.back()));
+            ckpt_pool.pop_back();
+        }
+        if (ckpts.back()->n != 2 * (size_t)N) VBD_TRY(ckpts.back()->alloc(2 * (size_t)N));
+        return snapshot(*ckpts.back());
+    }
     vbd::DBuf<float4> adj_lam, adj_lam2, adj_lpp, adj_G, adj_ax, adj_av, adj_seg, adj_save;
     // converged positions of the recorded sub-steps of the newest segment, kept as the forward runs
     // so that the backward starts without recomputing that segment
@@ -1068,9 +1080,7 @@ struct vbd_solver {
         CUDA_TRY(cudaMemcpyAsync(live_seg.p + slot * (size_t)N, x0.p, sizeof(float4) * (size_t)N,
                                  cudaMemcpyDeviceToDevice, stream));
         if (tape.size() % (size_t)ckpt_every == 0) {
-            ckpts.emplace_back(new vbd::DBuf<float4>());
-            VBD_TRY(ckpts.back()->alloc(2 * (size_t)N));
-            VBD_TRY(snapshot(*ckpts.back()));
+            VBD_TRY(add_ckpt());
         }
         return VBD_OK;
     }
@@ -1909,6 +1919,9 @@ int vbd_solver_record(vbd_solver* s, int32_t checkpoint_every) {
         VBD_FAIL(VBD_ERR_STATE, "the adjoint differentiates the VBDsolver semantics; set VBD_OPT_SEMANTICS to 0");
     DeviceScope scope(s->device);
     s->tape.clear();
+    // a new recording reuses the last one's buffers; stopping gives them back
+    if (checkpoint_every == 0) s->ckpt_pool.clear();
+    else for (auto& c : s->ckpts) s->ckpt_pool.push_back(std::move(c));
     s->ckpts.clear();
     s->ckpt_every = checkpoint_every;
     if (checkpoint_every > 0) {
@@ -1916,9 +1929,7 @@ int vbd_solver_record(vbd_solver* s, int32_t checkpoint_every) {
             s->drop_graphs();
             VBD_TRY(s->live_seg.alloc((size_t)checkpoint_every * s->N));
         }
-        s->ckpts.emplace_back(new vbd::DBuf<float4>());
-        VBD_TRY(s->ckpts.back()->alloc(2 * (size_t)s->N));
-        VBD_TRY(s->snapshot(*s->ckpts.back()));
+        VBD_TRY(s->add_ckpt());
         CUDA_TRY(cudaStreamSynchronize(s->stream));
     }
     return VBD_OK;
