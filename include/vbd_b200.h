@@ -301,23 +301,21 @@ int vbd_solver_status(vbd_solver* s, int64_t* singular_skips, int32_t* nonfinite
  *                        1 = run each step / solve as one cooperative launch that walks the colours
  *                        with a grid barrier after each one (bounded wait: a barrier that gives up
  *                        makes the next vbd_solver_sync return VBD_ERR_TIMEOUT);
- *                        2 = run each sub-step / solve as ONE thread-block cluster that keeps both
- *                        position buffers of the mesh (and the pre-sweep positions) in every CTA's
- *                        shared memory, exchanges updated positions through distributed shared
- *                        memory and separates the colours with the cluster's hardware barrier.  For
- *                        meshes whose positions fit (48 B per vertex within the device's per-CTA
- *                        shared memory: about 4,800 vertices on B200) with the factored records (VBD_OPT_LAYOUT 3 or
+ *                        2 = run each sub-step / solve as ONE thread-block cluster whose CTAs hold a
+ *                        tile of the mesh each (its records too where they fit) and send their
+ *                        borders' new positions to each other through distributed shared memory.  For
+ *                        meshes of at most 48 B per vertex within the device's per-CTA shared memory
+ *                        (about 4,800 vertices on B200) with the factored records (VBD_OPT_LAYOUT 3 or
  *                        4); VBD_ERR_INVALID_ARG otherwise.  Same results as the captured graph at the
  *                        same lane count.  Both persistent forms use VBD_OPT_LANES for every colour
  *                        (at least 4) and evaluate no energy history
- *   VBD_OPT_CLUSTER_CTAS: CTAs of the cluster walk, 1-16; 0 (default) = enough 256-thread
- *                        CTAs to sweep the largest colour in one round, at most 16.  Reading it
- *                        back gives the set count, or the automatic count for the current lanes
- *   VBD_OPT_CLUSTER_RESIDENT: 1 (default) = the cluster walk copies, once per sub-step, the element
- *                        records, inertial targets and incidence spans of the vertices each CTA
- *                        sweeps into that CTA's shared memory when they fit beside the positions,
- *                        so no colour waits on L2 for them; 0 = they are read from L2 each colour.
- *                        Same results either way
+ *   VBD_OPT_CLUSTER_CTAS: CTAs of the cluster walk, 1-16; 0 (default) = one per 16 free vertices, at most
+ *                        16.  Reading it back gives the set count, or the automatic count for the
+ *                        current lanes
+ *   VBD_OPT_CLUSTER_RESIDENT: 1 (default) = the cluster walk as above; 0 = every CTA keeps the positions of
+ *                        the whole mesh instead of a tile and reads the element records from L2 each
+ *                        colour (also where the tiles do not fit; automatic CTA count: enough 256-thread
+ *                        CTAs to sweep the largest colour in one round).  Same results either way
  *   VBD_OPT_ADJOINT_ALTERNATE: 1 = adjoint sweeps alternate the colour order (a forward and a
  *                        backward sweep form one symmetric Gauss-Seidel pair)
  *   VBD_OPT_SEMANTICS:   0 = the CPU solver's (VBDsolver, VBD.cpp:114-256): Neo-Hookean element,

@@ -100,6 +100,36 @@ int main(int argc, char** argv) {
     p.n = N;
     p.nfree = nfree;
     vbd::tile_lists(&p, cstart, til, bin, off.data(), inc.data(), tin.data(), 4);
+    // merged plans (the CTAs of a cluster): the lists of the merged tiles made directly, and each ghost
+    // entry the target of its vertex exactly once
+    for (int parts : {1, std::min(P, 3), std::min(P, 16)}) {
+        vbd::TilePlan m, d;
+        vbd::tile_merge(p, parts, cstart, &m);
+        std::vector<int32_t> mt(N, -1);
+        for (int v = 0; v < nfree; ++v) mt[v] = m.vtile[v];
+        d.P = parts;
+        d.n = N;
+        d.nfree = nfree;
+        vbd::tile_lists(&d, cstart, mt, bin, off.data(), inc.data(), tin.data(), 4);
+        REQUIRE(m.vlocal == d.vlocal && m.lid == d.lid && m.ghost == d.ghost && m.cb == d.cb);
+        REQUIRE(m.max_local == d.max_local && m.max_ids == d.max_ids);
+        std::set<int> targets;
+        size_t ghosts = 0;
+        for (int t = 0; t < parts; ++t) {
+            const vbd::TileHead& h = m.head[t];
+            REQUIRE(h.nown == d.head[t].nown && h.nghost == d.head[t].nghost && h.npinned == d.head[t].npinned);
+            ghosts += h.nghost;
+            const int32_t* at = &m.target_off[(size_t)t * (m.max_own + 1)];
+            REQUIRE(h.nown <= m.max_own && at[0] == 0 && at[h.nown] <= m.max_target);
+            for (int i = 0; i < h.nown; ++i)
+                for (int k = at[i]; k < at[i + 1]; ++k) {
+                    const int to = m.target[(size_t)t * m.max_target + k], r = to >> 16, l = to & 0xffff;
+                    REQUIRE(r < parts && r != t && l >= m.head[r].nown && l < m.head[r].nown + m.head[r].nghost);
+                    REQUIRE(m.lid[m.head[r].lid + l] == m.lid[h.lid + i] && targets.insert(to).second);
+                }
+        }
+        REQUIRE(targets.size() == ghosts);
+    }
     vbd::tile_groups(&p, L, W, off.data());
     REQUIRE((int)p.head.size() == P && p.max_local <= vbd::kTileMaxLocal);
     // local ids
@@ -227,6 +257,6 @@ int main(int argc, char** argv) {
         }
     }
     std::printf("ok %d vertices %d tiles max_local %d chunks %d (%.2f of the records)\n", N, P, p.max_local, nch,
-                nch * 64.0 / std::max(1, off[nfree]));
+                nch * (double)vbd::kTileChunk / std::max(1, off[nfree]));
     return 0;
 }

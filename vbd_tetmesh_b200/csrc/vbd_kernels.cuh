@@ -598,7 +598,7 @@ __device__ __forceinline__ void vertex_update(const SweepParams& p, int v, int l
 // the new position, or xi where |det H| <= 1e-8 (counted in status); block_solve also flags a
 // non-finite result.
 __device__ __forceinline__ float4 block_update(const Acc& acc, float4 xi, float4 yi, float dtsr,
-                                               unsigned long long* status) {
+                                               unsigned long long* status, bool count = true) {
     const float cm = yi.w * dtsr;
     const float H00 = cm + acc.h00, H01 = acc.h01, H02 = acc.h02;
     const float H11 = cm + acc.h11, H12 = acc.h12, H22 = cm + acc.h22;
@@ -619,7 +619,7 @@ __device__ __forceinline__ float4 block_update(const Acc& acc, float4 xi, float4
         xn.x = xi.x + inv * (A00 * f0 + A01 * f1 + A02 * f2);
         xn.y = xi.y + inv * (A01 * f0 + A11 * f1 + A12 * f2);
         xn.z = xi.z + inv * (A02 * f0 + A12 * f1 + A22 * f2);
-    } else {
+    } else if (count) {
         atomicAdd(status + ST_SINGULAR, 1ull);
     }
     return xn;
@@ -1002,9 +1002,6 @@ struct PersistParams {
     int init_from_inertia;    // start from x = y
     int expected_blocks;      // arrivals the barrier waits for (gridDim.x in normal use)
     float h, hgx, hgy, hgz;
-    // the cluster walk with resident element data: per CTA at most srec_records records and
-    // srec_owned vertices, srec_slices (colour, round) slices
-    int srec_records, srec_owned, srec_slices;
 };
 
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {

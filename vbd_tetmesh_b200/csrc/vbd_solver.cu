@@ -107,9 +107,8 @@ static SweepFn pick_sweep(int lanes, int layout, int prefetch, bool cache) {
     }
 }
 
-// The cluster walk reads the factored records (layouts 3 and 4), from L2 or resident in shared memory.
-template <int L> static void (*pick_cluster(int layout, bool resident))(PersistParams) {
-    if (resident) return layout == 3 ? &k_cluster_walk_srec<L, 3> : &k_cluster_walk_srec<L, 4>;
+// The cluster walk with whole-mesh copies reads the factored records (layouts 3 and 4) from L2.
+template <int L> static void (*pick_cluster(int layout))(PersistParams) {
     return layout == 3 ? &k_cluster_walk<L, 3> : &k_cluster_walk<L, 4>;
 }
 
@@ -118,13 +117,48 @@ template <int L> static void (*pick_cluster_adjoint(int layout))(AdjWalkParams) 
 }
 
 // The tile walk runs lanes / 2 threads per vertex; it reads its own record chunks, packed from the
-// factored records of either layout.
-template <bool ADJ, int W> static void (*pick_tile(int lanes))(TileParams) {
-    return lanes == 4 ? &k_tile_walk<2, ADJ, W> : lanes == 8 ? &k_tile_walk<4, ADJ, W> : &k_tile_walk<8, ADJ, W>;
+// factored records of either layout.  With `cluster` the tiles are the CTAs of one cluster.
+template <bool ADJ> static void (*pick_tile(int lanes, int warps, bool cluster))(TileParams) {  // ADJ: 8 warps
+    if (cluster)
+        return lanes == 4    ? &k_tile_walk<2, ADJ, 8, true>
+               : lanes == 8  ? &k_tile_walk<4, ADJ, 8, true>
+               : lanes == 16 ? &k_tile_walk<8, ADJ, 8, true>
+                             : &k_tile_walk<16, ADJ, 8, true>;
+    if (ADJ || warps == 8)
+        return lanes == 4 ? &k_tile_walk<2, ADJ, 8> : lanes == 8 ? &k_tile_walk<4, ADJ, 8> : &k_tile_walk<8, ADJ, 8>;
+    return lanes == 4   ? &k_tile_walk<2, false, 16>
+           : lanes == 8 ? &k_tile_walk<4, false, 16>
+                        : &k_tile_walk<8, false, 16>;
 }
-template <bool ADJ> static void (*pick_tile(int lanes, int warps))(TileParams) {
-    return warps == 8 ? pick_tile<ADJ, 8>(lanes) : pick_tile<ADJ, 16>(lanes);
-}
+
+// A tile plan on the device.
+struct TileSet {
+    TilePlan plan;
+    bool cluster = false;     // the tiles are the CTAs of one cluster
+    bool dirty = true;        // the chunks must be packed again (new records)
+    int layout = 0;           // layout they were packed from
+    int lanes = 0;            // lanes the device lists are for
+    // One allocation: the exchanged words and the start counter, the record chunks, the plan's lists.
+    DBuf<float4> mem;
+    float4 *words = nullptr, *chunk = nullptr;
+    int* lists = nullptr;
+    size_t nwords = 0;
+    enum { HEAD, GROUPS, WCOL, WSTREAM, TABLE, LID, GHOST, VTILE, VLOCAL, TARGET_OFF, TARGET, COUNT };
+    size_t at[COUNT + 1] = {};
+    const int* ints(int which) const { return lists + at[which]; }
+    unsigned long long started = 0;  // CTAs of all launches so far
+    unsigned tag = 1;                // next unused word tag
+    int stride = 1;                  // of the exchanged words
+    // cluster form: the forward and adjoint launches checked to fit the device, and the answers
+    const void* checked[2] = {nullptr, nullptr};
+    bool resident[2] = {false, false};
+    void reset(TilePlan&& p) {
+        plan = std::move(p);
+        dirty = true;
+        lanes = 0;
+        checked[0] = checked[1] = nullptr;
+    }
+};
 
 template <int L> static void (*pick_persistent(int layout))(PersistParams) {
     switch (layout) {
@@ -232,12 +266,7 @@ struct vbd_solver {
     // cluster holding the positions in shared memory (meshes of up to about 7,000 vertices)
     int persistent = 0;
     int cluster_ctas_opt = 0;                       // CTAs of the cluster walk (0 = from the colour sizes)
-    int cluster_resident = 1;  // the walk keeps each CTA's element records in shared memory where they fit
-    // the resident walk's plan for the mesh, kernel and CTA count it was made for
-    int sr_gen = -1, sr_ctas = 0, sr_records = 0, sr_owned = 0, sr_slices = 0;
-    const void* sr_fn = nullptr;
-    unsigned long long sr_smem = 0;
-    bool sr_ok = false;
+    int cluster_resident = 1;  // the cluster's CTAs hold a tile each and its records, not the whole mesh
     // launch shape resolved for the mesh, the kernel and the requested CTAs (the kernel's shared-memory
     // and cluster-size attributes are set per kernel)
     int cl_ctas = 0, cl_block = 0, cl_gen = -1, cl_req = 0;
@@ -280,20 +309,12 @@ struct vbd_solver {
     int adj_cur = 0;  // which of adj_lam / adj_lam2 holds lam
     // the tile walk (vbd_tile.cuh): its plan for the mesh, whether it runs in place of the captured
     // graph (chosen at init or by the autotuner, off once VBD_OPT_PERSISTENT is set), and its device data
-    vbd::TilePlan tplan;
+    vbd::TileSet tset;   // one tile per SM, exchanging words through L2
+    vbd::TileSet aset;   // tset's tiles swept by 8 warps, for the adjoint where tset has 16
+    vbd::TileSet cset;   // one tile per CTA of a cluster, its plan merged from tset's tiles
     int tile_walk = 0;
     bool persistent_set = false;
-    bool tile_dirty = true;     // chunks must be packed again (new records)
-    int tile_layout = 0;        // layout the chunks were packed from
-    int tile_lanes = 0;         // lanes the device data is for
     std::vector<int32_t> batch_mesh;  // mesh of each vertex, set by vbd_solver_init_batch for its init
-    vbd::DBuf<float4> t_chunk, t_words;  // t_words: 4 N exchanged words, then the start counter
-    vbd::DBuf<int> t_lists;              // the plan's lists, one after the other (tile_list offsets)
-    enum { TL_HEAD, TL_GROUPS, TL_WCOL, TL_WSTREAM, TL_TABLE, TL_LID, TL_GHOST, TL_VTILE, TL_VLOCAL, TL_COUNT };
-    size_t tile_list[TL_COUNT + 1] = {};
-    const int* tile_ints(int which) const { return t_lists.p + tile_list[which]; }
-    unsigned long long t_started = 0;   // CTAs of all tile launches so far
-    unsigned t_tag = 1;                 // next unused word tag
     int sm_count = 0, smem_optin = 0;
     long long launches = 0;
     std::vector<vbd::GraphEntry> graphs;
@@ -654,14 +675,23 @@ struct vbd_solver {
         return (int)std::max<long long>(1, std::min<long long>(16, (need + block - 1) / block));
     }
 
+    // Lets a kernel be launched with all the shared memory of a CTA.  The attribute belongs to the kernel, not to
+    // the handle: every handle sets the same value, so that threads cannot undo each other's.
+    cudaError_t allow_shared(const void* fn, bool cluster) const {
+        cudaFuncAttributes fa;
+        cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     smem_optin - (int)fa.sharedSizeBytes);
+        if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return e;
+    }
+
     template <class Params>
     int cluster_ctas_for(void (*fn)(Params), int L, size_t smem, int* out) {
         const int block = vbd::kClusterMaxBlock;
         int ctas = cluster_ctas_opt > 0 ? cluster_ctas_opt : cluster_auto_ctas(L);
-        CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                      1));
+        CUDA_TRY(allow_shared(reinterpret_cast<const void*>(fn), true));
         for (; ctas >= 1; --ctas) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(ctas);
@@ -788,90 +818,26 @@ struct vbd_solver {
         return check_launch();
     }
 
-    // Per-CTA sizes of the resident walk for L lanes and `ctas` CTAs of kClusterMaxBlock threads: the
-    // (colour, round) slices, and the most records and vertices any CTA sweeps (the kernel derives
-    // the same plan, k_cluster_walk_srec).
-    void srec_plan(int L, int ctas, int* records, int* owned, int* slices) const {
-        const int gpc = vbd::kClusterMaxBlock / L, G = ctas * gpc;
-        int S = 0, rec_max = 0, own_max = 0;
-        for (int c = 0; c < C; ++c) S += (cstart[c + 1] - cstart[c] + G - 1) / G;
-        for (int k = 0; k < ctas; ++k) {
-            long long rec = 0, own = 0;
-            for (int c = 0; c < C; ++c) {
-                const int vb = cstart[c], ve = cstart[c + 1];
-                for (int r = 0; r * G < ve - vb; ++r) {
-                    const int vf = vb + r * G + k * gpc;
-                    const int cnt = std::max(0, std::min(vf + gpc, ve) - vf);
-                    own += cnt;
-                    if (cnt) rec += h_inc_off[vf + cnt] - h_inc_off[vf];
-                }
-            }
-            rec_max = (int)std::max<long long>(rec_max, rec);
-            own_max = (int)std::max<long long>(own_max, own);
-        }
-        *records = rec_max;
-        *owned = own_max;
-        *slices = S;
-    }
-
-    // A sub-step (predict and finish) or a solve as one cluster launch: vbd::k_cluster_walk_srec where
-    // the CTAs' element data fits in shared memory (and VBD_OPT_CLUSTER_RESIDENT allows it), else
-    // vbd::k_cluster_walk.
+    // A sub-step (predict and finish) or a solve as one cluster launch: the tile walk of one cluster where it
+    // fits (and VBD_OPT_CLUSTER_RESIDENT allows it), else vbd::k_cluster_walk.
     int launch_cluster(int iters, float dtsr, bool accel, float rho, bool predict, bool finish, bool from_inertia,
                        float h, const float* hg) {
         const char* why = nullptr;
         if (!cluster_fit(&why)) VBD_FAIL(VBD_ERR_INVALID_ARG, "%s", why);
         VBD_TRY(upload_schedule(iters, accel, rho));
         const int L = lanes < 4 ? 4 : lanes;
+        if (cluster_resident && cluster_tiles(L, false))
+            return launch_tile(cset, iters, dtsr, accel, rho, from_inertia, h, predict ? hg : nullptr, false);
         void (*fn)(vbd::PersistParams) = nullptr;
-        void (*fn_res)(vbd::PersistParams) = nullptr;
         switch (L) {
-            case 4: fn = vbd::pick_cluster<4>(layout, false); fn_res = vbd::pick_cluster<4>(layout, true); break;
-            case 8: fn = vbd::pick_cluster<8>(layout, false); fn_res = vbd::pick_cluster<8>(layout, true); break;
-            case 16: fn = vbd::pick_cluster<16>(layout, false); fn_res = vbd::pick_cluster<16>(layout, true); break;
-            default: fn = vbd::pick_cluster<32>(layout, false); fn_res = vbd::pick_cluster<32>(layout, true); break;
+            case 4: fn = vbd::pick_cluster<4>(layout); break;
+            case 8: fn = vbd::pick_cluster<8>(layout); break;
+            case 16: fn = vbd::pick_cluster<16>(layout); break;
+            default: fn = vbd::pick_cluster<32>(layout); break;
         }
         VBD_TRY(resolve_cluster(fn, L));
         vbd::PersistParams w = walk_params(iters, dtsr, accel, predict, finish, from_inertia, h, hg);
-        size_t smem = cluster_smem();
-        if (cluster_resident) {
-            const void* f = reinterpret_cast<const void*>(fn_res);
-            if (!(sr_gen == shape_gen && sr_fn == f && sr_ctas == cl_ctas)) {
-                sr_gen = shape_gen;
-                sr_fn = f;
-                sr_ctas = cl_ctas;
-                sr_ok = false;
-                srec_plan(L, cl_ctas, &sr_records, &sr_owned, &sr_slices);
-                sr_smem = vbd::srec_layout(N, sr_records, sr_owned, sr_slices, C, layout).total;
-                int optin = 0;
-                CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-                if (sr_smem + 64 <= (unsigned long long)optin) {
-                    CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr_smem));
-                    CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-                    cudaLaunchConfig_t q = {};
-                    q.gridDim = dim3(cl_ctas);
-                    q.blockDim = dim3(cl_block);
-                    q.dynamicSmemBytes = (size_t)sr_smem;
-                    cudaLaunchAttribute qa[1];
-                    qa[0].id = cudaLaunchAttributeClusterDimension;
-                    qa[0].val.clusterDim.x = cl_ctas;
-                    qa[0].val.clusterDim.y = 1;
-                    qa[0].val.clusterDim.z = 1;
-                    q.attrs = qa;
-                    q.numAttrs = 1;
-                    int clusters = 0;
-                    sr_ok = cudaOccupancyMaxActiveClusters(&clusters, fn_res, &q) == cudaSuccess && clusters >= 1;
-                    (void)cudaGetLastError();
-                }
-            }
-            if (sr_ok) {
-                fn = fn_res;
-                smem = (size_t)sr_smem;
-                w.srec_records = sr_records;
-                w.srec_owned = sr_owned;
-                w.srec_slices = sr_slices;
-            }
-        }
+        const size_t smem = cluster_smem();
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(cl_ctas);
         cfg.blockDim = dim3(cl_block);
@@ -895,26 +861,36 @@ struct vbd_solver {
         return launch_persistent(iters, dtsr, accel, rho, predict, finish, from_inertia, h, hg);
     }
 
-    // Chunks per warp ring of a tile launch whose CTAs hold `vectors` local vectors.
-    int tile_ring(int warps, int vectors) const {
-        const long long fixed =
-            (long long)vbd::tile_smem(warps, 0, tplan.max_local, tplan.max_ids, tplan.max_groups, C, vectors) + 10240;
-        return (int)std::min<long long>(vbd::kTileMaxRing, (smem_optin - fixed) / (warps * vbd::kTileChunkBytes));
+    // Shared memory a tile launch whose CTAs hold `vectors` local vectors leaves for record chunks.
+    int tile_chunk_room(const vbd::TileSet& s, int vectors) const {
+        const long long fixed = (long long)vbd::tile_smem(s.plan.warps, 0, s.plan, C, vectors, s.cluster) + 10240;
+        return (int)std::max<long long>(0, (smem_optin - fixed) / vbd::kTileChunkBytes);
     }
-    // The kernel of 8 warps needs room for two groups' chunks where it can be had, for one at least; that of
-    // 16 warps for two chunks.
-    bool tile_fits(int vectors) const {
-        return tile_ring(tplan.warps, vectors) >= (tplan.warps == 8 ? tplan.max_rounds : 2);
+    // Chunks per warp ring.
+    int tile_ring(const vbd::TileSet& s, int vectors) const {
+        return std::min(vbd::kTileMaxRing, tile_chunk_room(s, vectors) / s.plan.warps);
+    }
+    // Whether every chunk of every tile stays in shared memory (the kernel of 8 warps).
+    bool tile_resident(const vbd::TileSet& s, int vectors) const {
+        return s.plan.warps == 8 && s.plan.max_chunks <= tile_chunk_room(s, vectors);
+    }
+    int tile_ring_chunks(const vbd::TileSet& s, int vectors) const {
+        return tile_resident(s, vectors) ? s.plan.max_chunks : s.plan.warps * tile_ring(s, vectors);
+    }
+    // The kernel of 8 warps holds a group's chunks at once, that of 16 warps two chunks at least.
+    bool tile_fits(const vbd::TileSet& s, int vectors) const {
+        return s.plan.max_local <= vbd::kTileMaxLocal &&
+               (tile_resident(s, vectors) || tile_ring(s, vectors) >= (s.plan.warps == 8 ? s.plan.max_rounds : 2));
     }
     // Warps of the tile CTAs for the current lanes.
     int tile_warps() const {
-        const double groups = (double)nfree / std::max(1, C) / std::max(1, tplan.P) * lanes / vbd::kTileChunk;
+        const double groups = (double)nfree / std::max(1, C) / std::max(1, tset.plan.P) * lanes / vbd::kTileChunk;
         return groups <= vbd::kTileFewGroups && (max_valence + lanes - 1) / lanes <= vbd::kTileMaxRing / 2 ? 8 : 16;
     }
     // Whether steps and solves run as tile walks.  Under a caller's stream capture they do not: each
     // launch needs tags of its own, which a replayed launch would repeat.
     bool use_tile() {
-        if (!tile_walk || tplan.P == 0 || semantics || timing || !use_graph || persistent || !colour_lanes.empty() ||
+        if (!tile_walk || tset.plan.P == 0 || semantics || timing || !use_graph || persistent || !colour_lanes.empty() ||
             layout < 3 || (lanes != 4 && lanes != 8 && lanes != 16) || ninc == 0)
             return false;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -923,48 +899,113 @@ struct vbd_solver {
             return false;
         }
         if (cs != cudaStreamCaptureStatusNone) return false;
-        if (tplan.lanes != lanes) vbd::tile_groups(&tplan, lanes, tile_warps(), h_inc_off.data());
-        return tile_fits(1);
+        if (tset.plan.lanes != lanes) vbd::tile_groups(&tset.plan, lanes, tile_warps(), h_inc_off.data());
+        return tile_fits(tset, 1);
+    }
+    // The adjoint's tiles: its kernel takes more than the 128 registers of 16 warps (with them it spills: 5.2 us
+    // a colour against 4.2 with 8 warps for the adjoint of 64 beams).
+    vbd::TileSet& adjoint_tiles() {
+        if (tset.plan.warps == 8) return tset;
+        if (aset.plan.lanes != lanes) {
+            vbd::TilePlan q = tset.plan;
+            vbd::tile_groups(&q, lanes, 8, h_inc_off.data());
+            aset.reset(std::move(q));
+        }
+        return aset;
     }
 
-    // The plan's lane-dependent part and the record chunks, made when first needed for the current lanes,
-    // layout and materials.
-    int ensure_tile() {
-        if (tile_lanes != lanes) {
+    // Plans the tiles of one cluster for L lanes and checks that a launch of the walk (or of its adjoint) can
+    // be resident.
+    bool cluster_tiles(int L, bool adjoint) {
+        if (tset.plan.P == 0 || C > vbd::kTileMaxColours || layout < 3) return false;
+        const int P = std::min({16, tset.plan.P, cluster_ctas_opt > 0 ? cluster_ctas_opt : std::max(1, nfree / vbd::kClusterTileMin)});
+        if (cset.plan.P != P || cset.plan.lanes != L) {
+            vbd::TilePlan q;
+            vbd::tile_merge(tset.plan, P, cstart, &q);
+            vbd::tile_groups(&q, L, 8, h_inc_off.data());
+            cset.reset(std::move(q));
+            cset.cluster = true;
+        }
+        const int which = adjoint ? 1 : 0, vectors = adjoint ? 3 : 2;
+        if (!tile_fits(cset, vectors)) return false;
+        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<true>(L, 8, true)
+                                                              : vbd::pick_tile<false>(L, 8, true));
+        if (cset.checked[which] != f) {
+            cset.checked[which] = f;
+            cset.resident[which] = false;
+            const size_t smem = vbd::tile_smem(8, tile_ring_chunks(cset, vectors), cset.plan, C, vectors, true);
+            if (allow_shared(f, true) == cudaSuccess) {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute attr[1];
+                cluster_config(&cfg, attr, P, 256, smem);
+                int clusters = 0;
+                cset.resident[which] = cudaOccupancyMaxActiveClusters(&clusters, f, &cfg) == cudaSuccess && clusters >= 1;
+            }
+            (void)cudaGetLastError();
+        }
+        return cset.resident[which];
+    }
+    // The automatic CTA count of VBD_OPT_CLUSTER_CTAS.
+    int cluster_auto(int L) { return cluster_resident && cluster_tiles(L, false) ? cset.plan.P : cluster_auto_ctas(L); }
+    void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int ctas, int threads, size_t smem) const {
+        cfg->gridDim = dim3(ctas);
+        cfg->blockDim = dim3(threads);
+        cfg->dynamicSmemBytes = smem;
+        cfg->stream = stream;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ctas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg->attrs = attr;
+        cfg->numAttrs = 1;
+    }
+
+    // The plan's lists and the record chunks on the device, made when first needed for the current lanes, layout
+    // and materials.
+    int ensure_tile(vbd::TileSet& s) {
+        vbd::TilePlan& q = s.plan;
+        if (s.lanes != q.lanes) {
             const struct {
                 const void* p;
                 size_t ints;
-            } lists[TL_COUNT] = {
-                {tplan.head.data(), tplan.head.size() * sizeof(vbd::TileHead) / 4},
-                {tplan.groups.data(), tplan.groups.size() * sizeof(vbd::TileGroup) / 4},
-                {tplan.wcol.data(), tplan.wcol.size()},
-                {tplan.wstream.data(), tplan.wstream.size()},
-                {tplan.chunk.data(), tplan.chunk.size()},
-                {tplan.lid.data(), tplan.lid.size()},
-                {tplan.ghost.data(), tplan.ghost.size()},
-                {tplan.vtile.data(), tplan.vtile.size()},
-                {tplan.vlocal.data(), tplan.vlocal.size()},
+            } lists[vbd::TileSet::COUNT] = {
+                {q.head.data(), q.head.size() * sizeof(vbd::TileHead) / 4},
+                {q.groups.data(), q.groups.size() * sizeof(vbd::TileGroup) / 4},
+                {q.wcol.data(), q.wcol.size()},
+                {q.wstream.data(), q.wstream.size()},
+                {q.chunk.data(), q.chunk.size()},
+                {q.lid.data(), q.lid.size()},
+                {q.ghost.data(), q.ghost.size()},
+                {q.vtile.data(), q.vtile.size()},
+                {q.vlocal.data(), q.vlocal.size()},
+                {q.target_off.data(), q.target_off.size()},
+                {q.target.data(), q.target.size()},
             };
-            for (int k = 0; k < TL_COUNT; ++k) tile_list[k + 1] = tile_list[k] + (lists[k].ints + 3) / 4 * 4;
-            std::vector<int> all(tile_list[TL_COUNT]);
-            for (int k = 0; k < TL_COUNT; ++k)
-                if (lists[k].ints) std::memcpy(all.data() + tile_list[k], lists[k].p, 4 * lists[k].ints);
-            if (t_lists.n < all.size()) VBD_TRY(t_lists.alloc(all.size()));
-            CUDA_TRY(cudaMemcpyAsync(t_lists.p, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, stream));
-            if (t_words.n != 4 * (size_t)N + 1) {
-                VBD_TRY(t_words.alloc(4 * (size_t)N + 1));
-                CUDA_TRY(cudaMemsetAsync(t_words.p, 0, sizeof(float4) * t_words.n, stream));
-                t_started = 0;
-                t_tag = 1;
+            for (int k = 0; k < vbd::TileSet::COUNT; ++k) s.at[k + 1] = s.at[k] + (lists[k].ints + 3) / 4 * 4;
+            std::vector<int> all(s.at[vbd::TileSet::COUNT]);
+            for (int k = 0; k < vbd::TileSet::COUNT; ++k)
+                if (lists[k].ints) std::memcpy(all.data() + s.at[k], lists[k].p, 4 * lists[k].ints);
+            s.stride = nfree <= (long long)vbd::kTileSpreadWords * q.P ? 8 : 1;
+            s.nwords = s.cluster ? 0 : 4 * (size_t)s.stride * N + 1;
+            const size_t nchunk = q.chunk.size() / 3 * (vbd::kTileChunkBytes / 16);
+            const size_t need = s.nwords + nchunk + all.size() / 4;
+            if (s.mem.n < need) {
+                if (s.cluster) drop_graphs();  // the adjoint's captured launches hold the addresses
+                VBD_TRY(s.mem.alloc(need));
             }
-            const size_t n4 = tplan.chunk.size() / 3 * (vbd::kTileChunkBytes / 16);
-            if (t_chunk.n != n4) VBD_TRY(t_chunk.alloc(n4));
+            s.words = s.mem.p;
+            s.chunk = s.words + s.nwords;
+            s.lists = reinterpret_cast<int*>(s.chunk + nchunk);
+            CUDA_TRY(cudaMemcpyAsync(s.lists, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, stream));
+            if (s.nwords) CUDA_TRY(cudaMemsetAsync(s.words, 0, sizeof(float4) * s.nwords, stream));
+            s.started = 0;
+            s.tag = 1;
             CUDA_TRY(cudaStreamSynchronize(stream));  // the host lists may change after this
-            tile_dirty = true;
-            tile_lanes = lanes;
+            s.dirty = true;
+            s.lanes = q.lanes;
         }
-        if (tile_dirty || tile_layout != layout) {
-            const int nch = (int)(tplan.chunk.size() / 3);
+        if (s.dirty || s.layout != layout) {
+            const int nch = (int)(q.chunk.size() / 3);
             vbd::SweepParams p{};
             p.inc_off = inc_off.p;
             p.crec = crec.p;
@@ -972,77 +1013,98 @@ struct vbd_solver {
             if (nch > 0) {
                 const unsigned grid = vbd::nblk((long long)nch * 32, 256);
                 auto fn = layout == 3 ? &vbd::k_pack_tile<3> : &vbd::k_pack_tile<4>;
-                fn<<<grid, 256, 0, stream>>>(p, tile_ints(TL_TABLE), nch, lanes,
-                                             reinterpret_cast<const vbd::TileGroup*>(tile_ints(TL_GROUPS)),
-                                             reinterpret_cast<const vbd::TileHead*>(tile_ints(TL_HEAD)), tile_ints(TL_LID),
-                                             tile_ints(TL_VTILE), tile_ints(TL_VLOCAL), nfree, t_chunk.p);
+                fn<<<grid, 256, 0, stream>>>(p, s.ints(vbd::TileSet::TABLE), nch, q.lanes,
+                                             reinterpret_cast<const vbd::TileGroup*>(s.ints(vbd::TileSet::GROUPS)),
+                                             reinterpret_cast<const vbd::TileHead*>(s.ints(vbd::TileSet::HEAD)),
+                                             s.ints(vbd::TileSet::LID), s.ints(vbd::TileSet::VTILE),
+                                             s.ints(vbd::TileSet::VLOCAL), nfree, s.chunk);
                 VBD_TRY(check_launch());
             }
-            tile_dirty = false;
-            tile_layout = layout;
+            s.dirty = false;
+            s.layout = layout;
         }
         return VBD_OK;
     }
 
-    vbd::TileParams tile_params(int k0, int k1, float dtsr, const float* omega, bool accel, int vectors) {
-        if ((unsigned long long)t_tag + (unsigned)(k1 - k0) > 0xfffffff0ull) {  // the tags start over
-            cudaMemsetAsync(t_words.p, 0, sizeof(float4) * 4 * (size_t)N, stream);
-            t_tag = 1;
-        }
+    int tile_params(vbd::TileSet& s, int k0, int k1, float dtsr, const float* omega, bool accel, int vectors,
+                    vbd::TileParams* out) {
+        using S = vbd::TileSet;
+        const vbd::TilePlan& q = s.plan;
         vbd::TileParams w{};
-        w.chunk = t_chunk.p;
-        w.head = reinterpret_cast<const vbd::TileHead*>(tile_ints(TL_HEAD));
-        w.lid = tile_ints(TL_LID);
-        w.groups = reinterpret_cast<const vbd::TileGroup*>(tile_ints(TL_GROUPS));
-        w.wcol = tile_ints(TL_WCOL);
-        w.ghost = tile_ints(TL_GHOST);
-        w.wstream = reinterpret_cast<const int2*>(tile_ints(TL_WSTREAM));
-        w.words = t_words.p;
-        w.arrived = reinterpret_cast<unsigned long long*>(t_words.p + 4 * (size_t)N);
-        w.arrived_target = (t_started += (unsigned)tplan.P);
+        if (!s.cluster) {
+            if ((unsigned long long)s.tag + (unsigned)(k1 - k0) > 0xfffffff0ull) {  // the tags start over
+                CUDA_TRY(cudaMemsetAsync(s.words, 0, sizeof(float4) * (s.nwords - 1), stream));
+                s.tag = 1;
+            }
+            w.words = s.words;
+            w.word_stride = s.stride;
+            w.arrived = reinterpret_cast<unsigned long long*>(s.words + s.nwords - 1);
+            w.arrived_target = (s.started += (unsigned)q.P);
+            w.tag = s.tag - (unsigned)k0;
+            s.tag += (unsigned)(k1 - k0);
+        }
+        w.chunk = s.chunk;
+        w.head = reinterpret_cast<const vbd::TileHead*>(s.ints(S::HEAD));
+        w.lid = s.ints(S::LID);
+        w.groups = reinterpret_cast<const vbd::TileGroup*>(s.ints(S::GROUPS));
+        w.wcol = s.ints(S::WCOL);
+        w.ghost = s.ints(S::GHOST);
+        w.wstream = reinterpret_cast<const int2*>(s.ints(S::WSTREAM));
+        w.target_off = s.ints(S::TARGET_OFF);
+        w.target = s.ints(S::TARGET);
+        w.max_own = q.max_own;
+        w.max_target = q.max_target;
         w.status = status.p;
         w.omega = omega;
-        w.tag = t_tag - (unsigned)k0;
-        t_tag += (unsigned)(k1 - k0);
         w.n = N;
         w.nfree = nfree;
         w.ncol = C;
         w.k0 = k0;
         w.k1 = k1;
-        w.ring = tile_ring(tplan.warps, vectors);
-        w.max_local = tplan.max_local;
-        w.max_ids = tplan.max_ids;
-        w.max_groups = tplan.max_groups;
-        w.max_rounds = tplan.max_rounds;
+        w.ring = tile_ring(s, vectors);
+        w.resident = tile_resident(s, vectors);
+        w.ring_chunks = tile_ring_chunks(s, vectors);
+        w.max_local = q.max_local;
+        w.max_ids = q.max_ids;
+        w.max_groups = q.max_groups;
+        w.max_rounds = q.max_rounds;
         w.dtsr = dtsr;
         w.keep_pp = accel ? 1 : 0;
         w.y = y.p;
-        return w;
+        *out = w;
+        return VBD_OK;
     }
 
-    int tile_launch(void (*fn)(vbd::TileParams), vbd::TileParams& w, int vectors) {
-        const size_t smem = vbd::tile_smem(tplan.warps, w.ring, w.max_local, w.max_ids, w.max_groups, C, vectors);
-        CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    int tile_launch(const vbd::TileSet& s, void (*fn)(vbd::TileParams), vbd::TileParams& w, int vectors) {
+        const size_t smem = vbd::tile_smem(s.plan.warps, w.ring_chunks, s.plan, C, vectors, s.cluster);
+        CUDA_TRY(allow_shared(reinterpret_cast<const void*>(fn), s.cluster));
+        if (s.cluster) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            cluster_config(&cfg, attr, s.plan.P, 32 * s.plan.warps, smem);
+            CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, w));
+            return check_launch();
+        }
         void* args[] = {&w};
-        CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(tplan.P), dim3(32 * tplan.warps), args,
+        CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(s.plan.P), dim3(32 * s.plan.warps), args,
                                              smem, stream));
         return check_launch();
     }
 
     // A sub-step (hg given: predictor and velocity update) or a solve as tile walks: one launch, or one
     // per energy evaluation with an energy history (emit_iterations' schedule).
-    int launch_tile(int iters, float dtsr, bool accel, float rho, bool from_inertia, float h, const float* hg,
-                    bool record_energy) {
+    int launch_tile(vbd::TileSet& s, int iters, float dtsr, bool accel, float rho, bool from_inertia, float h,
+                    const float* hg, bool record_energy) {
         VBD_TRY(upload_schedule(iters, accel, rho));
-        VBD_TRY(ensure_tile());
+        VBD_TRY(ensure_tile(s));
         int k0 = 0;
         do {
             int k1 = iters;
             if (record_energy) k1 = std::min(iters, k0 == 0 ? 1 : k0 + energy_every);
             // both position buffers in shared memory where that leaves the rings their depth
-            const int two = accel && tile_ring(tplan.warps, 2) >= vbd::kTileTwoRing;
-            vbd::TileParams w = tile_params(k0, k1, dtsr, d_omega.p, accel, 1 + two);
+            const int two = s.cluster || (accel && (tile_resident(s, 2) || (!tile_resident(s, 1) && tile_ring(s, 2) >= vbd::kTileTwoRing)));
+            vbd::TileParams w;
+            VBD_TRY(tile_params(s, k0, k1, dtsr, d_omega.p, accel, 1 + two, &w));
             w.two = two;
             w.x0 = x0.p;
             w.x1 = x1.p;
@@ -1058,7 +1120,7 @@ struct vbd_solver {
                 w.hgy = hg[1];
                 w.hgz = hg[2];
             }
-            VBD_TRY(tile_launch(vbd::pick_tile<false>(lanes, tplan.warps), w, 1 + two));
+            VBD_TRY(tile_launch(s, vbd::pick_tile<false>(s.plan.lanes, s.plan.warps, s.cluster), w, 1 + two));
             if (record_energy && k1 > k0 && (k1 - 1) % energy_every == 0) VBD_TRY(emit_energy_append(x0.p));
             k0 = k1;
         } while (k0 < iters);
@@ -1101,7 +1163,7 @@ struct vbd_solver {
         key.rho = t.rho;
         if (persistent && !timing)
             return launch_walk(t.iters, t.dtsr, t.accel != 0, t.rho, true, true, false, t.h, t.hg);
-        if (use_tile()) return launch_tile(t.iters, t.dtsr, t.accel != 0, t.rho, false, t.h, t.hg, false);
+        if (use_tile()) return launch_tile(tset, t.iters, t.dtsr, t.accel != 0, t.rho, false, t.h, t.hg, false);
         return run(key, [&] { return emit_substep(t.h, t.dtsr, t.hg, t.iters, t.accel != 0, t.rho); });
     }
 
@@ -1110,7 +1172,7 @@ struct vbd_solver {
     // getAcceleratorOmega(k, rho) (rho = 0: plain Gauss-Seidel), then the parameter gradients, the
     // pinned-vertex coupling and the step's adjoint update.
     int emit_adjoint_substep(const TapeStep& t, const float4* X, int sweeps, float rho,
-                             void (*walk)(vbd::AdjWalkParams) = nullptr, bool tile = false) {
+                             void (*walk)(vbd::AdjWalkParams) = nullptr, vbd::TileSet* tile = nullptr) {
         const float c = 0.999f / t.h;
         const int L = lanes < 4 ? 4 : lanes;
         vbd::k_adj_rhs<<<vbd::nblk(std::max(nfree, 1), 256), 256, 0, stream>>>(adj_ax.p, adj_av.p, adj_G.p, c, nfree);
@@ -1127,7 +1189,9 @@ struct vbd_solver {
             }
         }
         if (tile) {
-            vbd::TileParams w = tile_params(0, sweeps, t.dtsr, d_adj_omega.p, accel, 2);
+            const int vectors = tile->cluster ? 3 : 2;
+            vbd::TileParams w;
+            VBD_TRY(tile_params(*tile, 0, sweeps, t.dtsr, d_adj_omega.p, accel, vectors, &w));
             w.X = X;
             w.G = adj_G.p;
             w.pp = adj_lpp.p;
@@ -1137,7 +1201,7 @@ struct vbd_solver {
                 if (omega > 1.0f) cur ^= 1;
             }
             w.lam_out = cur ? adj_lam2.p : adj_lam.p;
-            VBD_TRY(tile_launch(vbd::pick_tile<true>(lanes, tplan.warps), w, 2));
+            VBD_TRY(tile_launch(*tile, vbd::pick_tile<true>(tile->plan.lanes, tile->plan.warps, tile->cluster), w, vectors));
         }
         for (int it = 1; it <= sweeps && !walk && !tile; ++it) {
             bool blend = false;
@@ -1216,17 +1280,33 @@ struct vbd_solver {
         key.dtsr = t.dtsr;
         key.rho = rho;
         void (*walk)(vbd::AdjWalkParams) = nullptr;
-        if (adj_walk()) {
+        vbd::TileSet* tile = nullptr;
+        if (!adj_alternate) {
+            const bool walk_tiles = adj_walk() && cluster_resident && cluster_tiles(lanes < 4 ? 4 : lanes, true);
+            if (walk_tiles) {
+                tile = &cset;
+            } else if (use_tile()) {
+                tile = &adjoint_tiles();
+                if (!tile_fits(*tile, 2)) tile = nullptr;
+            }
+        }
+        if (tile) {
+            VBD_TRY(upload_adj_schedule(sweeps, rho));
+            VBD_TRY(ensure_tile(*tile));
+        } else if (adj_walk()) {
             VBD_TRY(prepare_adj_walk(sweeps, rho, &walk));
             key.walk = 2;
             key.block = ca_ctas;
         }
-        if (!walk && !adj_alternate && use_tile() && tile_fits(2)) {
-            VBD_TRY(upload_adj_schedule(sweeps, rho));
-            VBD_TRY(ensure_tile());
-            VBD_TRY(emit_adjoint_substep(t, X, sweeps, rho, nullptr, true));
+        // a launch that exchanges words needs tags of its own each time: no graph
+        if (tile && !tile->cluster) {
+            VBD_TRY(emit_adjoint_substep(t, X, sweeps, rho, nullptr, tile));
         } else {
-            VBD_TRY(run(key, [&] { return emit_adjoint_substep(t, X, sweeps, rho, walk); }));
+            if (tile) {
+                key.walk = 3;
+                key.block = tile->plan.P;
+            }
+            VBD_TRY(run(key, [&] { return emit_adjoint_substep(t, X, sweeps, rho, walk, tile); }));
         }
         float omega = 1.0f;
         for (int it = 1; it <= sweeps && rho > 0.0f; ++it) {
@@ -1294,7 +1374,7 @@ struct vbd_solver {
     // Captured graphs bake in buffer addresses: every (re)allocation or release of the streamed
     // record copies invalidates them.
     int repack_stream() {
-        tile_dirty = true;
+        tset.dirty = aset.dirty = cset.dirty = true;
         if (layout != 1 && irec.p) {
             drop_graphs();
             irec.release();
@@ -1480,8 +1560,12 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     {
         int free_count = 0;
         for (int i = 0; i < N; ++i) free_count += fixed[i] ? 0 : 1;
-        if (free_count >= vbd::kTileMinVertices && T > 0) {
+        if (free_count > 0 && T > 0) {
+            // one per SM, kTileVertices at least; for small meshes a multiple of 16, which the cluster's CTAs
+            // share evenly
             plan.P = std::min(s->sm_count, free_count / vbd::kTileVertices);
+            if (free_count <= vbd::kClusterMeshVertices) plan.P = std::max(16, plan.P / 16 * 16);
+            plan.P = std::max(1, std::min(plan.P, free_count));
             plan.n = N;
             plan.nfree = free_count;
             const int32_t* mesh = (int)s->batch_mesh.size() == N ? s->batch_mesh.data() : nullptr;
@@ -1567,10 +1651,10 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
         vbd::tile_lists(&plan, cstart, tile_in, bnd_in, inc_off.data(), inc_tet.data(), &rec[0].ids.x,
                         (int)(sizeof(vbd::TetRec) / sizeof(int)));
     }
-    s->tplan = std::move(plan);
-    s->t_words.release();
-    s->tile_lanes = 0;
-    s->tile_walk = !s->persistent_set && s->tplan.P > 0 && s->tplan.max_local <= vbd::kTileMaxLocal;
+    s->tset.reset(std::move(plan));
+    s->aset.reset(vbd::TilePlan());
+    s->cset.reset(vbd::TilePlan());
+    s->tile_walk = !s->persistent_set && nfree >= vbd::kTileMinVertices;
 
     std::vector<float4> hx(N), hv(N), hy(N);
     for (int i = 0; i < N; ++i) {
@@ -1608,7 +1692,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     CUDA_TRY(cudaMemcpyAsync(s->y.p, hy.data(), b4, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->perm.p, perm.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->inc_off.p, inc_off.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice, s->stream));
-    s->h_inc_off = inc_off;  // the cluster walk's resident-record plan reads it on the host
+    s->h_inc_off = inc_off;  // the tile plans read it on the host
     CUDA_TRY(cudaMemcpyAsync(s->inc_tet.p, inc_tet.data(), sizeof(int) * inc_tet.size(), cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->inc_vertex.p, inc_vertex.data(), sizeof(int) * inc_vertex.size(), cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->rec.p, rec.data(), sizeof(vbd::TetRec) * rec.size(), cudaMemcpyHostToDevice, s->stream));
@@ -1662,7 +1746,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     s->d_cstart.release();
     s->have_materials = tet_mu != nullptr;
     VBD_TRY(s->repack_stream());
-    if (s->use_tile()) VBD_TRY(s->ensure_tile());
+    if (s->use_tile()) VBD_TRY(s->ensure_tile(s->tset));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     s->ready = true;
     return VBD_OK;
@@ -1825,7 +1909,7 @@ int vbd_solver_solve(vbd_solver* s, int32_t iterations, float dt_sqr_reciprocal,
         return s->launch_walk(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, false, false,
                               init_mode == VBD_INIT_FROM_INERTIA, 1.0f, nullptr);
     if (s->use_tile())
-        return s->launch_tile(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode == VBD_INIT_FROM_INERTIA,
+        return s->launch_tile(s->tset, iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode == VBD_INIT_FROM_INERTIA,
                               1.0f, nullptr, false);
     return s->run(key, [&] { return s->emit_solve(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode); });
 }
@@ -1874,7 +1958,7 @@ int vbd_solver_step(vbd_solver* s, float dt, int32_t substeps, int32_t iteration
         if (s->persistent && !s->timing && nenergy == 0)
             VBD_TRY(s->launch_walk(iterations, dtsr, use_acceleration != 0, rho, true, true, false, h, hg));
         else if (s->use_tile())
-            VBD_TRY(s->launch_tile(iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0));
+            VBD_TRY(s->launch_tile(s->tset, iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0));
         else
             VBD_TRY(s->run(key, [&] {
                 return s->emit_substep(h, dtsr, hg, iterations, use_acceleration != 0, rho, nenergy > 0);
@@ -2152,6 +2236,10 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
             s->persistent = value;
             s->persistent_set = true;
             s->tile_walk = 0;
+            if (value == 2 && s->ready && s->cluster_resident && s->cluster_tiles(s->lanes < 4 ? 4 : s->lanes, false)) {
+                VBD_TRY(s->ensure_tile(s->cset));
+                CUDA_TRY(cudaStreamSynchronize(s->stream));
+            }
             return VBD_OK;
         case VBD_OPT_CLUSTER_CTAS:
             if (value < 0 || value > 16) VBD_FAIL(VBD_ERR_INVALID_ARG, "cluster CTAs must be 0 (automatic) to 16");
@@ -2216,7 +2304,7 @@ int vbd_solver_get_option(vbd_solver* s, int32_t option, int32_t* value) {
         case VBD_OPT_CLUSTER_RESIDENT: *value = s->cluster_resident; return VBD_OK;
         case VBD_OPT_CLUSTER_CTAS:
             *value = s->cluster_ctas_opt > 0 || !s->ready ? s->cluster_ctas_opt
-                                                           : s->cluster_auto_ctas(s->lanes < 4 ? 4 : s->lanes);
+                                                           : s->cluster_auto(s->lanes < 4 ? 4 : s->lanes);
             return VBD_OK;
         case VBD_OPT_SEMANTICS: *value = s->semantics; return VBD_OK;
         case VBD_OPT_L2_PREFETCH: *value = s->l2_prefetch; return VBD_OK;
@@ -2451,7 +2539,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
         c.colour_lanes.clear();
         rc = try_cand(c);
         // the tile walk at each lane count it runs
-        if (s->tplan.P > 0 && base.layout >= 3)
+        if (s->tset.plan.P > 0 && base.layout >= 3)
             for (int L : {4, 8, 16}) {
                 if (rc) break;
                 Cand k = base;
@@ -2482,7 +2570,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
             // the chosen walk's CTA count around the automatic one (fewer CTAs send fewer copies of
             // each update; more take fewer rounds)
             if (!rc && best.persistent == 2 && best.ctas == 0) {
-                const int a = s->cluster_auto_ctas(best.lanes < 4 ? 4 : best.lanes);
+                const int a = s->cluster_auto(best.lanes < 4 ? 4 : best.lanes);
                 const Cand walk = best;
                 for (int n : {a / 2, (3 * a) / 4, a + (a + 1) / 2, 16}) {
                     n = std::min(16, std::max(1, n));

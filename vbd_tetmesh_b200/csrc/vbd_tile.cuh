@@ -22,8 +22,8 @@
 // gathers that neighbour).
 //
 // What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
-// one SM to another's poll, 885 on average) plus one vertex's chain per colour: 1.6 to 2 us a colour
-// against 2.3 to 2.6 us a launch.  Large tiles by issue and the chunk stream: 64^3 cube 3.4 against 4.1 ms
+// one SM to another's poll, 885 on average) plus one vertex's chain per colour (about 1,000 cycles from
+// the barrier to its publication): 1.4 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by issue and the chunk stream: 64^3 cube 3.4 against 4.1 ms
 // a step of 400 colours, 4.0 TB/s of DRAM reads.
 // Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
 // records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds
@@ -44,7 +44,8 @@ struct TileParams {
     const int* wcol;            // [P][warps][C + 1]: first group of each warp and colour
     const int* ghost;           // [P][C + 1]
     const int2* wstream;        // [P][warps]
-    float4* words;              // exchanged words: [parity][n] x~, then [parity][n] blended
+    float4* words;              // exchanged words: [parity][n] x~, then [parity][n] blended, word_stride apart
+    int word_stride;
     unsigned long long* arrived;
     unsigned long long arrived_target;  // *arrived once every CTA of this launch has started
     unsigned long long* status;
@@ -53,6 +54,13 @@ struct TileParams {
     int n, nfree, ncol, k0, k1; // iterations [k0, k1) of the schedule
     int ring, max_local, max_ids, max_groups, max_rounds;
     int two;                    // both position buffers in shared memory
+    int ring_chunks;            // chunks of all the CTA's rings
+    int resident;               // W = 8: the rings hold every chunk of the tile, copied once
+    // cluster exchange: where each own vertex's results go, [own vertex] first target, then the targets
+    // (CTA rank << 16 | local id there)
+    const int* target_off;      // [P][max_own + 1]
+    const int* target;          // [P][max_target]
+    int max_own, max_target;
     float dtsr;
     int keep_pp;
     // forward: positions start and end in x0
@@ -72,13 +80,14 @@ struct TileParams {
 };
 
 // Dynamic shared memory of a CTA: the rings, the local vectors (`vectors` of them, one entry more each),
-// the groups, the internal ids of the own vertices and ghosts, the first ghost of each colour, and the
-// first group of each warp and colour.
-__host__ __device__ inline size_t tile_smem(int warps, int ring, int max_local, int max_ids, int max_groups, int ncol,
-                                            int vectors) {
-    return (size_t)warps * ring * kTileChunkBytes + 16u * (size_t)(max_local + 1) * vectors +
-           sizeof(TileGroup) * (size_t)max_groups + 4u * (size_t)max_ids + 4u * (size_t)(warps + 1) * (ncol + 1);
+// the groups, the internal ids of the own vertices and ghosts, the first ghost of each colour, the first
+// group of each warp and colour, and (cluster exchange) the own vertices' targets.
+inline size_t tile_smem(int warps, int ring_chunks, const TilePlan& p, int ncol, int vectors, bool cluster) {
+    return (size_t)ring_chunks * kTileChunkBytes + 16u * (size_t)(p.max_local + 1) * vectors +
+           sizeof(TileGroup) * (size_t)p.max_groups + 4u * (size_t)p.max_ids + 4u * (size_t)(warps + 1) * (ncol + 1) +
+           (cluster ? 4u * (size_t)(p.max_own + 1 + p.max_target) : 0u);
 }
+constexpr int kTileMaxColours = 64;  // of a cluster exchange: one mbarrier per colour
 
 // The 128-bit words: one relaxed, single-copy-atomic access each.
 __device__ __forceinline__ void word_store(float4* p, float x, float y, float z, unsigned tag) {
@@ -148,9 +157,11 @@ struct TileRing {
 };
 
 __device__ __forceinline__ void ring_issue(const TileParams& p, TileRing& r, unsigned buf, int slot, int lane) {
+    constexpr int kBytes = kTileChunkBytes;
+    static_assert(kBytes == 5 * 512 + 256, "176 pieces of 16 bytes");
     if (r.left > 0) {
-        const char* src = reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kTileChunkBytes + 16 * lane;
-        const unsigned dst = buf + (unsigned)(slot * kTileChunkBytes + 16 * lane);
+        const char* src = reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kBytes + 16 * lane;
+        const unsigned dst = buf + (unsigned)(slot * kBytes + 16 * lane);
 #pragma unroll
         for (int i = 0; i < 5; ++i)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512 * i), "l"(src + 512 * i) : "memory");
@@ -164,13 +175,14 @@ __device__ __forceinline__ void ring_issue(const TileParams& p, TileRing& r, uns
 // The same as one bulk copy, completing on the slot's mbarrier (W = 16).
 __device__ __forceinline__ void ring_issue_bulk(const TileParams& p, TileRing& r, unsigned buf, unsigned bar, int slot,
                                                 int lane) {
+    constexpr unsigned kBytes = kTileChunkBytes;
     if (r.left <= 0) return;
     if (lane == 0) {
-        mbar_expect(bar + 8u * slot, kTileChunkBytes);
+        mbar_expect(bar + 8u * slot, kBytes);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         buf + (unsigned)(slot * kTileChunkBytes)),
-                     "l"(reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kTileChunkBytes),
-                     "r"((unsigned)kTileChunkBytes), "r"(bar + 8u * slot)
+                         buf + (unsigned)(slot * kBytes)),
+                     "l"(reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kBytes),
+                     "r"(kBytes), "r"(bar + 8u * slot)
                      : "memory");
     }
     --r.left;
@@ -195,8 +207,6 @@ __device__ __forceinline__ bool ring_wait_bulk(const TileParams& p, unsigned bar
     }
     return __all_sync(0xffffffffu, done);
 }
-static_assert(kTileChunkBytes == 5 * 512 + 256, "ring_issue copies 176 pieces of 16 bytes");
-
 // Waits until at most `pending` of the newest commit groups are outstanding.
 template <int N> __device__ __forceinline__ void ring_wait_for() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
@@ -243,8 +253,9 @@ __device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.f, -1.f), 
 __device__ __forceinline__ F2 dot2(F2 a0, F2 b0, F2 a1, F2 b1, F2 a2, F2 b2) {
     return fma2(a2, b2, fma2(a0, b0, mul2(a1, b1)));
 }
-// a b - c d given nc = -c, rounded as nvcc contracts it.
-__device__ __forceinline__ F2 cross2(F2 a, F2 b, F2 nc, F2 d) { return fma2(a, b, mul2(nc, d)); }
+// a b - c d, rounded as nvcc contracts it; given nc = -c it is one instruction shorter.
+__device__ __forceinline__ F2 cross2(F2 a, F2 b, F2 c, F2 d) { return fma2(a, b, neg2(mul2(c, d))); }
+__device__ __forceinline__ F2 cross2n(F2 a, F2 b, F2 nc, F2 d) { return fma2(a, b, mul2(nc, d)); }
 
 __device__ __forceinline__ void load_if(bool pred, const float4* p, float4& v) {
     asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
@@ -293,10 +304,9 @@ struct Acc2 {
     }
 };
 
-// The geometry of two records: edge vectors d_k and the columns c_k of cof(D) (c_0 = d_1 x d_2, ...).  A
-// product a b - c d needs one negated factor; those of d_1 and d_2 serve all three columns.
+// The geometry of two records: edge vectors d_k and the columns c_k of cof(D) (c_0 = d_1 x d_2, ...).
 struct Geom2 {
-    F2 d[3][3], c[3][3], n1[3], n2[3];
+    F2 d[3][3], c[3][3];
 };
 __device__ __forceinline__ void tile_edges(const int4 id, float4 xi, const float4* X, Geom2& q) {
     const unsigned a0 = id.x, a1 = id.y, b0 = id.z, b1 = id.w;
@@ -308,17 +318,15 @@ __device__ __forceinline__ void tile_edges(const int4 id, float4 xi, const float
         q.d[k][1] = f2(pa[k].y - xi.y, pb[k].y - xi.y);
         q.d[k][2] = f2(pa[k].z - xi.z, pb[k].z - xi.z);
     }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        q.n1[i] = neg2(q.d[1][i]);
-        q.n2[i] = neg2(q.d[2][i]);
-    }
+    // the negated d_1 and d_2 serve all three columns
+    const F2 n1[3] = {neg2(q.d[1][0]), neg2(q.d[1][1]), neg2(q.d[1][2])};
+    const F2 n2[3] = {neg2(q.d[2][0]), neg2(q.d[2][1]), neg2(q.d[2][2])};
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
-        q.c[0][i] = cross2(q.d[1][i1], q.d[2][i2], q.n1[i2], q.d[2][i1]);
-        q.c[1][i] = cross2(q.d[2][i1], q.d[0][i2], q.n2[i2], q.d[0][i1]);
-        q.c[2][i] = cross2(q.d[0][i1], q.d[1][i2], q.d[0][i2], q.n1[i1]);
+        q.c[0][i] = cross2n(q.d[1][i1], q.d[2][i2], n1[i2], q.d[2][i1]);
+        q.c[1][i] = cross2n(q.d[2][i1], q.d[0][i2], n2[i2], q.d[0][i1]);
+        q.c[2][i] = cross2n(q.d[0][i1], q.d[1][i2], q.d[0][i2], n1[i1]);
     }
 }
 
@@ -351,23 +359,25 @@ __device__ __forceinline__ void tile_contrib(const TilePair& r, const int4 id, f
 }
 
 // fact_adjoint for two records at once.  A padding record reads the zero entry `zero` of L.
+__device__ __forceinline__ void tile_lambdas(const int4 id, const float4* L, int zero, F2 m[3][3]) {
+    const unsigned a0 = id.x, a1 = id.y, b0 = id.z, b1 = id.w;
+    const bool va = a1 >> 16, vb = b1 >> 16;
+    const float4 la[3] = {L[va ? a0 & 0xffffu : zero], L[va ? a0 >> 16 : zero], L[va ? a1 & 0xffffu : zero]};
+    const float4 lb[3] = {L[vb ? b0 & 0xffffu : zero], L[vb ? b0 >> 16 : zero], L[vb ? b1 & 0xffffu : zero]};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        m[k][0] = f2(la[k].x, lb[k].x);
+        m[k][1] = f2(la[k].y, lb[k].y);
+        m[k][2] = f2(la[k].z, lb[k].z);
+    }
+}
+
 __device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, float4 xi, const float4* X,
                                              const float4* L, int zero, Acc2& acc) {
     Geom2 q;
     tile_edges(id, xi, X, q);
     F2 m[3][3];
-    {
-        const unsigned a0 = id.x, a1 = id.y, b0 = id.z, b1 = id.w;
-        const bool va = a1 >> 16, vb = b1 >> 16;
-        const float4 la[3] = {L[va ? a0 & 0xffffu : zero], L[va ? a0 >> 16 : zero], L[va ? a1 & 0xffffu : zero]};
-        const float4 lb[3] = {L[vb ? b0 & 0xffffu : zero], L[vb ? b0 >> 16 : zero], L[vb ? b1 & 0xffffu : zero]};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            m[k][0] = f2(la[k].x, lb[k].x);
-            m[k][1] = f2(la[k].y, lb[k].y);
-            m[k][2] = f2(la[k].z, lb[k].z);
-        }
-    }
+    tile_lambdas(id, L, zero, m);
     const F2 detm = r.detm();
     const F2 jm1 = fma2(dot2(q.d[0][0], q.c[0][0], q.d[0][1], q.c[0][1], q.d[0][2], q.c[0][2]), detm, f2(-1.f, -1.f));
     F2 dJ;
@@ -377,39 +387,43 @@ __device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, f
         const F2 t2 = dot2(q.c[2][0], m[2][0], q.c[2][1], m[2][1], q.c[2][2], m[2][2]);
         dJ = mul2(detm, add2(add2(t0, t1), t2));
     }
-    const F2 n0[3] = {neg2(q.d[0][0]), neg2(q.d[0][1]), neg2(q.d[0][2])};
-    const ulonglong2 sw = r.s2w0(), w12 = r.w12(), s01 = r.s01(), ab = r.ab();
+    ulonglong2 sw = r.s2w0(), w12 = r.w12();
     F2 C[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) C[i] = dot2(q.c[0][i], sw.y, q.c[1][i], w12.x, q.c[2][i], w12.y);
+    const ulonglong2 ab = r.ab(), s01 = r.s01();
+    {
+        const F2 am = mul2(ab.x, neg2(add2(add2(s01.x, s01.y), sw.x)));
+        const F2 b0 = mul2(ab.y, C[0]), b1 = mul2(ab.y, C[1]), b2 = mul2(ab.y, C[2]);
+        acc.h00 = add2(acc.h00, fma2(b0, C[0], am));
+        acc.h01 = fma2(b0, C[1], acc.h01);
+        acc.h02 = fma2(b0, C[2], acc.h02);
+        acc.h11 = add2(acc.h11, fma2(b1, C[1], am));
+        acc.h12 = fma2(b1, C[2], acc.h12);
+        acc.h22 = add2(acc.h22, fma2(b2, C[2], am));
+    }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
         // lam_1 x d_2 + d_1 x lam_2 and cyclic
-        const F2 e0 = add2(cross2(m[1][i1], q.d[2][i2], m[1][i2], q.n2[i1]), cross2(q.d[1][i1], m[2][i2], q.n1[i2], m[2][i1]));
-        const F2 e1 = add2(cross2(m[2][i1], q.d[0][i2], m[2][i2], n0[i1]), cross2(q.d[2][i1], m[0][i2], q.n2[i2], m[0][i1]));
-        const F2 e2 = add2(cross2(m[0][i1], q.d[1][i2], m[0][i2], q.n1[i1]), cross2(q.d[0][i1], m[1][i2], n0[i2], m[1][i1]));
-        C[i] = dot2(q.c[0][i], sw.y, q.c[1][i], w12.x, q.c[2][i], w12.y);
+        const F2 e0 = add2(cross2(m[1][i1], q.d[2][i2], m[1][i2], q.d[2][i1]), cross2(q.d[1][i1], m[2][i2], q.d[1][i2], m[2][i1]));
+        const F2 e1 = add2(cross2(m[2][i1], q.d[0][i2], m[2][i2], q.d[0][i1]), cross2(q.d[2][i1], m[0][i2], q.d[2][i2], m[0][i1]));
+        const F2 e2 = add2(cross2(m[0][i1], q.d[1][i2], m[0][i2], q.d[1][i1]), cross2(q.d[0][i1], m[1][i2], q.d[0][i2], m[1][i1]));
         const F2 dF = dot2(m[0][i], s01.x, m[1][i], s01.y, m[2][i], sw.x);
         const F2 dC = dot2(e0, sw.y, e1, w12.x, e2, w12.y);
         F2& g = i == 0 ? acc.g0 : i == 1 ? acc.g1 : acc.g2;
         g = add2(g, fma2(ab.x, sub2(dF, dC), mul2(ab.y, fma2(dJ, C[i], mul2(jm1, dC)))));
     }
-    const F2 am = mul2(ab.x, neg2(add2(add2(s01.x, s01.y), sw.x)));
-    const F2 b0 = mul2(ab.y, C[0]), b1 = mul2(ab.y, C[1]), b2 = mul2(ab.y, C[2]);
-    acc.h00 = add2(acc.h00, fma2(b0, C[0], am));
-    acc.h01 = fma2(b0, C[1], acc.h01);
-    acc.h02 = fma2(b0, C[2], acc.h02);
-    acc.h11 = add2(acc.h11, fma2(b1, C[1], am));
-    acc.h12 = fma2(b1, C[2], acc.h12);
-    acc.h22 = add2(acc.h22, fma2(b2, C[2], am));
 }
 
-// Record chunks from the packed incidence records (layout 3 or 4): chunk i holds round `r` of a group;
+// Record chunks from the packed incidence records (layout 3 or 4): a chunk holds one round of a group;
 // vertex slot k's threads t take incidences r L + t and r L + t + L/2.  Neighbour ids become local.
 template <int LAYOUT>
 __global__ void __launch_bounds__(256) k_pack_tile(SweepParams p, const int* __restrict__ table, int nchunks, int lanes,
-                                                   const TileGroup* __restrict__ groups, const TileHead* __restrict__ head,
-                                                   const int* __restrict__ lid, const int* __restrict__ vtile,
-                                                   const int* __restrict__ vlocal, int nfree, float4* __restrict__ out) {
+                                                   const TileGroup* __restrict__ groups,
+                                                   const TileHead* __restrict__ head, const int* __restrict__ lid,
+                                                   const int* __restrict__ vtile, const int* __restrict__ vlocal,
+                                                   int nfree, float4* __restrict__ out) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= nchunks) return;
@@ -453,37 +467,54 @@ __global__ void __launch_bounds__(256) k_pack_tile(SweepParams p, const int* __r
     reinterpret_cast<float2*>(o + 160)[lane] = make_float2(r[0].detm, r[1].detm);
 }
 
-// T threads per vertex (2 T lanes' partial sums), W warps.  W = 8 is the form for tiles with little work
-// per colour, where a colour lasts as long as one vertex's dependency chain: everything that does not
-// depend on the neighbours is fetched before the barrier, and up to two ring slots are refilled only
-// after the group's results are out.  W = 16 is the form for tiles that keep an SM's issue slots and
-// memory streams busy, held to 128 registers.
-template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
+// T threads per vertex (2 T lanes' partial sums, two per thread in the two-wide FP32 instructions), W warps.
+// W = 8 is the form for tiles with little work per colour, where a colour lasts as long as one vertex's
+// dependency chain: everything that does not depend on the neighbours is fetched before the barrier, and
+// the chunks stay in shared memory where they fit, else are refilled only after the group's results are
+// out.  (One lane per thread in plain FP32 measured 1.32 against 1.41 us a colour on the beam, but 1.75
+// against 1.68 on the 16^3 cube and 2.16 against 1.86 on the 24^3.)  W = 16 is the form for tiles that keep
+// an SM's issue slots and memory streams busy, held to 128 registers.
+//
+// CL: the tiles are the CTAs of one thread-block cluster, and a vertex's results go straight into its
+// neighbours' ghost entries with st.async, completing on the receiver's mbarrier of that colour, instead
+// of through words in L2.  A receiver knows the bytes each colour brings.  A sender's colour c of
+// iteration k + 1 cannot reach a receiver still waiting for colour c of iteration k: it holds a value
+// that receiver computed after that wait (the argument for the words, above), so one barrier per colour
+// is enough, armed for the next iteration when its wait ends; bytes that arrive before that are held
+// against the same phase.
+template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     extern __shared__ __align__(16) unsigned char tsm[];
     constexpr int NT = W * 32;
     constexpr bool LAT = W <= 8;
+    static_assert(LAT || !CL, "the cluster exchange is the W = 8 form's");
     __shared__ __align__(8) unsigned long long bars[LAT ? 1 : W * kTileMaxRing];
+    __shared__ __align__(8) unsigned long long cbars[CL ? kTileMaxColours : 1];
     __shared__ float4 stage[LAT ? 1 : W * 64 / T];  // W = 16: own data of each warp's next group
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x;
+    const bool two = CL || p.two;
     const TileHead h = p.head[tile];
-    char* ring_buf = reinterpret_cast<char*>(tsm) + (size_t)warp * p.ring * kTileChunkBytes;
-    float4* sx = reinterpret_cast<float4*>(tsm + (size_t)W * p.ring * kTileChunkBytes);  // x (or lambda)
-    float4* sX = sx + (p.max_local + 1);                  // adjoint: X; forward: the blended buffer (p.two)
-    TileGroup* sg = reinterpret_cast<TileGroup*>(sx + (size_t)(p.max_local + 1) * (ADJ || p.two ? 2 : 1));
+    const bool resident = LAT && p.resident;
+    const int2 ws = p.wstream[tile * W + warp];
+    const int slots = resident ? ws.y : p.ring;  // of this warp's ring
+    char* ring_buf = reinterpret_cast<char*>(tsm) +
+                     (size_t)(resident ? ws.x - p.wstream[tile * W].x : warp * p.ring) * kTileChunkBytes;
+    float4* sx = reinterpret_cast<float4*>(tsm + (size_t)p.ring_chunks * kTileChunkBytes);  // x (or lambda)
+    float4* sb = sx + (two ? p.max_local + 1 : 0);                  // the blended buffer
+    float4* sX = sb + (ADJ ? p.max_local + 1 : 0);                  // adjoint: X
+    TileGroup* sg = reinterpret_cast<TileGroup*>(sX + p.max_local + 1);
     int* gid = reinterpret_cast<int*>(sg + p.max_groups);  // internal ids of own vertices and ghosts
     int* ghost = gid + p.max_ids;
     int* wcols = ghost + p.ncol + 1;
+    int* toff = wcols + W * (p.ncol + 1);
+    int* targets = toff + p.max_own + 1;
 
     const unsigned ring_smem = (unsigned)__cvta_generic_to_shared(ring_buf);
     TileRing ring;
-    {
-        const int2 ws = p.wstream[tile * W + warp];
-        ring.first = ring.next = ws.x;
-        ring.end = ws.x + ws.y;
-        ring.left = ws.y * (p.k1 - p.k0);
-        ring.slot = 0;
-    }
+    ring.first = ring.next = ws.x;
+    ring.end = ws.x + ws.y;
+    ring.left = ws.y * (p.k1 - p.k0);
+    ring.slot = 0;
     const unsigned bar = LAT ? 0u : (unsigned)__cvta_generic_to_shared(bars + warp * kTileMaxRing);
     unsigned parity = 0;  // W = 16: of the ring's current round
     if (!LAT) {
@@ -494,11 +525,11 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
         }
         __syncwarp();
     }
-    for (int i = 0; i < p.ring; ++i) {
+    for (int i = 0; i < slots; ++i) {
         if (LAT) ring_issue(p, ring, ring_smem, i, lane);
         else ring_issue_bulk(p, ring, ring_smem, bar, i, lane);
     }
-    if (tid == 0) atomicAdd(p.arrived, 1ull);
+    if (!CL && tid == 0) atomicAdd(p.arrived, 1ull);
 
     for (int i = tid; i < h.ngroups; i += NT) sg[i] = p.groups[h.group + i];
     for (int i = tid; i <= p.ncol; i += NT) ghost[i] = p.ghost[tile * (p.ncol + 1) + i];
@@ -506,13 +537,36 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
     const int* lid = p.lid + h.lid;
     const int nloc = h.nown + h.nghost + h.npinned;
     for (int i = tid; i < h.nown + h.nghost; i += NT) gid[i] = lid[i];
+    // Cluster exchange: the bytes colour c of iteration k brings this CTA; nobody reads x~ of the last
+    // colour when the iteration blends, and nothing of the last iteration's last colour.
+    const unsigned cbar0 = (unsigned)__cvta_generic_to_shared(cbars);
+    auto colour_bytes = [&](int k, int c, bool blend) {
+        const bool last = c == p.ncol - 1, more = k < p.k1 - 1;
+        const unsigned words = ((last ? !blend && more : true) ? 1u : 0u) + (blend && more ? 1u : 0u);
+        return 16u * words * (unsigned)(ghost[c + 1] - ghost[c]);
+    };
+    if constexpr (CL) {
+        for (int i = tid; i <= h.nown; i += NT) toff[i] = p.target_off[tile * (p.max_own + 1) + i];
+        __syncthreads();
+        for (int i = tid; i < toff[h.nown]; i += NT) targets[i] = p.target[tile * p.max_target + i];
+        if (tid == 0) {
+            for (int c = 0; c < p.ncol; ++c) {
+                mbar_init(cbar0 + 8u * c);
+                const unsigned b = p.k1 > p.k0 ? colour_bytes(p.k0, c, __ldg(p.omega + p.k0) > 1.0f) : 0u;
+                if (b) mbar_expect(cbar0 + 8u * c, b);
+            }
+            fence_mbar_init();
+        }
+    }
     if constexpr (ADJ) {
         for (int i = tid; i < nloc; i += NT) {
             const int g = lid[i];
             sX[i] = __ldg(p.X + g);
-            sx[i] = p.lam_in[g];
+            const float4 l = p.lam_in[g];
+            sx[i] = l;
+            if (CL) sb[i] = l;
         }
-        if (tid == 0) sx[p.max_local] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tid == 0) sx[p.max_local] = sb[p.max_local] = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
         // own vertices, and this CTA's share of the pinned ones
         const int gp = p.nfree + tile * NT + tid, step = gridDim.x * NT;
@@ -526,7 +580,7 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
             const int g = lid[i];
             const float4 a = p.from_inertia ? p.y[g] : p.x0[g];
             sx[i] = make_float4(a.x, a.y, a.z, 0.f);
-            if (p.two) sX[i] = make_float4(a.x, a.y, a.z, 0.f);
+            if (two) sb[i] = make_float4(a.x, a.y, a.z, 0.f);
         }
         if (p.from_inertia)  // x = y for the pinned vertices too (k_copy_xyz)
             for (int g = gp; g < p.n; g += step) {
@@ -534,35 +588,53 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
                 p.x0[g] = p.x1[g] = make_float4(a.x, a.y, a.z, 0.f);
             }
     }
+    if (CL) {  // every CTA's barriers and vectors are ready before any CTA sends
+        cluster_arrive();
+        cluster_wait();
+    }
     __syncthreads();
 
-    // Which ghost a thread polls first: W = 8 spreads them over the warps, the last one first (a warp's
-    // poll takes as long as its slowest lane, and the first warps sweep most).
-    const int poll_at = LAT ? lane * W + (W - 1 - warp) : NT - 1 - tid;
+    // Which ghost a thread polls first: W = 8 spreads them over the last warps (a warp's poll takes as long as
+    // its slowest lane, and the first warps sweep): 1.66 us a colour on the 16^3 cube, 1.72 over all warps.
+    // Two or four polls of a word in flight, spaced over the round trip, made stores land later: 1.87.
+    constexpr int kPollWarps = W / 2;
+    const int poll_at = !LAT               ? NT - 1 - tid
+                        : warp >= kPollWarps ? lane * kPollWarps + (W - 1 - warp)
+                                             : (32 + lane) * kPollWarps + (kPollWarps - 1 - warp);
     const int slot = lane / T, t = lane & (T - 1);
     const int* wcol = wcols + warp * (p.ncol + 1);
     const int wfirst = wcol[0], wlast = wcol[p.ncol];
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     // The warp's next group and its vertices' own data, fetched before the barrier that precedes its
-    // sweep: y (adjoint: G) by thread t = 0 of a vertex, the position before the last sweep by t = 1.  W = 8
-    // holds them in registers; W = 16 has none to spare and stages them in shared memory.
+    // sweep: y (adjoint: G) and the position before the last sweep.  W = 8 holds them in registers of every
+    // thread of the vertex; W = 16 has none to spare and stages them in shared memory.
     TileGroup next_g{};
-    float4 own = zero4;
+    float4 own = zero4, prev = zero4;
     float mass = 0.f;
+    int send_to = -1, send_more = 0, send_end = 0;  // CL: this thread's first target and the further ones
     float4* my_stage = stage + (LAT ? 0 : warp * (64 / T) + 2 * slot);
     auto load_group = [&](int gi) {
         const TileGroup g = sg[gi];
         const int gv = g.gv + slot;
-        const float4* src = (t == 0 ? (ADJ ? p.G : p.y) : p.pp) + gv;
         if (LAT) {
             next_g = g;
             // predicated loads into the same registers: no instruction waits for them before the solve
-            load_if(slot < g.count && t < 2, src, own);
-            if constexpr (ADJ) load_if(slot < g.count && t == 0, &p.y[gv].w, mass);
+            load_if(slot < g.count, (ADJ ? p.G : p.y) + gv, own);
+            load_if(slot < g.count, p.pp + gv, prev);
+            if constexpr (ADJ) load_if(slot < g.count, &p.y[gv].w, mass);
+            if constexpr (CL) {
+                send_to = -1;
+                send_more = send_end = 0;
+                if (slot < g.count) {
+                    send_more = toff[g.lv + slot] + t;
+                    send_end = toff[g.lv + slot + 1];
+                    if (send_more < send_end) send_to = targets[send_more];
+                }
+            }
         } else {
             if (slot < g.count && t < 2)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(my_stage + t)),
-                             "l"(src)
+                             "l"((t == 0 ? (ADJ ? p.G : p.y) : p.pp) + gv)
                              : "memory");
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
@@ -571,30 +643,34 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
     // Chunk i is commit group i.  W = 8: a group's chunks (at most p.max_rounds) have all landed before the
     // barrier that precedes its sweep, and its slots are refilled after its results are out.  W = 16: a
     // chunk is waited for when it is swept and refilled right after.
-    const int pending = p.ring - p.max_rounds;
+    const int pending = resident ? 0 : p.ring - p.max_rounds;
     auto chunk_at = [&](int s) { return TilePair{ring_buf + s * kTileChunkBytes, lane}; };
-    auto next_slot = [&](int s) { return s + 1 == p.ring ? 0 : s + 1; };
+    auto next_slot = [&](int s) { return s + 1 == slots ? 0 : s + 1; };
     if (p.k1 > p.k0 && wlast > wfirst) {
         load_group(wfirst);
         if (LAT) ring_wait(pending);
     }
     bool alive = true;
     float4* xs = sx;  // x (adjoint: lambda) of this iteration
-    float4* xb = sX;  // p.two: receives the blended positions
+    float4* xb = sb;  // two: receives the blended positions
+    float om_next = p.k1 > p.k0 ? __ldg(p.omega + p.k0) : 1.0f;
     for (int k = p.k0; k < p.k1 && alive; ++k) {
-        const float om = __ldg(p.omega + k);
-        const bool blend = om > 1.0f;
+        const float om = om_next;
+        om_next = __ldg(p.omega + min(k + 1, p.k1 - 1));  // known a whole iteration ahead
+        const bool blend = om > 1.0f, more = k < p.k1 - 1;
         const unsigned tag = p.tag + (unsigned)k;
         // the words of x~ and of the blended positions; W = 16 forms the addresses where it uses them
         auto words = [&](unsigned which) {
             unsigned at = which + (tag & 1u);
             if (!LAT) asm volatile("" : "+r"(at));
-            return p.words + (size_t)at * p.n;
+            return p.words + (size_t)at * p.n * p.word_stride;
         };
         int gi = wfirst;
         for (int c = 0; c < p.ncol; ++c) {
             const int gend = wcol[c + 1];
-            int p0 = 0, p1 = 0;  // the ghosts of colour c (last threads first: the last warps sweep least)
+            const bool last = c == p.ncol - 1;
+            const bool need_x = last ? !blend && more : true, need_b = blend && more;  // by other tiles
+            int p0 = 0, p1 = 0;  // the ghosts of colour c
             if (LAT) p0 = ghost[c] + poll_at, p1 = ghost[c + 1];
             __syncthreads();  // everything colour c reads is in shared memory
             while (gi < gend) {
@@ -642,50 +718,62 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
                 // W = 16 reads the group again instead of holding it
                 const TileGroup g = LAT ? next_g : sg[gi];
                 const bool active = slot < g.count;
-                const int lv = g.lv + slot;
-                // lanes t and t + T, then the T threads: group_reduce's order for 2 T lanes
+                const int lv = g.lv + slot, gv = g.gv + slot;
+                // lanes t and t + T, then the T threads: group_reduce's order for 2 T lanes.  Every thread of the
+                // vertex ends with the same sums.
                 Acc acc = acc2.sum();
                 group_reduce<T>(acc);
-                float4 y = own, q = own;
-                if (LAT) {
-                    if (blend) {  // the previous position, from the vertex's second thread
-                        q.x = __shfl_down_sync(0xffffffffu, own.x, 1);
-                        q.y = __shfl_down_sync(0xffffffffu, own.y, 1);
-                        q.z = __shfl_down_sync(0xffffffffu, own.z, 1);
-                    }
-                } else {
+                float4 y = own, q = prev;
+                if (!LAT) {
                     ring_wait_for<0>();
                     __syncwarp();
                     if (active && t == 0) {
                         y = my_stage[0];
                         q = my_stage[1];
-                        if constexpr (ADJ) mass = __ldg(&p.y[g.gv + slot].w);
+                        if constexpr (ADJ) mass = __ldg(&p.y[gv].w);
                     }
                 }
-                if (active && t == 0) {
-                    const int gv = g.gv + slot;
-                    float4 xn, xa, old;
+                if (active && (CL || t == 0)) {
+                    float4 xn, xa = zero4, old;
                     if constexpr (ADJ) {
                         old = xs[lv];
                         xn = adj_block_solve(acc, mass, p.dtsr, y);
                     } else {
                         old = xi;
-                        xn = block_update(acc, xi, y, p.dtsr, p.status);
+                        xn = block_update(acc, xi, y, p.dtsr, p.status, t == 0);
                     }
-                    if (slot < g.publish) word_store(words(0u) + gv, xn.x, xn.y, xn.z, tag);
-                    if (blend) {
-                        xa = ADJ ? adj_blend(xn, q, om) : cheb_blend(xn, q, om);
-                        if (!p.two || slot < g.publish) word_store(words(2u) + gv, xa.x, xa.y, xa.z, tag);
-                        if (p.two) xb[lv] = xa;
+                    if (CL) {
+                        if (blend) xa = ADJ ? adj_blend(xn, q, om) : cheb_blend(xn, q, om);
+                        for (int to = send_to; to >= 0;) {
+                            const unsigned r = (unsigned)to >> 16, at = (unsigned)to & 0xffffu;
+                            const unsigned rb = cluster_map(cbar0 + 8u * c, r);
+                            if (need_x) st_async(cluster_map((unsigned)__cvta_generic_to_shared(xs + at), r), xn, rb);
+                            if (need_b) st_async(cluster_map((unsigned)__cvta_generic_to_shared(xb + at), r), xa, rb);
+                            send_more += T;
+                            to = send_more < send_end ? targets[send_more] : -1;
+                        }
+                        if (t == 0 && blend) xb[lv] = xa;
+                    } else {
+                        if (slot < g.publish) word_store(words(0u) + (size_t)gv * p.word_stride, xn.x, xn.y, xn.z, tag);
+                        if (blend) {
+                            xa = ADJ ? adj_blend(xn, q, om) : cheb_blend(xn, q, om);
+                            if (!two || slot < g.publish) word_store(words(2u) + (size_t)gv * p.word_stride, xa.x, xa.y, xa.z, tag);
+                            if (two) xb[lv] = xa;
+                        }
                     }
-                    xs[lv] = xn;
-                    if (p.keep_pp) p.pp[gv] = old;
-                    if (!ADJ) flag_nonfinite(xn, p.status);
+                    if (t == 0) {
+                        xs[lv] = xn;
+                        if (p.keep_pp) p.pp[gv] = old;
+                        if (!ADJ) flag_nonfinite(xn, p.status);
+                    }
                 }
-                __syncwarp();  // the second thread may read p.pp of the same vertex next
+                __syncwarp();  // the other threads may read p.pp of the same vertex next
                 ++gi;
                 load_group(gi < wlast ? gi : wfirst);
-                if (LAT) {
+                if (LAT && resident) {
+                    ring.slot += rounds;
+                    if (ring.slot >= slots) ring.slot = 0;
+                } else if (LAT) {
                     for (; rounds > 0; --rounds) {
                         ring_issue(p, ring, ring_smem, ring.slot, lane);
                         ring.slot = next_slot(ring.slot);
@@ -693,52 +781,65 @@ template <int T, bool ADJ, int W> __global__ void __launch_bounds__(W * 32, 1) k
                     ring_wait(pending);
                 }
             }
-            // Colour c of the neighbouring tiles: x~, which the next colour reads.  Nobody reads x~ of the last
-            // colour when the iteration blends.  With both buffers here the blended words are taken as
-            // well, one colour late (they have landed by then and are needed only next iteration).
-            const bool last = c == p.ncol - 1, more = k < p.k1 - 1;
-            if (!LAT) p0 = ghost[c] + poll_at, p1 = ghost[c + 1];
-            if (blend && p.two && more) {
-                const int e = last ? ghost[c + 1] : ghost[c];
-                for (int i = (c ? ghost[c - 1] : ghost[0]) + poll_at; ok && i < e; i += NT) {
-                    const float4* w = words(2u) + gid[i];
-                    ok = tile_take(p, word_load(w), w, tag, xb + i);
+            if constexpr (CL) {
+                if ((need_x || need_b) && p1 > ghost[c]) {
+                    ok = ok && mbar_wait(cbar0 + 8u * c, (unsigned)(k - p.k0) & 1u, p.status);
+                    if (tid == 0 && more) {
+                        const unsigned b = colour_bytes(k + 1, c, om_next > 1.0f);
+                        if (b) mbar_expect(cbar0 + 8u * c, b);
+                    }
                 }
+            } else {
+                // Colour c of the neighbouring tiles: x~, which the next colour reads.  Nobody reads x~ of the last
+                // colour when the iteration blends.  With both buffers here the blended words are taken as
+                // well, one colour late (they have landed by then and are needed only next iteration).
+                if (!LAT) p0 = ghost[c] + poll_at, p1 = ghost[c + 1];
+                if (need_b && two) {
+                    const int e = last ? ghost[c + 1] : ghost[c];
+                    for (int i = (c ? ghost[c - 1] : ghost[0]) + poll_at; ok && i < e; i += NT) {
+                        const float4* w = words(2u) + (size_t)gid[i] * p.word_stride;
+                        ok = tile_take(p, word_load(w), w, tag, xb + i);
+                    }
+                }
+                if (need_x)
+                    for (int i = p0; ok && i < p1; i += NT) {
+                        const float4* w = words(0u) + (size_t)gid[i] * p.word_stride;
+                        ok = LAT ? tile_spin(p, w, tag, xs + i) : tile_take(p, word_load(w), w, tag, xs + i);
+                    }
             }
-            if (last ? !blend && more : true)
-                for (int i = p0; ok && i < p1; i += NT) {
-                    const float4* w = words(0u) + gid[i];
-                    ok = LAT ? tile_spin(p, w, tag, xs + i) : tile_take(p, word_load(w), w, tag, xs + i);
-                }
         }
         // one wait that gave up ends the walk
         alive = __syncthreads_and(ok) != 0;
         if (!alive || !blend) continue;
-        if (p.two) {
+        if (two) {
             float4* s = xs;
             xs = xb;
             xb = s;
             continue;
         }
         // the blended positions replace x~: own ones and ghosts
-        const int e = k == p.k1 - 1 ? h.nown : h.nown + h.nghost;
+        const int e = more ? h.nown + h.nghost : h.nown;
         constexpr int kBatch = 6;
         const float4* wb = words(2u);
         for (int i0 = tid; ok && i0 < e; i0 += kBatch * NT) {
             float4 w[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; ++u)
-                if (i0 + u * NT < e) w[u] = word_load(wb + gid[i0 + u * NT]);
+                if (i0 + u * NT < e) w[u] = word_load(wb + (size_t)gid[i0 + u * NT] * p.word_stride);
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
                 const int i = i0 + u * NT;
                 if (i >= e) continue;
                 if (__float_as_uint(w[u].w) == tag) xs[i] = make_float4(w[u].x, w[u].y, w[u].z, 0.f);
-                else ok = ok && tile_spin(p, wb + gid[i], tag, xs + i);
+                else ok = ok && tile_spin(p, wb + (size_t)gid[i] * p.word_stride, tag, xs + i);
             }
         }
     }
     ok = __syncthreads_and(alive && ok) != 0;
+    if (CL) {  // no CTA leaves while another may still send to it
+        cluster_arrive();
+        cluster_wait();
+    }
     // no copy outlives the walk (one that gave up has bulk copies under way; the waits are bounded)
     ring_wait_for<0>();
     if (!LAT && !ok) {

@@ -166,6 +166,84 @@ void tile_lists(TilePlan* plan, const std::vector<int>& cstart, const std::vecto
     }
 }
 
+void tile_merge(const TilePlan& fine, int parts, const std::vector<int>& cstart, TilePlan* out) {
+    TilePlan& p = *out;
+    const int C = fine.C, F = fine.P;
+    p.P = parts;
+    p.C = C;
+    p.n = fine.n;
+    p.nfree = fine.nfree;
+    p.vtile.resize(fine.nfree);
+    p.vlocal.assign(fine.nfree, 0);
+    for (int v = 0; v < fine.nfree; ++v) p.vtile[v] = (int)((long long)fine.vtile[v] * parts / F);
+    p.cb.assign((size_t)C * (parts + 1), 0);
+    p.bnd.assign((size_t)C * parts, 0);  // no words are published
+    for (int c = 0; c < C; ++c) {
+        int32_t* cb = &p.cb[(size_t)c * (parts + 1)];
+        int v = cstart[c];
+        for (int t = 0; t < parts; ++t) {
+            cb[t] = v;
+            while (v < cstart[c + 1] && p.vtile[v] == t) ++v;
+        }
+        cb[parts] = v;
+    }
+    p.head.assign(parts, TileHead{});
+    p.ghost.assign((size_t)parts * (C + 1), 0);
+    std::vector<std::vector<int32_t>> ext(parts);
+    for (int f = 0; f < F; ++f) {
+        const TileHead& h = fine.head[f];
+        const int t = (int)((long long)f * parts / F);
+        for (int i = h.lid + h.nown; i < h.lid + h.nown + h.nghost + h.npinned; ++i) {
+            const int u = fine.lid[i];
+            if (u >= fine.nfree || p.vtile[u] != t) ext[t].push_back(u);
+        }
+    }
+    for (int t = 0; t < parts; ++t) {
+        TileHead& h = p.head[t];
+        std::sort(ext[t].begin(), ext[t].end());
+        ext[t].erase(std::unique(ext[t].begin(), ext[t].end()), ext[t].end());
+        h.lid = (int)p.lid.size();
+        for (int c = 0; c < C; ++c)
+            for (int v = p.cb[(size_t)c * (parts + 1) + t]; v < p.cb[(size_t)c * (parts + 1) + t + 1]; ++v) {
+                p.vlocal[v] = h.nown++;
+                p.lid.push_back(v);
+            }
+        p.lid.insert(p.lid.end(), ext[t].begin(), ext[t].end());
+        h.nghost = (int)(std::lower_bound(ext[t].begin(), ext[t].end(), p.nfree) - ext[t].begin());
+        h.npinned = (int)ext[t].size() - h.nghost;
+        for (int c = 0; c <= C; ++c)
+            p.ghost[(size_t)t * (C + 1) + c] =
+                h.nown + (int)(std::lower_bound(ext[t].begin(), ext[t].end(), cstart[c]) - ext[t].begin());
+        p.max_own = std::max(p.max_own, h.nown);
+        p.max_ids = std::max(p.max_ids, h.nown + h.nghost);
+        p.max_local = std::max(p.max_local, h.nown + h.nghost + h.npinned);
+    }
+    std::vector<std::vector<std::vector<int32_t>>> to(parts);
+    for (int t = 0; t < parts; ++t) to[t].resize(p.head[t].nown);
+    for (int t = 0; t < parts; ++t)
+        for (int i = 0; i < p.head[t].nghost; ++i) {
+            const int u = ext[t][i];
+            to[p.vtile[u]][p.vlocal[u]].push_back((t << 16) | (p.head[t].nown + i));
+        }
+    for (int t = 0; t < parts; ++t) {
+        int n = 0;
+        for (const auto& l : to[t]) n += (int)l.size();
+        p.max_target = std::max(p.max_target, n);
+    }
+    p.target_off.assign((size_t)parts * (p.max_own + 1), 0);
+    p.target.assign((size_t)parts * std::max(1, p.max_target), 0);
+    for (int t = 0; t < parts; ++t) {
+        int n = 0;
+        int32_t* off = &p.target_off[(size_t)t * (p.max_own + 1)];
+        for (int i = 0; i < p.max_own; ++i) {
+            off[i] = n;
+            if (i < p.head[t].nown)
+                for (int x : to[t][i]) p.target[(size_t)t * p.max_target + n++] = x;
+        }
+        off[p.max_own] = n;
+    }
+}
+
 void tile_groups(TilePlan* plan, int lanes, int warps, const int32_t* inc_off) {
     TilePlan& p = *plan;
     p.lanes = lanes;
@@ -174,11 +252,12 @@ void tile_groups(TilePlan* plan, int lanes, int warps, const int32_t* inc_off) {
     p.chunk.clear();
     p.wcol.assign((size_t)p.P * warps * (p.C + 1), 0);
     p.wstream.assign((size_t)p.P * warps * 2, 0);
-    p.max_groups = p.max_rounds = 0;
+    p.max_groups = p.max_rounds = p.max_chunks = 0;
     const int per = kTileChunk / lanes;  // vertices per group
     for (int t = 0; t < p.P; ++t) {
         TileHead& h = p.head[t];
         h.group = (int)p.groups.size();
+        const int first = (int)(p.chunk.size() / 3);
         // colour c's groups go round the warps; each warp's groups and chunks lie in the order it sweeps them
         for (int w = 0; w < warps; ++w) {
             int32_t* ws = &p.wstream[((size_t)t * warps + w) * 2];
@@ -210,6 +289,7 @@ void tile_groups(TilePlan* plan, int lanes, int warps, const int32_t* inc_off) {
         }
         h.ngroups = (int)p.groups.size() - h.group;
         p.max_groups = std::max(p.max_groups, h.ngroups);
+        p.max_chunks = std::max(p.max_chunks, (int)(p.chunk.size() / 3) - first);
     }
 }
 

@@ -13,9 +13,9 @@ constexpr int kTileChunkBytes = kTileChunk * 44;
 constexpr int kTileMaxRing = 6;             // chunks a warp's ring holds at most
 constexpr int kTileMaxLocal = 65535;        // local vertex ids are 16 bits
 // A mesh gets a plan from this many free vertices.  Microseconds per colour of a step, tile walk against
-// captured graph (cubes of n^3 cells, one B200): n = 6 (294 free vertices) 1.61 / 2.33, 8 1.77 / 2.40, 16
-// 1.91 / 2.57, 24 2.07 / 3.31, 32 2.76 / 3.53, 48 4.8 / 5.5, 64 8.4 / 10.2.  Below it one or two tiles
-// would hold the mesh.
+// captured graph (cubes of n^3 cells, one B200): n = 6 (294 free vertices) 1.61 / 2.33, 12 1.50 / 2.50, 16
+// 1.51 / 2.57, 24 1.83 / 3.31, 32 2.73 / 3.53, 48 5.1 / 5.5, 64 8.4 / 10.2.  Below it a few vertices per
+// tile would only exchange words.
 constexpr int kTileMinVertices = 256;
 // Free vertices per tile at least, up to one tile per SM.  32, 64 and 128 measured 0.81, 0.81 and 0.86 ms a
 // step on the 12^3 to 16^3 cubes: a colour lasts one exchange and one vertex's chain either way.
@@ -24,6 +24,15 @@ constexpr int kTileVertices = 32;
 // warps: 28^3 cube (4.6 groups) 2.36 / 2.46, 32^3 (7.2) 2.99 / 2.76, 64 beams (7.7) 3.06 / 2.81, 64^3 (29)
 // 10.8 / 8.4.
 constexpr int kTileFewGroups = 6;
+// Up to this many free vertices per tile each exchanged word has a 128-byte line of its own: polls of the
+// words beside it delay a store's arrival.  Microseconds per colour with words 16 / 32 / 128 bytes apart:
+// 12^3 cube 1.59 / 1.53 / 1.47, 16^3 1.66 / 1.57 / 1.50, 24^3 (100 vertices a tile) 1.83 / 1.79 / 1.82, 28^3
+// 2.26 / 2.30 / 2.31, 64^3 8.41 / 8.62 / -.
+constexpr int kTileSpreadWords = 80;
+// Up to this many free vertices the number of tiles is a multiple of 16, so that a cluster's CTAs share them
+// evenly (VBD_OPT_PERSISTENT 2), with this many vertices per CTA at least.
+constexpr int kClusterMeshVertices = 5000;
+constexpr int kClusterTileMin = 16;
 // Ring depth that holding both position buffers must leave.
 constexpr int kTileTwoRing = 4;
 
@@ -51,13 +60,17 @@ struct TilePlan {
     std::vector<TileHead> head;    // [P]
     std::vector<int32_t> lid;      // local-to-internal ids of all tiles
     std::vector<int32_t> ghost;    // [P][C + 1]: first ghost of each colour (local id)
-    int max_local = 0, max_ids = 0, max_groups = 0, max_rounds = 0;
+    int max_local = 0, max_ids = 0, max_groups = 0, max_rounds = 0, max_chunks = 0;
     // for `lanes` threads' worth of partial sums per vertex:
     int lanes = 0, warps = 0;
     std::vector<TileGroup> groups;
     std::vector<int32_t> wcol;     // [P][warps][C + 1]: first group of each warp and colour, from the tile's first
     std::vector<int32_t> wstream;  // [P][warps][2]: first chunk and chunks of each warp
     std::vector<int32_t> chunk;    // [chunks][3]: tile, group, round
+    // of a merged plan: where each own vertex is a ghost, as tile << 16 | local id there
+    int max_own = 0, max_target = 0;
+    std::vector<int32_t> target_off;  // [P][max_own + 1], from the tile's first
+    std::vector<int32_t> target;      // [P][max_target]
 };
 
 // The tile of each vertex (-1 for pinned ones): recursive bisection of the free vertices, first by
@@ -73,6 +86,9 @@ void tile_boundary(int n, int ntet, const int32_t* tets, const std::vector<int32
 void tile_lists(TilePlan* plan, const std::vector<int>& cstart, const std::vector<int32_t>& tile_internal,
                 const std::vector<uint8_t>& boundary_internal, const int32_t* inc_off, const int32_t* inc_tet,
                 const int32_t* tets_internal, int tet_stride);
+
+// The plan with runs of consecutive tiles of `fine` merged into `parts` tiles, and its targets.
+void tile_merge(const TilePlan& fine, int parts, const std::vector<int>& cstart, TilePlan* out);
 
 // The groups and record chunks for `lanes` partial sums per vertex (two per thread) and CTAs of `warps` warps.
 void tile_groups(TilePlan* plan, int lanes, int warps, const int32_t* inc_off);
