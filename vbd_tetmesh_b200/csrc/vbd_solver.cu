@@ -118,23 +118,28 @@ template <int L> static void (*pick_cluster_adjoint(int layout))(AdjWalkParams) 
 
 // The tile walk runs lanes / 2 threads per vertex; it reads its own record chunks, packed from the
 // factored records of either layout.  With `cluster` the tiles are the CTAs of one cluster.
-template <bool ADJ> static void (*pick_tile(int lanes, int warps, bool cluster))(TileParams) {  // ADJ: 8 warps
+template <TileKind KIND> static void (*pick_tile(int lanes, int warps, bool cluster))(TileParams) {  // adjoint: 8 warps
     if (cluster)
-        return lanes == 4    ? &k_tile_walk<2, ADJ, 8, true>
-               : lanes == 8  ? &k_tile_walk<4, ADJ, 8, true>
-               : lanes == 16 ? &k_tile_walk<8, ADJ, 8, true>
-                             : &k_tile_walk<16, ADJ, 8, true>;
-    if (ADJ || warps == 8)
-        return lanes == 4 ? &k_tile_walk<2, ADJ, 8> : lanes == 8 ? &k_tile_walk<4, ADJ, 8> : &k_tile_walk<8, ADJ, 8>;
-    return lanes == 4   ? &k_tile_walk<2, false, 16>
-           : lanes == 8 ? &k_tile_walk<4, false, 16>
-                        : &k_tile_walk<8, false, 16>;
+        return lanes == 4    ? &k_tile_walk<2, KIND, 8, true>
+               : lanes == 8  ? &k_tile_walk<4, KIND, 8, true>
+               : lanes == 16 ? &k_tile_walk<8, KIND, 8, true>
+                             : &k_tile_walk<16, KIND, 8, true>;
+    if (KIND == kTileAdjoint || warps == 8)
+        return lanes == 4 ? &k_tile_walk<2, KIND, 8> : lanes == 8 ? &k_tile_walk<4, KIND, 8> : &k_tile_walk<8, KIND, 8>;
+    return lanes == 4   ? &k_tile_walk<2, kTileForward, 16>
+           : lanes == 8 ? &k_tile_walk<4, kTileForward, 16>
+                        : &k_tile_walk<8, kTileForward, 16>;
+}
+static void (*pick_tile_wrapper(int warps))(TileParams) {
+    return warps == 8 ? &k_tile_walk<16, kTileWrapper, 8> : &k_tile_walk<16, kTileWrapper, 16>;
 }
 
 // A tile plan on the device.
 struct TileSet {
     TilePlan plan;
     bool cluster = false;     // the tiles are the CTAs of one cluster
+    bool wrapper = false;     // VBD_GPU_Solver semantics
+    int chunk_bytes() const { return wrapper ? kWrapperChunkBytes : kTileChunkBytes; }
     bool dirty = true;        // the chunks must be packed again (new records)
     int layout = 0;           // layout they were packed from
     int lanes = 0;            // lanes the device lists are for
@@ -311,6 +316,7 @@ struct vbd_solver {
     // graph (chosen at init or by the autotuner, off once VBD_OPT_PERSISTENT is set), and its device data
     vbd::TileSet tset;   // one tile per SM, exchanging words through L2
     vbd::TileSet aset;   // tset's tiles swept by 8 warps, for the adjoint where tset has 16
+    vbd::TileSet wset;   // tset's tiles for VBD_GPU_Solver semantics
     vbd::TileSet cset;   // one tile per CTA of a cluster, its plan merged from tset's tiles
     int tile_walk = 0;
     bool persistent_set = false;
@@ -863,8 +869,9 @@ struct vbd_solver {
 
     // Shared memory a tile launch whose CTAs hold `vectors` local vectors leaves for record chunks.
     int tile_chunk_room(const vbd::TileSet& s, int vectors) const {
-        const long long fixed = (long long)vbd::tile_smem(s.plan.warps, 0, s.plan, C, vectors, s.cluster) + 10240;
-        return (int)std::max<long long>(0, (smem_optin - fixed) / vbd::kTileChunkBytes);
+        const long long fixed = (long long)vbd::tile_smem(s.plan.warps, 0, 0, s.plan, C, vectors, s.cluster) + 10240 +
+                                (s.wrapper ? 32 * 13 * 4 * s.plan.warps : 0);
+        return (int)std::max<long long>(0, (smem_optin - fixed) / s.chunk_bytes());
     }
     // Chunks per warp ring.
     int tile_ring(const vbd::TileSet& s, int vectors) const {
@@ -879,7 +886,7 @@ struct vbd_solver {
     }
     // The kernel of 8 warps holds a group's chunks at once, that of 16 warps two chunks at least.
     bool tile_fits(const vbd::TileSet& s, int vectors) const {
-        return s.plan.max_local <= vbd::kTileMaxLocal &&
+        return s.plan.max_local <= (s.wrapper ? vbd::kWrapperMaxLocal : vbd::kTileMaxLocal) &&
                (tile_resident(s, vectors) || tile_ring(s, vectors) >= (s.plan.warps == 8 ? s.plan.max_rounds : 2));
     }
     // Warps of the tile CTAs for the current lanes.
@@ -890,17 +897,32 @@ struct vbd_solver {
     // Whether steps and solves run as tile walks.  Under a caller's stream capture they do not: each
     // launch needs tags of its own, which a replayed launch would repeat.
     bool use_tile() {
-        if (!tile_walk || tset.plan.P == 0 || semantics || timing || !use_graph || persistent || !colour_lanes.empty() ||
-            layout < 3 || (lanes != 4 && lanes != 8 && lanes != 16) || ninc == 0)
-            return false;
+        if (!tile_walk || tset.plan.P == 0 || timing || !use_graph || persistent || ninc == 0) return false;
+        // VBD_GPU_Solver semantics read the tet records, with lanes of their own
+        if (!semantics && (!colour_lanes.empty() || layout < 3 || (lanes != 4 && lanes != 8 && lanes != 16))) return false;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
             (void)cudaGetLastError();
             return false;
         }
         if (cs != cudaStreamCaptureStatusNone) return false;
-        if (tset.plan.lanes != lanes) vbd::tile_groups(&tset.plan, lanes, tile_warps(), h_inc_off.data());
-        return tile_fits(tset, 1);
+        if (semantics) {
+            if (wset.plan.P == 0) {
+                vbd::TilePlan q = tset.plan;
+                vbd::tile_groups(&q, vbd::kWrapperTileLanes, wrapper_warps(), h_inc_off.data());
+                wset.reset(std::move(q));
+                wset.wrapper = true;
+            }
+        } else if (tset.plan.lanes != lanes) {
+            vbd::tile_groups(&tset.plan, lanes, tile_warps(), h_inc_off.data());
+        }
+        return tile_fits(walk_tiles(), 1);
+    }
+    vbd::TileSet& walk_tiles() { return semantics ? wset : tset; }
+    // Groups per colour and tile up to which 8 warps sweep them.
+    int wrapper_warps() const {
+        const double groups = (double)nfree / std::max(1, C) / std::max(1, tset.plan.P) * vbd::kWrapperTileLanes / vbd::kTileChunk;
+        return groups <= vbd::kTileFewGroups && max_valence <= vbd::kWrapperTileLanes * (vbd::kTileMaxRing / 2) ? 8 : 16;
     }
     // The adjoint's tiles: its kernel takes more than the 128 registers of 16 warps (with them it spills: 5.2 us
     // a colour against 4.2 with 8 warps for the adjoint of 64 beams).
@@ -928,12 +950,12 @@ struct vbd_solver {
         }
         const int which = adjoint ? 1 : 0, vectors = adjoint ? 3 : 2;
         if (!tile_fits(cset, vectors)) return false;
-        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<true>(L, 8, true)
-                                                              : vbd::pick_tile<false>(L, 8, true));
+        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<vbd::kTileAdjoint>(L, 8, true)
+                                                              : vbd::pick_tile<vbd::kTileForward>(L, 8, true));
         if (cset.checked[which] != f) {
             cset.checked[which] = f;
             cset.resident[which] = false;
-            const size_t smem = vbd::tile_smem(8, tile_ring_chunks(cset, vectors), cset.plan, C, vectors, true);
+            const size_t smem = vbd::tile_smem(8, tile_ring_chunks(cset, vectors), cset.chunk_bytes(), cset.plan, C, vectors, true);
             if (allow_shared(f, true) == cudaSuccess) {
                 cudaLaunchConfig_t cfg = {};
                 cudaLaunchAttribute attr[1];
@@ -987,7 +1009,7 @@ struct vbd_solver {
                 if (lists[k].ints) std::memcpy(all.data() + s.at[k], lists[k].p, 4 * lists[k].ints);
             s.stride = nfree <= (long long)vbd::kTileSpreadWords * q.P ? 8 : 1;
             s.nwords = s.cluster ? 0 : 4 * (size_t)s.stride * N + 1;
-            const size_t nchunk = q.chunk.size() / 3 * (vbd::kTileChunkBytes / 16);
+            const size_t nchunk = q.chunk.size() / 3 * (size_t)(s.chunk_bytes() / 16);
             const size_t need = s.nwords + nchunk + all.size() / 4;
             if (s.mem.n < need) {
                 if (s.cluster) drop_graphs();  // the adjoint's captured launches hold the addresses
@@ -1004,7 +1026,18 @@ struct vbd_solver {
             s.dirty = true;
             s.lanes = q.lanes;
         }
-        if (s.dirty || s.layout != layout) {
+        if (s.wrapper && s.dirty) {
+            const int nch = (int)(q.chunk.size() / 3);
+            if (nch > 0) {
+                vbd::k_pack_wrapper<<<vbd::nblk((long long)nch * 32, 256), 256, 0, stream>>>(
+                    inc_off.p, inc_tet.p, rec.p, s.ints(vbd::TileSet::TABLE), nch,
+                    reinterpret_cast<const vbd::TileGroup*>(s.ints(vbd::TileSet::GROUPS)),
+                    reinterpret_cast<const vbd::TileHead*>(s.ints(vbd::TileSet::HEAD)), s.ints(vbd::TileSet::LID),
+                    s.ints(vbd::TileSet::VTILE), s.ints(vbd::TileSet::VLOCAL), nfree, s.chunk);
+                VBD_TRY(check_launch());
+            }
+            s.dirty = false;
+        } else if (!s.wrapper && (s.dirty || s.layout != layout)) {
             const int nch = (int)(q.chunk.size() / 3);
             vbd::SweepParams p{};
             p.inc_off = inc_off.p;
@@ -1076,7 +1109,7 @@ struct vbd_solver {
     }
 
     int tile_launch(const vbd::TileSet& s, void (*fn)(vbd::TileParams), vbd::TileParams& w, int vectors) {
-        const size_t smem = vbd::tile_smem(s.plan.warps, w.ring_chunks, s.plan, C, vectors, s.cluster);
+        const size_t smem = vbd::tile_smem(s.plan.warps, w.ring_chunks, s.chunk_bytes(), s.plan, C, vectors, s.cluster);
         CUDA_TRY(allow_shared(reinterpret_cast<const void*>(fn), s.cluster));
         if (s.cluster) {
             cudaLaunchConfig_t cfg = {};
@@ -1097,6 +1130,12 @@ struct vbd_solver {
                     const float* hg, bool record_energy) {
         VBD_TRY(upload_schedule(iters, accel, rho));
         VBD_TRY(ensure_tile(s));
+        if (s.wrapper && hg) {
+            // every vertex starts from its inertial target, which a tile's ghosts need before the walk
+            vbd::k_predict<<<vbd::nblk(N, 256), 256, 0, stream>>>(x0.p, v.p, xprev.p, y.p, nfree, N, h, hg[0], hg[1], hg[2]);
+            VBD_TRY(check_launch());
+            from_inertia = true;
+        }
         int k0 = 0;
         do {
             int k1 = iters;
@@ -1111,7 +1150,7 @@ struct vbd_solver {
             w.pp = pp.p;
             w.v = v.p;
             w.xprev = xprev.p;
-            w.predict = hg && k0 == 0;
+            w.predict = hg && k0 == 0 && !s.wrapper;
             w.finish = hg && k1 == iters;
             w.from_inertia = from_inertia && k0 == 0;
             w.h = h;
@@ -1120,7 +1159,9 @@ struct vbd_solver {
                 w.hgy = hg[1];
                 w.hgz = hg[2];
             }
-            VBD_TRY(tile_launch(s, vbd::pick_tile<false>(s.plan.lanes, s.plan.warps, s.cluster), w, 1 + two));
+            VBD_TRY(tile_launch(s, s.wrapper ? vbd::pick_tile_wrapper(s.plan.warps)
+                                         : vbd::pick_tile<vbd::kTileForward>(s.plan.lanes, s.plan.warps, s.cluster),
+                                w, 1 + two));
             if (record_energy && k1 > k0 && (k1 - 1) % energy_every == 0) VBD_TRY(emit_energy_append(x0.p));
             k0 = k1;
         } while (k0 < iters);
@@ -1201,7 +1242,7 @@ struct vbd_solver {
                 if (omega > 1.0f) cur ^= 1;
             }
             w.lam_out = cur ? adj_lam2.p : adj_lam.p;
-            VBD_TRY(tile_launch(*tile, vbd::pick_tile<true>(tile->plan.lanes, tile->plan.warps, tile->cluster), w, vectors));
+            VBD_TRY(tile_launch(*tile, vbd::pick_tile<vbd::kTileAdjoint>(tile->plan.lanes, tile->plan.warps, tile->cluster), w, vectors));
         }
         for (int it = 1; it <= sweeps && !walk && !tile; ++it) {
             bool blend = false;
@@ -1374,7 +1415,7 @@ struct vbd_solver {
     // Captured graphs bake in buffer addresses: every (re)allocation or release of the streamed
     // record copies invalidates them.
     int repack_stream() {
-        tset.dirty = aset.dirty = cset.dirty = true;
+        tset.dirty = aset.dirty = cset.dirty = wset.dirty = true;
         if (layout != 1 && irec.p) {
             drop_graphs();
             irec.release();
@@ -1654,6 +1695,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     s->tset.reset(std::move(plan));
     s->aset.reset(vbd::TilePlan());
     s->cset.reset(vbd::TilePlan());
+    s->wset.reset(vbd::TilePlan());
     s->tile_walk = !s->persistent_set && nfree >= vbd::kTileMinVertices;
 
     std::vector<float4> hx(N), hv(N), hy(N);
@@ -1746,7 +1788,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     s->d_cstart.release();
     s->have_materials = tet_mu != nullptr;
     VBD_TRY(s->repack_stream());
-    if (s->use_tile()) VBD_TRY(s->ensure_tile(s->tset));
+    if (s->use_tile()) VBD_TRY(s->ensure_tile(s->walk_tiles()));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     s->ready = true;
     return VBD_OK;
@@ -1909,7 +1951,7 @@ int vbd_solver_solve(vbd_solver* s, int32_t iterations, float dt_sqr_reciprocal,
         return s->launch_walk(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, false, false,
                               init_mode == VBD_INIT_FROM_INERTIA, 1.0f, nullptr);
     if (s->use_tile())
-        return s->launch_tile(s->tset, iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode == VBD_INIT_FROM_INERTIA,
+        return s->launch_tile(s->walk_tiles(), iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode == VBD_INIT_FROM_INERTIA,
                               1.0f, nullptr, false);
     return s->run(key, [&] { return s->emit_solve(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode); });
 }
@@ -1958,7 +2000,7 @@ int vbd_solver_step(vbd_solver* s, float dt, int32_t substeps, int32_t iteration
         if (s->persistent && !s->timing && nenergy == 0)
             VBD_TRY(s->launch_walk(iterations, dtsr, use_acceleration != 0, rho, true, true, false, h, hg));
         else if (s->use_tile())
-            VBD_TRY(s->launch_tile(s->tset, iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0));
+            VBD_TRY(s->launch_tile(s->walk_tiles(), iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0));
         else
             VBD_TRY(s->run(key, [&] {
                 return s->emit_substep(h, dtsr, hg, iterations, use_acceleration != 0, rho, nenergy > 0);
@@ -2258,6 +2300,10 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
             if (value && s->ckpt_every > 0)
                 VBD_FAIL(VBD_ERR_STATE, "recording for the adjoint is on; the adjoint needs the VBDsolver semantics");
             s->semantics = value;
+            if (value && s->ready && s->use_tile()) {
+                VBD_TRY(s->ensure_tile(s->wset));
+                CUDA_TRY(cudaStreamSynchronize(s->stream));
+            }
             return VBD_OK;
         case VBD_OPT_ADJOINT_ALTERNATE:
             s->adj_alternate = value ? 1 : 0;
@@ -2529,6 +2575,12 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
             if (!(rc = beats(overall, best, &better)) && better) best = overall;
         }
         if (!rc) rc = time_of(best, &best_ms);  // the incumbent at this phase's length, for phase 4
+    }
+    // VBD_GPU_Solver semantics: the tile walk against the captured graph
+    if (!rc && s->semantics && s->tset.plan.P > 0) {
+        Cand k = best;
+        k.tile = 1;
+        rc = try_cand(k);
     }
     // Phase 4: the whole step as one persistent colour-walking launch (uniform lanes, no per-colour
     // shape) against the captured graph.

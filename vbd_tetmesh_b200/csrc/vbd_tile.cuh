@@ -82,8 +82,8 @@ struct TileParams {
 // Dynamic shared memory of a CTA: the rings, the local vectors (`vectors` of them, one entry more each),
 // the groups, the internal ids of the own vertices and ghosts, the first ghost of each colour, the first
 // group of each warp and colour, and (cluster exchange) the own vertices' targets.
-inline size_t tile_smem(int warps, int ring_chunks, const TilePlan& p, int ncol, int vectors, bool cluster) {
-    return (size_t)ring_chunks * kTileChunkBytes + 16u * (size_t)(p.max_local + 1) * vectors +
+inline size_t tile_smem(int warps, int ring_chunks, int chunk_bytes, const TilePlan& p, int ncol, int vectors, bool cluster) {
+    return (size_t)ring_chunks * chunk_bytes + 16u * (size_t)(p.max_local + 1) * vectors +
            sizeof(TileGroup) * (size_t)p.max_groups + 4u * (size_t)p.max_ids + 4u * (size_t)(warps + 1) * (ncol + 1) +
            (cluster ? 4u * (size_t)(p.max_own + 1 + p.max_target) : 0u);
 }
@@ -156,26 +156,27 @@ struct TileRing {
     int slot;              // slot of the next chunk to sweep
 };
 
+template <int kBytes>
 __device__ __forceinline__ void ring_issue(const TileParams& p, TileRing& r, unsigned buf, int slot, int lane) {
-    constexpr int kBytes = kTileChunkBytes;
-    static_assert(kBytes == 5 * 512 + 256, "176 pieces of 16 bytes");
+    constexpr int kFull = kBytes / 512;
+    static_assert(kBytes == kFull * 512 + 256, "16-byte pieces, the last of half the lanes");
     if (r.left > 0) {
         const char* src = reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kBytes + 16 * lane;
         const unsigned dst = buf + (unsigned)(slot * kBytes + 16 * lane);
 #pragma unroll
-        for (int i = 0; i < 5; ++i)
+        for (int i = 0; i < kFull; ++i)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512 * i), "l"(src + 512 * i) : "memory");
         if (lane < 16)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 2560), "l"(src + 2560) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512 * kFull), "l"(src + 512 * kFull) : "memory");
         --r.left;
         if (++r.next == r.end) r.next = r.first;
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 // The same as one bulk copy, completing on the slot's mbarrier (W = 16).
+template <unsigned kBytes>
 __device__ __forceinline__ void ring_issue_bulk(const TileParams& p, TileRing& r, unsigned buf, unsigned bar, int slot,
                                                 int lane) {
-    constexpr unsigned kBytes = kTileChunkBytes;
     if (r.left <= 0) return;
     if (lane == 0) {
         mbar_expect(bar + 8u * slot, kBytes);
@@ -416,6 +417,180 @@ __device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, f
     }
 }
 
+// The corotated element of VBD_GPU_Solver semantics (corot_block) for two records at once: every
+// operation rounds as nvcc contracts corot_block, so that the sums have k_sweep_wrapper's bits.  The
+// minors of the row-0 determinant are the cofactors of row 0 (the middle one negated); the middle one,
+// which appears with both signs, is a difference of two rounded products.
+// Padding repeats a record of its vertex and is not added.
+__device__ __forceinline__ float cross1(float a, float b, float c, float d) { return fmaf(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ float dot1(float a0, float b0, float a1, float b1, float a2, float b2) {
+    return fmaf(a2, b2, fmaf(a0, b0, __fmul_rn(a1, b1)));
+}
+// The difference of two products, each rounded: ptxas contracts mul.rn.f32x2 into add.rn.f32x2, which the scalar
+// instruction prevents.
+__device__ __forceinline__ F2 sub_rn(F2 a, F2 b) {
+    return f2(__fsub_rn(f2_lo(a), f2_lo(b)), __fsub_rn(f2_hi(a), f2_hi(b)));
+}
+struct CorotSums {
+    float h[9], f[3];
+};
+__device__ __forceinline__ void tile_corot(const char* buf, int lane, const float4* X, CorotSums& acc) {
+    auto two = [&](int k) { return reinterpret_cast<const ulonglong2*>(buf)[32 * k + lane]; };
+    const int4 id = reinterpret_cast<const int4*>(buf)[224 + lane];
+    F2 F[3][3];
+    {
+        const unsigned a0 = id.x, a1 = id.y, b0 = id.z, b1 = id.w;
+        const float4 pa = X[a0 & 0xffffu], pb = X[b0 & 0xffffu];
+        const float4 qa[3] = {X[a0 >> 16], X[a1 & 0xffffu], X[(a1 >> 16) & 0x7fffu]};
+        const float4 qb[3] = {X[b0 >> 16], X[b1 & 0xffffu], X[(b1 >> 16) & 0x7fffu]};
+        F2 d[3][3];  // [axis][column]
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            d[0][k] = f2(qa[k].x - pa.x, qb[k].x - pb.x);
+            d[1][k] = f2(qa[k].y - pa.y, qb[k].y - pb.y);
+            d[2][k] = f2(qa[k].z - pa.z, qb[k].z - pb.z);
+        }
+        const ulonglong2 m01 = two(0), m23 = two(1), m45 = two(2), m67 = two(3);
+        const F2 m8 = two(4).x;
+        const F2 M[3][3] = {{m01.x, m01.y, m23.x}, {m23.y, m45.x, m45.y}, {m67.x, m67.y, m8}};
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) F[a][b] = dot2(d[a][0], M[0][b], d[a][1], M[1][b], d[a][2], M[2][b]);
+    }
+    F2 R[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) R[a][b] = F[a][b];
+    const F2 half = f2(0.5f, 0.5f);
+#pragma unroll 1
+    for (int it = 0; it < 5; ++it) {
+        F2 C[3][3];
+        const F2 n1[3] = {neg2(R[1][0]), neg2(R[1][1]), neg2(R[1][2])};
+        const F2 n2[3] = {neg2(R[2][0]), neg2(R[2][1]), neg2(R[2][2])};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+            C[0][i] = i == 1 ? sub_rn(mul2(R[1][2], R[2][0]), mul2(R[1][0], R[2][2]))
+                             : cross2n(R[1][i1], R[2][i2], n1[i2], R[2][i1]);
+            C[1][i] = cross2n(R[2][i1], R[0][i2], n2[i2], R[0][i1]);
+            C[2][i] = cross2n(R[0][i1], R[1][i2], R[0][i2], n1[i1]);
+        }
+        const F2 det = dot2(R[0][0], C[0][0], R[0][1], C[0][1], R[0][2], C[0][2]);
+        const float da = f2_lo(det), db = f2_hi(det);
+        const bool stop_a = fabsf(da) < 1e-8f, stop_b = fabsf(db) < 1e-8f;
+        const F2 inv = f2(__frcp_rn(da), __frcp_rn(db));
+        if (!stop_a && !stop_b) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) R[a][b] = mul2(half, fma2(C[a][b], inv, R[a][b]));
+        } else {  // a record whose steps have ended keeps its R (and ends here again next time)
+            if (stop_a && stop_b) break;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const F2 n = mul2(half, fma2(C[a][b], inv, R[a][b]));
+                    R[a][b] = f2(stop_a ? f2_lo(R[a][b]) : f2_lo(n), stop_b ? f2_hi(R[a][b]) : f2_hi(n));
+                }
+        }
+    }
+    F2 tr = 0ull;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) tr = fma2(R[a][b], F[a][b], tr);
+    tr = add2(tr, f2(-3.f, -3.f));
+    const ulonglong2 q01 = two(5), qv = two(6);
+    const F2 q0 = two(4).y, q1 = q01.x, q2 = q01.y, vol = qv.x, m2 = qv.y;  // m2 = 2 mu
+    const F2 lam = reinterpret_cast<const F2*>(buf + 256 * 16)[lane];
+    const F2 lt = mul2(lam, tr), nvol = neg2(vol), diag = dot2(q0, q0, q1, q1, q2, q2);
+    F2 RQ[3], lr[3];
+    const bool va = (id.y >= 0), vb = (id.w >= 0);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        F2 P[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) P[b] = fma2(lt, R[a][b], mul2(m2, sub2(F[a][b], R[a][b])));
+        const F2 s = dot2(P[0], q0, P[1], q1, P[2], q2);
+        if (va) acc.f[a] = fmaf(f2_lo(nvol), f2_lo(s), acc.f[a]);
+        if (vb) acc.f[a] = fmaf(f2_hi(nvol), f2_hi(s), acc.f[a]);
+        RQ[a] = dot2(R[a][0], q0, R[a][1], q1, R[a][2], q2);
+        lr[a] = mul2(lam, RQ[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const F2 in = a == b ? fma2(m2, diag, mul2(lr[a], RQ[a])) : fma2(lr[a], RQ[b], 0ull);
+            if (va) acc.h[3 * a + b] = fmaf(f2_lo(vol), f2_lo(in), acc.h[3 * a + b]);
+            if (vb) acc.h[3 * a + b] = fmaf(f2_hi(vol), f2_hi(in), acc.h[3 * a + b]);
+        }
+}
+
+// k_sweep_wrapper's update of a vertex from its 16 threads' sums: thread t < 12 adds component t in lane order,
+// then every thread solves.  `red` holds 32 x 13 floats of the warp.
+__device__ __forceinline__ float4 wrapper_update(const CorotSums& acc, float* red, int lane, float4 xi, float4 y,
+                                                 float dtsr, unsigned long long* status, bool count) {
+    const int slot = lane >> 4, t = lane & 15;
+    __syncwarp();  // the last group's sums have been read
+#pragma unroll
+    for (int k = 0; k < 9; ++k) red[13 * lane + k] = acc.h[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) red[13 * lane + 9 + k] = acc.f[k];
+    __syncwarp();
+    const float coeff = __fmul_rn(y.w, dtsr);
+    float s = t == 9    ? __fmul_rn(coeff, __fsub_rn(y.x, xi.x))
+              : t == 10 ? __fmul_rn(coeff, __fsub_rn(y.y, xi.y))
+              : t >= 11 ? __fmul_rn(coeff, __fsub_rn(y.z, xi.z))
+              : t % 4 == 0 ? __fmul_rn(coeff, 1.000001f)
+                           : 0.0f;
+    const float* col = red + 13 * 16 * slot + min(t, 11);
+#pragma unroll
+    for (int src = 0; src < 16; ++src) s = __fadd_rn(s, col[13 * src]);
+    float A[3][3], f[3], C[3][3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) A[k / 3][k % 3] = __shfl_sync(0xffffffffu, s, k, 16);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) f[k] = __shfl_sync(0xffffffffu, s, 9 + k, 16);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+        C[0][i] = i == 1 ? __fsub_rn(__fmul_rn(A[1][2], A[2][0]), __fmul_rn(A[1][0], A[2][2]))
+                         : cross1(A[1][i1], A[2][i2], A[1][i2], A[2][i1]);
+        C[1][i] = cross1(A[2][i1], A[0][i2], A[2][i2], A[0][i1]);
+        C[2][i] = cross1(A[0][i1], A[1][i2], A[0][i2], A[1][i1]);
+    }
+    const float det = dot1(A[0][0], C[0][0], A[0][1], C[0][1], A[0][2], C[0][2]);
+    float4 xn = xi;
+    if (fabsf(det) < 1.0e-8f) {
+        if (count) atomicAdd(status + ST_SINGULAR, 1ull);
+    } else {
+        const float inv = __frcp_rn(det);
+        xn.x = fmaf(inv, dot1(C[0][0], f[0], C[1][0], f[1], C[2][0], f[2]), xi.x);
+        xn.y = fmaf(inv, dot1(C[0][1], f[0], C[1][1], f[1], C[2][1], f[2]), xi.y);
+        xn.z = fmaf(inv, dot1(C[0][2], f[0], C[1][2], f[1], C[2][2], f[2]), xi.z);
+    }
+    return xn;
+}
+
+// Local id of vertex v in a tile: an own vertex's, or by its place among the tile's ghosts and pinned neighbours
+// (ascending ids).
+__device__ __forceinline__ int tile_local(int v, int tile, const TileHead& h, const int* lid, const int* vtile,
+                                          const int* vlocal, int nfree) {
+    if (v < nfree && vtile[v] == tile) return vlocal[v];
+    const int* e = lid + h.lid + h.nown;
+    int lo = 0, hi = h.nghost + h.npinned;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (e[mid] < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return h.nown + lo;
+}
+
 // Record chunks from the packed incidence records (layout 3 or 4): a chunk holds one round of a group;
 // vertex slot k's threads t take incidences r L + t and r L + t + L/2.  Neighbour ids become local.
 template <int LAYOUT>
@@ -432,17 +607,7 @@ __global__ void __launch_bounds__(256) k_pack_tile(SweepParams p, const int* __r
     const TileHead h = head[tile];
     const int T = lanes / 2;
     const int slot = lane / T, t = lane % T;
-    auto local = [&](int v) {
-        if (v < nfree && vtile[v] == tile) return vlocal[v];
-        const int* e = lid + h.lid + h.nown;  // ghosts and pinned neighbours, ascending ids
-        int lo = 0, hi = h.nghost + h.npinned;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (e[mid] < v) lo = mid + 1;
-            else hi = mid;
-        }
-        return h.nown + lo;
-    };
+    auto local = [&](int v) { return tile_local(v, tile, h, lid, vtile, vlocal, nfree); };
     FactRec r[2];
     int id0[2], id1[2];
     const int self = g.lv + min(slot, g.count - 1);  // padding: the vertex itself
@@ -467,6 +632,56 @@ __global__ void __launch_bounds__(256) k_pack_tile(SweepParams p, const int* __r
     reinterpret_cast<float2*>(o + 160)[lane] = make_float2(r[0].detm, r[1].detm);
 }
 
+// The chunks of VBD_GPU_Solver semantics, from the tet records: slot k's threads t take incidences 32 r + t and
+// 32 r + t + 16.  A pair of fields per thread: Dm^-1 (9), Dm^-1's row of the vertex q (3), V0, 2 mu, then the
+// tets' local ids (bit 31 of the second word: padding, a repeated record), then lambda.
+__global__ void __launch_bounds__(256) k_pack_wrapper(const int* __restrict__ inc_off, const int* __restrict__ inc_tet,
+                                                      const TetRec* __restrict__ rec, const int* __restrict__ table,
+                                                      int nchunks, const TileGroup* __restrict__ groups,
+                                                      const TileHead* __restrict__ head, const int* __restrict__ lid,
+                                                      const int* __restrict__ vtile, const int* __restrict__ vlocal,
+                                                      int nfree, float4* __restrict__ out) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= nchunks) return;
+    const int tile = table[3 * i], round = table[3 * i + 2];
+    const TileGroup g = groups[table[3 * i + 1]];
+    const TileHead h = head[tile];
+    const int slot = lane >> 4, t = lane & 15;
+    const int v = g.gv + min(slot, g.count - 1), self = g.lv + min(slot, g.count - 1);
+    const int j0 = inc_off[v], j1 = inc_off[v + 1];
+    float fld[15][2];
+    int ids[2][2];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const int j = j0 + kWrapperTileLanes * round + t + 16 * b;
+        const bool valid = slot < g.count && j < j1;
+        for (int k = 0; k < 15; ++k) fld[k][b] = 0.f;
+        int l[4] = {self, self, self, self};
+        if (j1 > j0) {
+            const TetRec r = rec[inc_tet[valid ? j : j0]];
+            const int q[4] = {r.ids.x, r.ids.y, r.ids.z, r.ids.w};
+            const float D[9] = {r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, r.b.w, r.c.x};
+            const int n = q[0] == v ? 0 : q[1] == v ? 1 : q[2] == v ? 2 : 3;
+            for (int k = 0; k < 9; ++k) fld[k][b] = D[k];
+            for (int k = 0; k < 3; ++k)
+                fld[9 + k][b] = n == 0 ? -D[k] - D[3 + k] - D[6 + k] : D[3 * (n - 1) + k];
+            fld[12][b] = r.c.y;
+            fld[13][b] = 2.0f * r.c.z;
+            fld[14][b] = r.c.w;
+            for (int k = 0; k < 4; ++k) l[k] = tile_local(q[k], tile, h, lid, vtile, vlocal, nfree);
+        }
+        ids[b][0] = l[0] | (l[1] << 16);
+        ids[b][1] = l[2] | (l[3] << 16) | (valid ? 0 : (int)0x80000000u);
+    }
+    float4* o = out + (size_t)i * (kWrapperChunkBytes / 16);
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+        o[32 * k + lane] = make_float4(fld[2 * k][0], fld[2 * k][1], fld[2 * k + 1][0], fld[2 * k + 1][1]);
+    reinterpret_cast<int4*>(o)[224 + lane] = make_int4(ids[0][0], ids[0][1], ids[1][0], ids[1][1]);
+    reinterpret_cast<float2*>(o + 256)[lane] = make_float2(fld[14][0], fld[14][1]);
+}
+
 // T threads per vertex (2 T lanes' partial sums, two per thread in the two-wide FP32 instructions), W warps.
 // W = 8 is the form for tiles with little work per colour, where a colour lasts as long as one vertex's
 // dependency chain: everything that does not depend on the neighbours is fetched before the barrier, and
@@ -482,13 +697,19 @@ __global__ void __launch_bounds__(256) k_pack_tile(SweepParams p, const int* __r
 // that receiver computed after that wait (the argument for the words, above), so one barrier per colour
 // is enough, armed for the next iteration when its wait ends; bytes that arrive before that are held
 // against the same phase.
-template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
+enum TileKind { kTileForward, kTileAdjoint, kTileWrapper };
+template <int T, TileKind KIND, int W, bool CL = false>
+__global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     extern __shared__ __align__(16) unsigned char tsm[];
+    constexpr bool ADJ = KIND == kTileAdjoint, WRAP = KIND == kTileWrapper;
+    constexpr int kBytes = WRAP ? kWrapperChunkBytes : kTileChunkBytes;
+    static_assert(!WRAP || (T == 16 && !CL), "two vertices a warp");
     constexpr int NT = W * 32;
     constexpr bool LAT = W <= 8;
     static_assert(LAT || !CL, "the cluster exchange is the W = 8 form's");
     __shared__ __align__(8) unsigned long long bars[LAT ? 1 : W * kTileMaxRing];
     __shared__ __align__(8) unsigned long long cbars[CL ? kTileMaxColours : 1];
+    __shared__ float red[WRAP ? W * 32 * 13 : 1];
     __shared__ float4 stage[LAT ? 1 : W * 64 / T];  // W = 16: own data of each warp's next group
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x;
@@ -498,8 +719,8 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
     const int2 ws = p.wstream[tile * W + warp];
     const int slots = resident ? ws.y : p.ring;  // of this warp's ring
     char* ring_buf = reinterpret_cast<char*>(tsm) +
-                     (size_t)(resident ? ws.x - p.wstream[tile * W].x : warp * p.ring) * kTileChunkBytes;
-    float4* sx = reinterpret_cast<float4*>(tsm + (size_t)p.ring_chunks * kTileChunkBytes);  // x (or lambda)
+                     (size_t)(resident ? ws.x - p.wstream[tile * W].x : warp * p.ring) * kBytes;
+    float4* sx = reinterpret_cast<float4*>(tsm + (size_t)p.ring_chunks * kBytes);  // x (or lambda)
     float4* sb = sx + (two ? p.max_local + 1 : 0);                  // the blended buffer
     float4* sX = sb + (ADJ ? p.max_local + 1 : 0);                  // adjoint: X
     TileGroup* sg = reinterpret_cast<TileGroup*>(sX + p.max_local + 1);
@@ -526,8 +747,8 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
         __syncwarp();
     }
     for (int i = 0; i < slots; ++i) {
-        if (LAT) ring_issue(p, ring, ring_smem, i, lane);
-        else ring_issue_bulk(p, ring, ring_smem, bar, i, lane);
+        if (LAT) ring_issue<kBytes>(p, ring, ring_smem, i, lane);
+        else ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, i, lane);
     }
     if (!CL && tid == 0) atomicAdd(p.arrived, 1ull);
 
@@ -644,7 +865,7 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
     // barrier that precedes its sweep, and its slots are refilled after its results are out.  W = 16: a
     // chunk is waited for when it is swept and refilled right after.
     const int pending = resident ? 0 : p.ring - p.max_rounds;
-    auto chunk_at = [&](int s) { return TilePair{ring_buf + s * kTileChunkBytes, lane}; };
+    auto chunk_at = [&](int s) { return TilePair{ring_buf + s * kBytes, lane}; };
     auto next_slot = [&](int s) { return s + 1 == slots ? 0 : s + 1; };
     if (p.k1 > p.k0 && wlast > wfirst) {
         load_group(wfirst);
@@ -682,8 +903,18 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
                     rounds = g.rounds;
                 }
                 Acc2 acc2;
-                acc2.zero();
-                if constexpr (LAT) {
+                CorotSums sums;
+                if constexpr (WRAP) {
+#pragma unroll
+                    for (int i = 0; i < 9; ++i) sums.h[i] = 0.f;
+                    sums.f[0] = sums.f[1] = sums.f[2] = 0.f;
+                } else {
+                    acc2.zero();
+                }
+                if constexpr (LAT && WRAP) {
+                    for (int at = ring.slot, left = rounds; left > 0; --left, at = next_slot(at))
+                        tile_corot(ring_buf + at * kBytes, lane, xs, sums);
+                } else if constexpr (LAT) {
                     // two chunks at a time: their gathers and products are independent, the sums in order
                     int at = ring.slot, left = rounds;
                     for (; left > 1; left -= 2) {
@@ -709,10 +940,11 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
                         ring.slot = next_slot(used);
                         if (ring.slot == 0) parity ^= 1u;
                         const TilePair rec = chunk_at(used);
-                        if constexpr (ADJ) tile_adjoint(rec, rec.ids(), xi, sX, xs, p.max_local, acc2);
+                        if constexpr (WRAP) tile_corot(rec.buf, lane, xs, sums);
+                        else if constexpr (ADJ) tile_adjoint(rec, rec.ids(), xi, sX, xs, p.max_local, acc2);
                         else tile_contrib(rec, rec.ids(), xi, xs, acc2);
                         __syncwarp();  // every lane has read slot `used`
-                        ring_issue_bulk(p, ring, ring_smem, bar, used, lane);
+                        ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, used, lane);
                     }
                 }
                 // W = 16 reads the group again instead of holding it
@@ -721,18 +953,24 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
                 const int lv = g.lv + slot, gv = g.gv + slot;
                 // lanes t and t + T, then the T threads: group_reduce's order for 2 T lanes.  Every thread of the
                 // vertex ends with the same sums.
-                Acc acc = acc2.sum();
-                group_reduce<T>(acc);
+                Acc acc;
+                if constexpr (!WRAP) {
+                    acc = acc2.sum();
+                    group_reduce<T>(acc);
+                }
                 float4 y = own, q = prev;
                 if (!LAT) {
                     ring_wait_for<0>();
                     __syncwarp();
-                    if (active && t == 0) {
+                    if (active && (WRAP || t == 0)) {
                         y = my_stage[0];
                         q = my_stage[1];
                         if constexpr (ADJ) mass = __ldg(&p.y[gv].w);
                     }
                 }
+                float4 xw;
+                if constexpr (WRAP)
+                    xw = wrapper_update(sums, red + warp * 32 * 13, lane, xi, y, p.dtsr, p.status, active && t == 0);
                 if (active && (CL || t == 0)) {
                     float4 xn, xa = zero4, old;
                     if constexpr (ADJ) {
@@ -740,7 +978,8 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
                         xn = adj_block_solve(acc, mass, p.dtsr, y);
                     } else {
                         old = xi;
-                        xn = block_update(acc, xi, y, p.dtsr, p.status, t == 0);
+                        if constexpr (WRAP) xn = xw;
+                        else xn = block_update(acc, xi, y, p.dtsr, p.status, t == 0);
                     }
                     if (CL) {
                         if (blend) xa = ADJ ? adj_blend(xn, q, om) : cheb_blend(xn, q, om);
@@ -775,7 +1014,7 @@ template <int T, bool ADJ, int W, bool CL = false> __global__ void __launch_boun
                     if (ring.slot >= slots) ring.slot = 0;
                 } else if (LAT) {
                     for (; rounds > 0; --rounds) {
-                        ring_issue(p, ring, ring_smem, ring.slot, lane);
+                        ring_issue<kBytes>(p, ring, ring_smem, ring.slot, lane);
                         ring.slot = next_slot(ring.slot);
                     }
                     ring_wait(pending);

@@ -10,6 +10,10 @@ namespace vbd {
 constexpr int kTileMaxWarps = 16;           // warps of a tile's CTA: 8 or 16 (TilePlan::warps)
 constexpr int kTileChunk = 64;              // incidences per record chunk: two per thread of a warp
 constexpr int kTileChunkBytes = kTileChunk * 44;
+// VBD_GPU_Solver semantics: a chunk holds two vertices' incidences (16 threads each, two incidences per thread)
+constexpr int kWrapperTileLanes = 32;
+constexpr int kWrapperChunkBytes = kTileChunk * 68;
+constexpr int kWrapperMaxLocal = 32767;     // the 16th bit of an id marks padding
 constexpr int kTileMaxRing = 6;             // chunks a warp's ring holds at most
 constexpr int kTileMaxLocal = 65535;        // local vertex ids are 16 bits
 // A mesh gets a plan from this many free vertices.  Microseconds per colour of a step, tile walk against
