@@ -123,3 +123,81 @@ def test_two_solvers_on_two_threads(gpu_device):
         solvers[k].close()
         for a, b in zip(alone[k], out[k]):
             np.testing.assert_array_equal(a, b)
+
+
+def delaunay(n, seed, around=60):
+    """A Delaunay mesh of n random points and a centre with `around` points about it: valences from 4 to 40 and,
+    at the centre, to twice `around`."""
+    from scipy.spatial import Delaunay
+
+    rng = np.random.default_rng(seed)
+    shell = rng.normal(size=(around, 3))
+    shell = 0.5 + 0.12 * shell / np.linalg.norm(shell, axis=1)[:, None]
+    pts = np.concatenate([rng.uniform(0, 1, (n, 3)), shell, [[0.5, 0.5, 0.5]]])
+    pts = pts[(np.linalg.norm(pts - 0.5, axis=1) > 0.119) | (np.arange(len(pts)) == len(pts) - 1)]
+    tets = Delaunay(pts).simplices.astype(np.int32)
+    e = pts[tets[:, 1:]] - pts[tets[:, :1]]
+    vol = np.linalg.det(e) / 6
+    tets[vol < 0, 2:] = tets[vol < 0, 3:1:-1]
+    tets = tets[np.abs(vol) > 2e-6]
+    p = pts.astype(np.float32)
+    mu, lam = meshgen.lame(1e5, 0.3)
+    t = len(tets)
+    return meshgen.Mesh(p.copy(), p.copy(), np.zeros_like(p), tets, (p[:, 0] < 0.1).astype(np.uint8),
+                        np.full(t, mu, np.float32), np.full(t, lam, np.float32))
+
+
+# more incidences per vertex than one round holds, at every lane count
+@pytest.mark.parametrize("lanes,around", [(4, 60), (8, 60), (16, 60), (16, 12)])
+def test_tile_walk_high_valence_equals_graph(gpu_device, lanes, around):
+    m = delaunay(900, 1, around)
+    assert np.bincount(m.tets.ravel()).max() > 32
+
+    def run(s):
+        out = step(s, 1 / 240, 6, True)
+        s.record(2)
+        s.step(1 / 240, 5, G, True, 0.9)
+        return [*out, *s.backward(np.ones((m.num_verts, 3)), None, 6, 0.9)]
+
+    both(lambda: build_solver(m, lanes=lanes), run)
+
+
+# VBD_GPU_Solver semantics: 8 and 16 warps, records resident and streamed, two rounds per vertex, ragged groups,
+# large initial velocities (the corotated steps have work to do), a batch
+@pytest.mark.parametrize("make", [
+    lambda: meshgen.jittered_block(7, 6, 5, seed=5, per_tet_sigma=0.3), lambda: meshgen.cube(18), lambda: meshgen.cube(26),
+    lambda: delaunay(900, 2), lambda: meshgen.concat(meshgen.batched_blocks(num_meshes=9, lo=2, hi=9, seed=4)),
+], ids=["block", "cube18", "cube26", "delaunay", "batch"])
+def test_wrapper_semantics_tile_equals_graph(gpu_device, make):
+    m = make()
+
+    def run(s):
+        s.set_option(_capi.OPT_SEMANTICS, 1)
+        out = [*step(s, 1 / 120, 10, True)]
+        s.set_materials(m.mu * 2, m.lam * 3)
+        out += [*step(s, 1 / 120, 7, False, substeps=2, steps=1)]
+        s.update_inertia_from_cpu(m.x)
+        for mode in (0, 1):
+            s.solve_vbd(6, 14400.0, True, 0.9, mode)
+            out.append(s.get_positions())
+        return out
+
+    both(lambda: build_batch_solver(m) if isinstance(m, meshgen.Batch) else build_solver(m), run)
+
+
+def test_wrapper_semantics_degenerate_elements_equal_graph(gpu_device):
+    """Elements whose rotation steps stop at |det| < 1e-8 (flattened cells) and non-finite positions."""
+    m = meshgen.jittered_block(9, 8, 7, seed=6)
+    m.x = m.x.copy()
+    m.x[(m.ijk[:, 0] >= 4) & (m.ijk[:, 0] <= 6), 0] = 0.25
+    m.x[100] = m.x[101]
+    m.x[300, 2], m.x[301, 1] = np.nan, np.inf
+
+    def run(s):
+        s.set_option(_capi.OPT_SEMANTICS, 1)
+        s.update_inertia_from_cpu(m.x)
+        s.solve_vbd(2, 3600.0, True, 0.9, 0)
+        x = s.get_positions()
+        return x, np.array(s.status())
+
+    both(lambda: build_solver(m), run)

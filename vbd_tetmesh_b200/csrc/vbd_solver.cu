@@ -118,17 +118,18 @@ template <int L> static void (*pick_cluster_adjoint(int layout))(AdjWalkParams) 
 
 // The tile walk runs lanes / 2 threads per vertex; it reads its own record chunks, packed from the
 // factored records of either layout.  With `cluster` the tiles are the CTAs of one cluster.
-template <TileKind KIND> static void (*pick_tile(int lanes, int warps, bool cluster))(TileParams) {  // adjoint: 8 warps
-    if (cluster)
-        return lanes == 4    ? &k_tile_walk<2, KIND, 8, true>
-               : lanes == 8  ? &k_tile_walk<4, KIND, 8, true>
-               : lanes == 16 ? &k_tile_walk<8, KIND, 8, true>
-                             : &k_tile_walk<16, KIND, 8, true>;
-    if (KIND == kTileAdjoint || warps == 8)
-        return lanes == 4 ? &k_tile_walk<2, KIND, 8> : lanes == 8 ? &k_tile_walk<4, KIND, 8> : &k_tile_walk<8, KIND, 8>;
-    return lanes == 4   ? &k_tile_walk<2, kTileForward, 16>
-           : lanes == 8 ? &k_tile_walk<4, kTileForward, 16>
-                        : &k_tile_walk<8, kTileForward, 16>;
+template <TileKind KIND, int W, bool CL> static void (*pick_tile_form(int lanes, bool stack))(TileParams) {
+    if (stack)
+        return lanes == 8    ? &k_tile_walk<4, KIND, W, CL, true>
+               : lanes == 16 ? &k_tile_walk<8, KIND, W, CL, true>
+                             : &k_tile_walk<16, KIND, W, CL, true>;
+    if (CL && lanes == 32) return &k_tile_walk<16, KIND, 8, true>;
+    return lanes == 4 ? &k_tile_walk<2, KIND, W, CL> : lanes == 8 ? &k_tile_walk<4, KIND, W, CL> : &k_tile_walk<8, KIND, W, CL>;
+}
+template <TileKind KIND> static void (*pick_tile(const TilePlan& p, bool cluster))(TileParams) {  // adjoint: 8 warps
+    if (cluster) return pick_tile_form<KIND, 8, true>(p.lanes, p.stack);
+    if (KIND == kTileAdjoint || p.warps == 8) return pick_tile_form<KIND, 8, false>(p.lanes, p.stack);
+    return pick_tile_form<kTileForward, 16, false>(p.lanes, p.stack);
 }
 static void (*pick_tile_wrapper(int warps))(TileParams) {
     return warps == 8 ? &k_tile_walk<16, kTileWrapper, 8> : &k_tile_walk<16, kTileWrapper, 16>;
@@ -142,7 +143,8 @@ struct TileSet {
     int chunk_bytes() const { return wrapper ? kWrapperChunkBytes : kTileChunkBytes; }
     bool dirty = true;        // the chunks must be packed again (new records)
     int layout = 0;           // layout they were packed from
-    int lanes = 0;            // lanes the device lists are for
+    int sums = 0;             // the solver's lanes the plan's groups are for
+    int lanes = 0, warps = 0; // the plan's lanes and warps the device lists are for
     // One allocation: the exchanged words and the start counter, the record chunks, the plan's lists.
     DBuf<float4> mem;
     float4 *words = nullptr, *chunk = nullptr;
@@ -160,7 +162,7 @@ struct TileSet {
     void reset(TilePlan&& p) {
         plan = std::move(p);
         dirty = true;
-        lanes = 0;
+        sums = lanes = 0;
         checked[0] = checked[1] = nullptr;
     }
 };
@@ -315,7 +317,7 @@ struct vbd_solver {
     // the tile walk (vbd_tile.cuh): its plan for the mesh, whether it runs in place of the captured
     // graph (chosen at init or by the autotuner, off once VBD_OPT_PERSISTENT is set), and its device data
     vbd::TileSet tset;   // one tile per SM, exchanging words through L2
-    vbd::TileSet aset;   // tset's tiles swept by 8 warps, for the adjoint where tset has 16
+    vbd::TileSet aset;   // tset's tiles as the adjoint sweeps them, where tset has 16 warps or would not stay resident
     vbd::TileSet wset;   // tset's tiles for VBD_GPU_Solver semantics
     vbd::TileSet cset;   // one tile per CTA of a cluster, its plan merged from tset's tiles
     int tile_walk = 0;
@@ -889,10 +891,24 @@ struct vbd_solver {
         return s.plan.max_local <= (s.wrapper ? vbd::kWrapperMaxLocal : vbd::kTileMaxLocal) &&
                (tile_resident(s, vectors) || tile_ring(s, vectors) >= (s.plan.warps == 8 ? s.plan.max_rounds : 2));
     }
-    // Warps of the tile CTAs for the current lanes.
-    int tile_warps() const {
-        const double groups = (double)nfree / std::max(1, C) / std::max(1, tset.plan.P) * lanes / vbd::kTileChunk;
-        return groups <= vbd::kTileFewGroups && (max_valence + lanes - 1) / lanes <= vbd::kTileMaxRing / 2 ? 8 : 16;
+    // Cuts a set's tiles into groups for L lanes and CTAs of `warps` warps (0: chosen here).  A thread's two
+    // incidences are those of two lanes, or (stack) of one lane in turn: half the rounds, and twice the
+    // threads, shuffles and solves per vertex.  Stacked where the SM's four schedulers then have about one
+    // group of a colour each, so that a colour lasts one vertex's chain: microseconds a colour stacked / not,
+    // 16x4x4 beam 1.30 / 1.39, 16^3 cube 1.45 / 1.51, 32x8x8 beam 1.37 / 1.48 (its adjoint 1.52 / 1.80); with
+    // more groups 8 beams 1.62 / 1.50, 24^3 2.16 / 1.84, and with 16 warps 32^3 3.22 / 2.74, 64^3 10.5 / 8.4.
+    void group_tiles(vbd::TileSet& s, int L, int warps, int vectors) {
+        const double groups = (double)nfree / std::max(1, C) / std::max(1, s.plan.P) * L / vbd::kTileChunk;
+        const int rounds = (max_valence + L - 1) / L;
+        const bool few = groups <= vbd::kTileFewGroups && rounds <= vbd::kTileMaxRing / 2;
+        const int w = warps ? warps : few ? 8 : 16;
+        s.sums = L;
+        s.plan.stack = L <= 16 && rounds > 1 && w == 8;
+        vbd::tile_groups(&s.plan, s.plan.stack ? 2 * L : L, w, h_inc_off.data());
+        if (s.plan.stack && (s.plan.max_colour_groups > vbd::kTileStackGroups || !tile_resident(s, vectors))) {
+            s.plan.stack = false;
+            vbd::tile_groups(&s.plan, L, w, h_inc_off.data());
+        }
     }
     // Whether steps and solves run as tile walks.  Under a caller's stream capture they do not: each
     // launch needs tags of its own, which a replayed launch would repeat.
@@ -913,25 +929,26 @@ struct vbd_solver {
                 wset.reset(std::move(q));
                 wset.wrapper = true;
             }
-        } else if (tset.plan.lanes != lanes) {
-            vbd::tile_groups(&tset.plan, lanes, tile_warps(), h_inc_off.data());
+        } else if (tset.sums != lanes) {
+            group_tiles(tset, lanes, 0, 2);
         }
         return tile_fits(walk_tiles(), 1);
     }
     vbd::TileSet& walk_tiles() { return semantics ? wset : tset; }
-    // Groups per colour and tile up to which 8 warps sweep them.
+    // Warps of VBD_GPU_Solver semantics: microseconds per colour with 8 / 16, 16^3 cube (2 groups a colour and
+    // tile) 2.56 / 2.91, 24^3 (6) 4.5 / 3.8, 32^3 7.5 / 6.4.
     int wrapper_warps() const {
         const double groups = (double)nfree / std::max(1, C) / std::max(1, tset.plan.P) * vbd::kWrapperTileLanes / vbd::kTileChunk;
-        return groups <= vbd::kTileFewGroups && max_valence <= vbd::kWrapperTileLanes * (vbd::kTileMaxRing / 2) ? 8 : 16;
+        return groups <= vbd::kWrapperFewGroups && max_valence <= vbd::kWrapperTileLanes * (vbd::kTileMaxRing / 2) ? 8 : 16;
     }
     // The adjoint's tiles: its kernel takes more than the 128 registers of 16 warps (with them it spills: 5.2 us
     // a colour against 4.2 with 8 warps for the adjoint of 64 beams).
     vbd::TileSet& adjoint_tiles() {
-        if (tset.plan.warps == 8) return tset;
-        if (aset.plan.lanes != lanes) {
+        if (tset.plan.warps == 8 && (!tset.plan.stack || tile_resident(tset, 3))) return tset;
+        if (aset.sums != lanes) {
             vbd::TilePlan q = tset.plan;
-            vbd::tile_groups(&q, lanes, 8, h_inc_off.data());
             aset.reset(std::move(q));
+            group_tiles(aset, lanes, 8, 3);
         }
         return aset;
     }
@@ -941,17 +958,17 @@ struct vbd_solver {
     bool cluster_tiles(int L, bool adjoint) {
         if (tset.plan.P == 0 || C > vbd::kTileMaxColours || layout < 3) return false;
         const int P = std::min({16, tset.plan.P, cluster_ctas_opt > 0 ? cluster_ctas_opt : std::max(1, nfree / vbd::kClusterTileMin)});
-        if (cset.plan.P != P || cset.plan.lanes != L) {
+        if (cset.plan.P != P || cset.sums != L) {
             vbd::TilePlan q;
             vbd::tile_merge(tset.plan, P, cstart, &q);
-            vbd::tile_groups(&q, L, 8, h_inc_off.data());
             cset.reset(std::move(q));
             cset.cluster = true;
+            group_tiles(cset, L, 8, 3);
         }
         const int which = adjoint ? 1 : 0, vectors = adjoint ? 3 : 2;
         if (!tile_fits(cset, vectors)) return false;
-        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<vbd::kTileAdjoint>(L, 8, true)
-                                                              : vbd::pick_tile<vbd::kTileForward>(L, 8, true));
+        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<vbd::kTileAdjoint>(cset.plan, true)
+                                                              : vbd::pick_tile<vbd::kTileForward>(cset.plan, true));
         if (cset.checked[which] != f) {
             cset.checked[which] = f;
             cset.resident[which] = false;
@@ -986,7 +1003,7 @@ struct vbd_solver {
     // and materials.
     int ensure_tile(vbd::TileSet& s) {
         vbd::TilePlan& q = s.plan;
-        if (s.lanes != q.lanes) {
+        if (s.lanes != q.lanes || s.warps != q.warps) {
             const struct {
                 const void* p;
                 size_t ints;
@@ -1025,6 +1042,7 @@ struct vbd_solver {
             CUDA_TRY(cudaStreamSynchronize(stream));  // the host lists may change after this
             s.dirty = true;
             s.lanes = q.lanes;
+            s.warps = q.warps;
         }
         if (s.wrapper && s.dirty) {
             const int nch = (int)(q.chunk.size() / 3);
@@ -1160,7 +1178,7 @@ struct vbd_solver {
                 w.hgz = hg[2];
             }
             VBD_TRY(tile_launch(s, s.wrapper ? vbd::pick_tile_wrapper(s.plan.warps)
-                                         : vbd::pick_tile<vbd::kTileForward>(s.plan.lanes, s.plan.warps, s.cluster),
+                                         : vbd::pick_tile<vbd::kTileForward>(s.plan, s.cluster),
                                 w, 1 + two));
             if (record_energy && k1 > k0 && (k1 - 1) % energy_every == 0) VBD_TRY(emit_energy_append(x0.p));
             k0 = k1;
@@ -1242,7 +1260,7 @@ struct vbd_solver {
                 if (omega > 1.0f) cur ^= 1;
             }
             w.lam_out = cur ? adj_lam2.p : adj_lam.p;
-            VBD_TRY(tile_launch(*tile, vbd::pick_tile<vbd::kTileAdjoint>(tile->plan.lanes, tile->plan.warps, tile->cluster), w, vectors));
+            VBD_TRY(tile_launch(*tile, vbd::pick_tile<vbd::kTileAdjoint>(tile->plan, tile->cluster), w, vectors));
         }
         for (int it = 1; it <= sweeps && !walk && !tile; ++it) {
             bool blend = false;

@@ -31,6 +31,8 @@
 // half the warps' shuffles and idle solve lanes of the per-colour kernel.
 #pragma once
 
+#include <type_traits>
+
 #include "vbd_cluster.cuh"
 #include "vbd_tile_plan.h"
 
@@ -286,10 +288,23 @@ struct TilePair {
     __device__ __forceinline__ F2 detm() const { return reinterpret_cast<const F2*>(buf + 160 * 16)[lane]; }
 };
 
-// Sums of two lanes of one vertex.
+// What a thread's two records add up to: the sums of two lanes of one vertex (Acc2), or of one lane that takes
+// the first record, then the second (Acc1).
 struct Acc2 {
     F2 h00, h01, h02, h11, h12, h22, g0, g1, g2;
     __device__ __forceinline__ void zero() { h00 = h01 = h02 = h11 = h12 = h22 = g0 = g1 = g2 = 0ull; }
+    __device__ __forceinline__ void grad(int i, F2 x) {
+        F2& g = i == 0 ? g0 : i == 1 ? g1 : g2;
+        g = add2(g, x);
+    }
+    __device__ __forceinline__ void diag(int i, F2 x) {
+        F2& h = i == 0 ? h00 : i == 1 ? h11 : h22;
+        h = add2(h, x);
+    }
+    __device__ __forceinline__ void off(int i, F2 x, F2 y) {
+        F2& h = i == 0 ? h01 : i == 1 ? h02 : h12;
+        h = fma2(x, y, h);
+    }
     __device__ __forceinline__ Acc sum() const {
         Acc r;
         r.h00 = f2_lo(h00) + f2_hi(h00);
@@ -301,6 +316,25 @@ struct Acc2 {
         r.g0 = f2_lo(g0) + f2_hi(g0);
         r.g1 = f2_lo(g1) + f2_hi(g1);
         r.g2 = f2_lo(g2) + f2_hi(g2);
+        return r;
+    }
+};
+struct Acc1 {
+    float d[3], o[3], g[3];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) d[i] = o[i] = g[i] = 0.f;
+    }
+    __device__ __forceinline__ void grad(int i, F2 x) { g[i] = __fadd_rn(__fadd_rn(g[i], f2_lo(x)), f2_hi(x)); }
+    __device__ __forceinline__ void diag(int i, F2 x) { d[i] = __fadd_rn(__fadd_rn(d[i], f2_lo(x)), f2_hi(x)); }
+    __device__ __forceinline__ void off(int i, F2 x, F2 y) {
+        o[i] = fmaf(f2_hi(x), f2_hi(y), fmaf(f2_lo(x), f2_lo(y), o[i]));
+    }
+    __device__ __forceinline__ Acc sum() const {
+        Acc r;
+        r.h00 = d[0], r.h11 = d[1], r.h22 = d[2];
+        r.h01 = o[0], r.h02 = o[1], r.h12 = o[2];
+        r.g0 = g[0], r.g1 = g[1], r.g2 = g[2];
         return r;
     }
 };
@@ -334,7 +368,8 @@ __device__ __forceinline__ void tile_edges(const int4 id, float4 xi, const float
 // fact_contrib for two records at once, operation for operation as nvcc contracts it, so that each
 // half has fact_contrib's bits.  A record that is only padding has zero fields and the vertex itself
 // as its neighbours: d = 0, and it adds zero to every sum.
-__device__ __forceinline__ void tile_contrib(const TilePair& r, const int4 id, float4 xi, const float4* X, Acc2& acc) {
+template <class Sums>
+__device__ __forceinline__ void tile_contrib(const TilePair& r, const int4 id, float4 xi, const float4* X, Sums& acc) {
     Geom2 q;
     tile_edges(id, xi, X, q);
     const ulonglong2 ab = r.ab();
@@ -346,17 +381,16 @@ __device__ __forceinline__ void tile_contrib(const TilePair& r, const int4 id, f
     for (int i = 0; i < 3; ++i) {
         C[i] = dot2(q.c[0][i], sw.y, q.c[1][i], w12.x, q.c[2][i], w12.y);
         const F2 Fq = dot2(q.d[0][i], s01.x, q.d[1][i], s01.y, q.d[2][i], sw.x);
-        F2& g = i == 0 ? acc.g0 : i == 1 ? acc.g1 : acc.g2;
-        g = add2(g, fma2(ab.x, sub2(Fq, C[i]), mul2(bj, C[i])));
+        acc.grad(i, fma2(ab.x, sub2(Fq, C[i]), mul2(bj, C[i])));
     }
     const F2 am = mul2(ab.x, neg2(add2(add2(s01.x, s01.y), sw.x)));
     const F2 b0 = mul2(ab.y, C[0]), b1 = mul2(ab.y, C[1]), b2 = mul2(ab.y, C[2]);
-    acc.h00 = add2(acc.h00, fma2(b0, C[0], am));
-    acc.h01 = fma2(b0, C[1], acc.h01);
-    acc.h02 = fma2(b0, C[2], acc.h02);
-    acc.h11 = add2(acc.h11, fma2(b1, C[1], am));
-    acc.h12 = fma2(b1, C[2], acc.h12);
-    acc.h22 = add2(acc.h22, fma2(b2, C[2], am));
+    acc.diag(0, fma2(b0, C[0], am));
+    acc.off(0, b0, C[1]);
+    acc.off(1, b0, C[2]);
+    acc.diag(1, fma2(b1, C[1], am));
+    acc.off(2, b1, C[2]);
+    acc.diag(2, fma2(b2, C[2], am));
 }
 
 // fact_adjoint for two records at once.  A padding record reads the zero entry `zero` of L.
@@ -373,8 +407,9 @@ __device__ __forceinline__ void tile_lambdas(const int4 id, const float4* L, int
     }
 }
 
+template <class Sums>
 __device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, float4 xi, const float4* X,
-                                             const float4* L, int zero, Acc2& acc) {
+                                             const float4* L, int zero, Sums& acc) {
     Geom2 q;
     tile_edges(id, xi, X, q);
     F2 m[3][3];
@@ -396,12 +431,12 @@ __device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, f
     {
         const F2 am = mul2(ab.x, neg2(add2(add2(s01.x, s01.y), sw.x)));
         const F2 b0 = mul2(ab.y, C[0]), b1 = mul2(ab.y, C[1]), b2 = mul2(ab.y, C[2]);
-        acc.h00 = add2(acc.h00, fma2(b0, C[0], am));
-        acc.h01 = fma2(b0, C[1], acc.h01);
-        acc.h02 = fma2(b0, C[2], acc.h02);
-        acc.h11 = add2(acc.h11, fma2(b1, C[1], am));
-        acc.h12 = fma2(b1, C[2], acc.h12);
-        acc.h22 = add2(acc.h22, fma2(b2, C[2], am));
+        acc.diag(0, fma2(b0, C[0], am));
+        acc.off(0, b0, C[1]);
+        acc.off(1, b0, C[2]);
+        acc.diag(1, fma2(b1, C[1], am));
+        acc.off(2, b1, C[2]);
+        acc.diag(2, fma2(b2, C[2], am));
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -412,8 +447,7 @@ __device__ __forceinline__ void tile_adjoint(const TilePair& r, const int4 id, f
         const F2 e2 = add2(cross2(m[0][i1], q.d[1][i2], m[0][i2], q.d[1][i1]), cross2(q.d[0][i1], m[1][i2], q.d[0][i2], m[1][i1]));
         const F2 dF = dot2(m[0][i], s01.x, m[1][i], s01.y, m[2][i], sw.x);
         const F2 dC = dot2(e0, sw.y, e1, w12.x, e2, w12.y);
-        F2& g = i == 0 ? acc.g0 : i == 1 ? acc.g1 : acc.g2;
-        g = add2(g, fma2(ab.x, sub2(dF, dC), mul2(ab.y, fma2(dJ, C[i], mul2(jm1, dC)))));
+        acc.grad(i, fma2(ab.x, sub2(dF, dC), mul2(ab.y, fma2(dJ, C[i], mul2(jm1, dC)))));
     }
 }
 
@@ -698,7 +732,7 @@ __global__ void __launch_bounds__(256) k_pack_wrapper(const int* __restrict__ in
 // is enough, armed for the next iteration when its wait ends; bytes that arrive before that are held
 // against the same phase.
 enum TileKind { kTileForward, kTileAdjoint, kTileWrapper };
-template <int T, TileKind KIND, int W, bool CL = false>
+template <int T, TileKind KIND, int W, bool CL = false, bool STACK = false>
 __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     extern __shared__ __align__(16) unsigned char tsm[];
     constexpr bool ADJ = KIND == kTileAdjoint, WRAP = KIND == kTileWrapper;
@@ -902,7 +936,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
                     if (slot < g.count) xi = (ADJ ? sX : xs)[g.lv + slot];
                     rounds = g.rounds;
                 }
-                Acc2 acc2;
+                std::conditional_t<STACK, Acc1, Acc2> acc2;
                 CorotSums sums;
                 if constexpr (WRAP) {
 #pragma unroll

@@ -252,8 +252,13 @@ void tile_groups(TilePlan* plan, int lanes, int warps, const int32_t* inc_off) {
     p.chunk.clear();
     p.wcol.assign((size_t)p.P * warps * (p.C + 1), 0);
     p.wstream.assign((size_t)p.P * warps * 2, 0);
-    p.max_groups = p.max_rounds = p.max_chunks = 0;
+    p.max_groups = p.max_rounds = p.max_chunks = p.max_colour_groups = 0;
     const int per = kTileChunk / lanes;  // vertices per group
+    for (int c = 0; c < p.C; ++c)
+        for (int t = 0; t < p.P; ++t) {
+            const int32_t* cb = &p.cb[(size_t)c * (p.P + 1) + t];
+            p.max_colour_groups = std::max(p.max_colour_groups, (cb[1] - cb[0] + per - 1) / per);
+        }
     for (int t = 0; t < p.P; ++t) {
         TileHead& h = p.head[t];
         h.group = (int)p.groups.size();

@@ -13,6 +13,7 @@ constexpr int kTileChunkBytes = kTileChunk * 44;
 // VBD_GPU_Solver semantics: a chunk holds two vertices' incidences (16 threads each, two incidences per thread)
 constexpr int kWrapperTileLanes = 32;
 constexpr int kWrapperChunkBytes = kTileChunk * 68;
+constexpr int kWrapperFewGroups = 4;
 constexpr int kWrapperMaxLocal = 32767;     // the 16th bit of an id marks padding
 constexpr int kTileMaxRing = 6;             // chunks a warp's ring holds at most
 constexpr int kTileMaxLocal = 65535;        // local vertex ids are 16 bits
@@ -28,6 +29,9 @@ constexpr int kTileVertices = 32;
 // warps: 28^3 cube (4.6 groups) 2.36 / 2.46, 32^3 (7.2) 2.99 / 2.76, 64 beams (7.7) 3.06 / 2.81, 64^3 (29)
 // 10.8 / 8.4.
 constexpr int kTileFewGroups = 6;
+// Groups of a colour in a tile up to which a thread's two incidences belong to one lane (TilePlan::stack): at
+// 5 the 14^3 cube takes 1.43 us a colour against 1.51, at 6 the 12^3 1.51 / 1.51 and the 18^3 1.57 / 1.55.
+constexpr int kTileStackGroups = 5;
 // Up to this many free vertices per tile each exchanged word has a 128-byte line of its own: polls of the
 // words beside it delay a store's arrival.  Microseconds per colour with words 16 / 32 / 128 bytes apart:
 // 12^3 cube 1.59 / 1.53 / 1.47, 16^3 1.66 / 1.57 / 1.50, 24^3 (100 vertices a tile) 1.83 / 1.79 / 1.82, 28^3
@@ -67,6 +71,8 @@ struct TilePlan {
     int max_local = 0, max_ids = 0, max_groups = 0, max_rounds = 0, max_chunks = 0;
     // for `lanes` threads' worth of partial sums per vertex:
     int lanes = 0, warps = 0;
+    int max_colour_groups = 0;     // of one colour and tile
+    bool stack = false;            // a thread's two incidences belong to one lane (lanes = 2 x threads' sums)
     std::vector<TileGroup> groups;
     std::vector<int32_t> wcol;     // [P][warps][C + 1]: first group of each warp and colour, from the tile's first
     std::vector<int32_t> wstream;  // [P][warps][2]: first chunk and chunks of each warp
