@@ -388,7 +388,7 @@ int vbd_solver_get_colour_lanes(vbd_solver* s, int32_t num_colours, int32_t* lan
  *      layouts; each candidate is timed alternately with the incumbent (twice each, 2 x repeats
  *      steps) against drift;
  *   4. the persistent colour-walking kernel (VBD_OPT_PERSISTENT 1) against the captured graph,
- *      then, where the mesh fits, the cluster walk (VBD_OPT_PERSISTENT 2) at 4, 8, 16 and 32
+ *      the tile walk (VBD_OPT_PERSISTENT) at 4, 8 and 16 threads per vertex, then, where the mesh fits, the cluster walk (VBD_OPT_PERSISTENT 2) at 4, 8, 16 and 32
  *      threads per vertex with record layouts 3 and 4, and, when it wins, its CTA count
  *      (VBD_OPT_CLUSTER_CTAS) at about 1/2, 3/4 and 3/2 of the automatic count and at 16.
  * Phases 2-4 replace the choice only when faster by more than 1%.  chosen (may be null) receives 5

@@ -156,6 +156,7 @@ struct TileSet {
     unsigned long long started = 0;  // CTAs of all launches so far
     unsigned tag = 1;                // next unused word tag
     int stride = 1;                  // of the exchanged words
+    bool no_room = false;            // its memory could not be had
     // cluster form: the forward and adjoint launches checked to fit the device, and the answers
     const void* checked[2] = {nullptr, nullptr};
     bool resident[2] = {false, false};
@@ -163,6 +164,7 @@ struct TileSet {
         plan = std::move(p);
         dirty = true;
         sums = lanes = 0;
+        no_room = false;
         checked[0] = checked[1] = nullptr;
     }
 };
@@ -903,6 +905,7 @@ struct vbd_solver {
         const bool few = groups <= vbd::kTileFewGroups && rounds <= vbd::kTileMaxRing / 2;
         const int w = warps ? warps : few ? 8 : 16;
         s.sums = L;
+        s.no_room = false;
         s.plan.stack = L <= 16 && rounds > 1 && w == 8;
         vbd::tile_groups(&s.plan, s.plan.stack ? 2 * L : L, w, h_inc_off.data());
         if (s.plan.stack && (s.plan.max_colour_groups > vbd::kTileStackGroups || !tile_resident(s, vectors))) {
@@ -932,7 +935,17 @@ struct vbd_solver {
         } else if (tset.sums != lanes) {
             group_tiles(tset, lanes, 0, 2);
         }
-        return tile_fits(walk_tiles(), 1);
+        return tile_fits(walk_tiles(), 1) && tile_room(walk_tiles());
+    }
+    // Whether the device has (or just gave) the memory of a set's records and words; without it the per-colour
+    // launches run.
+    bool tile_room(vbd::TileSet& s) {
+        if (!s.no_room && ensure_tile(s) == VBD_ERR_ALLOC) {
+            vbd::clear_error();
+            (void)cudaGetLastError();
+            s.no_room = true;
+        }
+        return !s.no_room;
     }
     vbd::TileSet& walk_tiles() { return semantics ? wset : tset; }
     // Warps of VBD_GPU_Solver semantics: microseconds per colour with 8 / 16, 16^3 cube (2 groups a colour and
@@ -1004,6 +1017,7 @@ struct vbd_solver {
     int ensure_tile(vbd::TileSet& s) {
         vbd::TilePlan& q = s.plan;
         if (s.lanes != q.lanes || s.warps != q.warps) {
+            s.lanes = 0;  // until the new lists are there
             const struct {
                 const void* p;
                 size_t ints;
@@ -1077,6 +1091,16 @@ struct vbd_solver {
         return VBD_OK;
     }
 
+    // The share of the chunk stream that stays in L2 from one iteration to the next.  A stream larger than L2
+    // read in order finds nothing of the last iteration there; 48 MB of it held with evict-last, and the rest
+    // evict-first, leave the words and vertex state their place.  Microseconds per colour with 0 / 24 / 48 /
+    // 72 / 96 MB held, and plain loads: 48^3 cube 4.61 / 4.60 / 4.57 / 4.62 / 5.02, 5.05; 64^3 8.24 / 8.09 / 8.09 / 8.30 /
+    // 8.36, 8.40; 128 meshes 8.75 / 8.79 / 8.90 / 9.09 / 9.18, 9.24.  A stream that fits stays by itself (32
+    // meshes 3.31 with 48 MB held, 3.26 plain).
+    float tile_keep(const vbd::TileSet& s) const {
+        const double bytes = (double)(s.plan.chunk.size() / 3) * s.chunk_bytes();
+        return !record_cache || bytes <= vbd::kTileStreamFits ? 1.0f : (float)(vbd::kTileStreamKept / bytes);
+    }
     int tile_params(vbd::TileSet& s, int k0, int k1, float dtsr, const float* omega, bool accel, int vectors,
                     vbd::TileParams* out) {
         using S = vbd::TileSet;
@@ -1113,6 +1137,7 @@ struct vbd_solver {
         w.k0 = k0;
         w.k1 = k1;
         w.ring = tile_ring(s, vectors);
+        w.keep = tile_keep(s);
         w.resident = tile_resident(s, vectors);
         w.ring_chunks = tile_ring_chunks(s, vectors);
         w.max_local = q.max_local;
@@ -1346,7 +1371,7 @@ struct vbd_solver {
                 tile = &cset;
             } else if (use_tile()) {
                 tile = &adjoint_tiles();
-                if (!tile_fits(*tile, 2)) tile = nullptr;
+                if (!tile_fits(*tile, 2) || !tile_room(*tile)) tile = nullptr;
             }
         }
         if (tile) {

@@ -23,12 +23,15 @@
 //
 // What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
 // one SM to another's poll, 885 on average) plus one vertex's chain per colour (about 1,000 cycles from
-// the barrier to its publication): 1.4 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by issue and the chunk stream: 64^3 cube 3.4 against 4.1 ms
-// a step of 400 colours, 4.0 TB/s of DRAM reads.
+// the barrier to its publication): 1.3 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by
+// issue and the chunk stream: 64^3 cube 3.45 against 4.17 ms a step of 400 colours, 4.0 TB/s of DRAM
+// reads.  VBD_GPU_Solver semantics: 425-vertex beam 2.6 against 4.6 us a colour, 32^3 cube 6.6 against 9.6.
 // Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
 // records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds
 // the sums of lanes t and t + L/2 (group_reduce's first addition), so a vertex takes L/2 threads:
-// half the warps' shuffles and idle solve lanes of the per-colour kernel.
+// half the warps' shuffles and idle solve lanes of the per-colour kernel.  Or (STACK, and always with
+// VBD_GPU_Solver semantics) it takes records t and t + L of one lane, one after the other: L threads, half
+// the rounds.
 #pragma once
 
 #include <type_traits>
@@ -56,6 +59,7 @@ struct TileParams {
     int n, nfree, ncol, k0, k1; // iterations [k0, k1) of the schedule
     int ring, max_local, max_ids, max_groups, max_rounds;
     int two;                    // both position buffers in shared memory
+    float keep;                 // W = 16: share of the chunk stream kept in L2 (evict-last; the rest evict-first); 1 = plain
     int ring_chunks;            // chunks of all the CTA's rings
     int resident;               // W = 8: the rings hold every chunk of the tile, copied once
     // cluster exchange: where each own vertex's results go, [own vertex] first target, then the targets
@@ -178,14 +182,14 @@ __device__ __forceinline__ void ring_issue(const TileParams& p, TileRing& r, uns
 // The same as one bulk copy, completing on the slot's mbarrier (W = 16).
 template <unsigned kBytes>
 __device__ __forceinline__ void ring_issue_bulk(const TileParams& p, TileRing& r, unsigned buf, unsigned bar, int slot,
-                                                int lane) {
+                                                int lane, unsigned long long policy) {
     if (r.left <= 0) return;
     if (lane == 0) {
         mbar_expect(bar + 8u * slot, kBytes);
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
                          buf + (unsigned)(slot * kBytes)),
                      "l"(reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kBytes),
-                     "r"(kBytes), "r"(bar + 8u * slot)
+                     "r"(kBytes), "r"(bar + 8u * slot), "l"(policy)
                      : "memory");
     }
     --r.left;
@@ -720,7 +724,7 @@ __global__ void __launch_bounds__(256) k_pack_wrapper(const int* __restrict__ in
 // W = 8 is the form for tiles with little work per colour, where a colour lasts as long as one vertex's
 // dependency chain: everything that does not depend on the neighbours is fetched before the barrier, and
 // the chunks stay in shared memory where they fit, else are refilled only after the group's results are
-// out.  (One lane per thread in plain FP32 measured 1.32 against 1.41 us a colour on the beam, but 1.75
+// out.  (One lane per thread and round in plain FP32 measured 1.32 against 1.41 us a colour on the beam, but 1.75
 // against 1.68 on the 16^3 cube and 2.16 against 1.86 on the 24^3.)  W = 16 is the form for tiles that keep
 // an SM's issue slots and memory streams busy, held to 128 registers.
 //
@@ -771,6 +775,13 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     ring.left = ws.y * (p.k1 - p.k0);
     ring.slot = 0;
     const unsigned bar = LAT ? 0u : (unsigned)__cvta_generic_to_shared(bars + warp * kTileMaxRing);
+    unsigned long long policy = 0;
+    if (!LAT) {
+        if (p.keep < 1.f)
+            asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(policy) : "f"(p.keep));
+        else
+            asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+    }
     unsigned parity = 0;  // W = 16: of the ring's current round
     if (!LAT) {
         if (lane == 0) {
@@ -782,7 +793,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     }
     for (int i = 0; i < slots; ++i) {
         if (LAT) ring_issue<kBytes>(p, ring, ring_smem, i, lane);
-        else ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, i, lane);
+        else ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, i, lane, policy);
     }
     if (!CL && tid == 0) atomicAdd(p.arrived, 1ull);
 
@@ -978,7 +989,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
                         else if constexpr (ADJ) tile_adjoint(rec, rec.ids(), xi, sX, xs, p.max_local, acc2);
                         else tile_contrib(rec, rec.ids(), xi, xs, acc2);
                         __syncwarp();  // every lane has read slot `used`
-                        ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, used, lane);
+                        ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, used, lane, policy);
                     }
                 }
                 // W = 16 reads the group again instead of holding it
