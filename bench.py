@@ -12,9 +12,9 @@ E = 1e6 Pa, nu = 0.4, density 1000, bottom face pinned, seeded initial velocitie
   timed steps outside the timed events.
 * e2e: the same metric through the C ABI with host buffers: each step uploads positions and
   velocities from pinned host memory, steps, and reads both back.
-* roofline: the colour-sweep kernel (400 of a step's 402 launches): its algorithmic bytes per launch
-  (60 B per incident tet + 96 B per swept vertex) over the timed region's CUDA-event time per sweep
-  launch; a second pass with an event pair around every sweep launched on its own is reported
+* roofline: the colour sweeps (a tile walk runs a step's 400 in one launch; else 400 of its 402
+  launches): the algorithmic bytes of one (60 B per incident tet + 96 B per swept vertex) over the
+  timed region's CUDA-event time per sweep; a second pass with an event pair around every sweep launched on its own is reported
   beside it as "isolated".
 * cpu_baseline (rank 0, N = 1): the reference's own CPU sources (oracle/_ref, compiled against the
   Eigen-API subset) on all host cores, one cube iteration per sample; the oracle's reference-cost
@@ -480,7 +480,8 @@ def bench_batched(args, rank, world, local, stream, dist, barrier):
     achieved = sw_bytes / step_s / 1e9 if sw_bytes else None
     roofline = {
         "bound": "hbm",
-        "kernel": "vbd::k_sweep (colour sweeps of all meshes, one launch per colour)",
+        "kernel": "vbd::k_tile_walk (all colour sweeps of a step)" if 0 < launches_b < sw_launches
+                  else "vbd::k_sweep (colour sweeps of all meshes, one launch per colour)",
         "achieved": achieved,
         "peak": peak,
         "peak_source": peak_kind,
@@ -551,10 +552,10 @@ def bench_beam(local, stream, autotune=True):
         s.sync()
         launches = s.kernel_launches() - launches_before
         persistent = s.get_option(_capi.OPT_PERSISTENT)
-        path = {0: "captured CUDA graph", 1: "persistent kernel with grid barriers",
+        path = {0: "captured CUDA graph" if launches > 2 else "tile walk (one cooperative launch per step)", 1: "persistent kernel with grid barriers",
                 2: "cluster walk (one thread-block cluster, positions in distributed shared memory)"}[persistent]
         graph_ms = None
-        if persistent:  # the same shape through the captured graph of per-colour launches
+        if persistent or launches <= 2:  # the same shape through the captured graph of per-colour launches
             s.set_option(_capi.OPT_PERSISTENT, 0)
             s.set_positions(m.x)
             s.set_velocities(m.v)
@@ -623,7 +624,10 @@ def bench_adjoint(local, stream, autotune=True):
         tf, tb = forward_backward()
         # the same shape through the captured graph of per-colour launches, for comparison
         graph = None
-        if persistent:
+        launches0 = s.kernel_launches()
+        s.step(st["dt"], 1, st["gravity"], True, st["rho"])
+        walks = s.kernel_launches() - launches0 <= 2
+        if persistent or walks:
             s.set_option(_capi.OPT_PERSISTENT, 0)
             gf, gb = forward_backward()
             graph = {"forward_ms": gf * 1e3, "backward_ms": gb * 1e3, "backward_over_forward": gb / gf}
@@ -649,7 +653,7 @@ def bench_adjoint(local, stream, autotune=True):
         "adjoint_sweeps_per_step": st["adjoint_iterations"],
         "adjoint_rho": st["adjoint_rho"],
         "autotuned": tuned,
-        "forward_path": {0: "captured CUDA graph", 1: "persistent kernel", 2: "cluster walk"}[persistent],
+        "forward_path": {0: "tile walk" if walks else "captured CUDA graph", 1: "persistent kernel", 2: "cluster walk"}[persistent],
         "same_shape_captured_graph": graph,
         "accuracy": "checked in tests/test_gpu_adjoint.py: <= 1e-3 relative vs the FP64 implicit adjoint",
         "roofline": {
@@ -853,10 +857,9 @@ def main():
         e2e_value = units / e2e_max
 
     peak, peak_kind = measured_peaks()
-    # The sweep kernel's average launch duration in the timed region: the region's time (CUDA events
-    # on the solver's stream, max over ranks) over the sweep launches in it.  The predictor and
-    # velocity kernels (2 of 402 launches, 0.3% of the step's device time in the ncu launch list)
-    # are charged to the sweeps, so this bounds the sweep's bandwidth from below.  The second pass,
+    # A colour sweep's average duration in the timed region: the region's time (CUDA events on the
+    # solver's stream, max over ranks) over the colour sweeps in it, which the kernel-timing pass
+    # launches one by one.  The predictor and the velocity update are charged to the sweeps, so this bounds the sweep's bandwidth from below.  The second pass,
     # one event pair around every sweep launched on its own (no graph, no PDL overlap), is reported
     # beside it as "isolated".
     achieved = iso_achieved = launch_us = None
@@ -869,7 +872,8 @@ def main():
     # kernel (profiles/sweep_cube64_dram.txt) times this run's algorithmic bytes per launch
     traffic = None
     prof = os.path.join(ROOT, "profiles", "sweep_cube64_dram.txt")
-    if os.path.exists(prof) and sweep_launches:
+    tile = 0 < launches < sweep_launches  # the steps ran as tile walks: one launch each
+    if os.path.exists(prof) and sweep_launches and not tile:
         for line in open(prof):
             if line.startswith("dram_traffic_over_algorithmic"):
                 traffic = float(line.split("=")[1].split()[0]) * sweep_bytes / sweep_launches
@@ -901,7 +905,8 @@ def main():
         "gpu_launches": int(launches),
         "roofline": {
             "bound": "hbm",
-            "kernel": "vbd::k_sweep (colour sweep)",
+            "kernel": "vbd::k_tile_walk (all colour sweeps of a step; figures per colour sweep)" if tile
+                      else "vbd::k_sweep (colour sweep)",
             "achieved": achieved,
             "peak": peak,
             "peak_source": peak_kind,

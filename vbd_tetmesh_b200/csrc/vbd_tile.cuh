@@ -24,7 +24,7 @@
 // What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
 // one SM to another's poll, 885 on average) plus one vertex's chain per colour (about 1,000 cycles from
 // the barrier to its publication): 1.3 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by
-// issue and the chunk stream: 64^3 cube 3.45 against 4.17 ms a step of 400 colours, 4.0 TB/s of DRAM
+// issue and the chunk stream: 64^3 cube 3.34 against 4.17 ms a step of 400 colours, 4.0 TB/s of DRAM
 // reads.  VBD_GPU_Solver semantics: 425-vertex beam 2.6 against 4.6 us a colour, 32^3 cube 6.6 against 9.6.
 // Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
 // records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds

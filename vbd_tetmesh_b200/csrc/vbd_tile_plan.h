@@ -18,8 +18,8 @@ constexpr int kWrapperMaxLocal = 32767;     // the 16th bit of an id marks paddi
 constexpr int kTileMaxRing = 6;             // chunks a warp's ring holds at most
 constexpr int kTileMaxLocal = 65535;        // local vertex ids are 16 bits
 // A mesh gets a plan from this many free vertices.  Microseconds per colour of a step, tile walk against
-// captured graph (cubes of n^3 cells, one B200): n = 6 (294 free vertices) 1.61 / 2.33, 12 1.50 / 2.50, 16
-// 1.51 / 2.57, 24 1.83 / 3.31, 32 2.73 / 3.53, 48 5.1 / 5.5, 64 8.4 / 10.2.  Below it a few vertices per
+// captured graph (cubes of n^3 cells, one B200): n = 6 (294 free vertices) 1.29 / 2.33, 12 1.51 / 2.50, 16
+// 1.51 / 2.57, 24 1.84 / 3.31, 32 2.73 / 3.53, 48 4.57 / 5.5, 64 8.07 / 10.2.  Below it a few vertices per
 // tile would only exchange words.
 constexpr int kTileMinVertices = 256;
 // Free vertices per tile at least, up to one tile per SM.  32, 64 and 128 measured 0.81, 0.81 and 0.86 ms a
@@ -42,7 +42,7 @@ constexpr int kTileSpreadWords = 80;
 constexpr int kClusterMeshVertices = 5000;
 constexpr int kClusterTileMin = 16;
 // Bytes of a chunk stream that L2 (126 MB) holds beside the rest, and those held of a larger one.
-constexpr double kTileStreamFits = 90e6;
+constexpr double kTileStreamFits = 110e6;
 constexpr double kTileStreamKept = 48e6;
 // Ring depth that holding both position buffers must leave.
 constexpr int kTileTwoRing = 4;
