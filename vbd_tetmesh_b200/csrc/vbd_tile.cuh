@@ -180,17 +180,23 @@ __device__ __forceinline__ void ring_issue(const TileParams& p, TileRing& r, uns
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 // The same as one bulk copy, completing on the slot's mbarrier (W = 16).
-template <unsigned kBytes>
+template <unsigned kBytes, bool HINT>
 __device__ __forceinline__ void ring_issue_bulk(const TileParams& p, TileRing& r, unsigned buf, unsigned bar, int slot,
                                                 int lane, unsigned long long policy) {
     if (r.left <= 0) return;
     if (lane == 0) {
         mbar_expect(bar + 8u * slot, kBytes);
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
-                         buf + (unsigned)(slot * kBytes)),
-                     "l"(reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kBytes),
-                     "r"(kBytes), "r"(bar + 8u * slot), "l"(policy)
-                     : "memory");
+        const char* src = reinterpret_cast<const char*>(p.chunk) + (size_t)r.next * kBytes;
+        const unsigned dst = buf + (unsigned)(slot * kBytes);
+        if constexpr (HINT)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+                "l"(src), "r"(kBytes), "r"(bar + 8u * slot), "l"(policy)
+                : "memory");
+        else
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                         "r"(kBytes), "r"(bar + 8u * slot)
+                         : "memory");
     }
     --r.left;
     if (++r.next == r.end) r.next = r.first;
@@ -775,8 +781,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     ring.left = ws.y * (p.k1 - p.k0);
     ring.slot = 0;
     const unsigned bar = LAT ? 0u : (unsigned)__cvta_generic_to_shared(bars + warp * kTileMaxRing);
+    // VBD_GPU_Solver semantics have no registers left for the policy (32^3 cube 2.72 to 2.75 ms with it, 2.64 to 2.69 without)
+    constexpr bool HINT = !LAT && !WRAP;
     unsigned long long policy = 0;
-    if (!LAT) {
+    if (HINT) {
         if (p.keep < 1.f)
             asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(policy) : "f"(p.keep));
         else
@@ -793,7 +801,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     }
     for (int i = 0; i < slots; ++i) {
         if (LAT) ring_issue<kBytes>(p, ring, ring_smem, i, lane);
-        else ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, i, lane, policy);
+        else ring_issue_bulk<kBytes, HINT>(p, ring, ring_smem, bar, i, lane, policy);
     }
     if (!CL && tid == 0) atomicAdd(p.arrived, 1ull);
 
@@ -989,7 +997,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
                         else if constexpr (ADJ) tile_adjoint(rec, rec.ids(), xi, sX, xs, p.max_local, acc2);
                         else tile_contrib(rec, rec.ids(), xi, xs, acc2);
                         __syncwarp();  // every lane has read slot `used`
-                        ring_issue_bulk<kBytes>(p, ring, ring_smem, bar, used, lane, policy);
+                        ring_issue_bulk<kBytes, HINT>(p, ring, ring_smem, bar, used, lane, policy);
                     }
                 }
                 // W = 16 reads the group again instead of holding it

@@ -41,8 +41,9 @@ constexpr int kTileSpreadWords = 80;
 // evenly (VBD_OPT_PERSISTENT 2), with this many vertices per CTA at least.
 constexpr int kClusterMeshVertices = 5000;
 constexpr int kClusterTileMin = 16;
-// Bytes of a chunk stream that L2 (126 MB) holds beside the rest, and those held of a larger one.
-constexpr double kTileStreamFits = 110e6;
+// Bytes of a chunk stream that L2 (126 MB) holds beside the rest, and those held of a larger one (the 44^3
+// cube's 92 MB: 3.95 us a colour with 48 MB held, 4.40 plain).
+constexpr double kTileStreamFits = 90e6;
 constexpr double kTileStreamKept = 48e6;
 // Ring depth that holding both position buffers must leave.
 constexpr int kTileTwoRing = 4;
