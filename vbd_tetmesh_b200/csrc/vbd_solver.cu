@@ -759,7 +759,10 @@ struct vbd_solver {
             w[it - 1] = rho > 0.0f ? omega : 1.0f;
         }
         if (w != adj_omega_cache) {
-            if (d_adj_omega.n < w.size()) VBD_TRY(d_adj_omega.alloc(w.size()));
+            if (d_adj_omega.n < w.size()) {
+                drop_graphs();  // the cluster adjoint's captured launches hold the address
+                VBD_TRY(d_adj_omega.alloc(w.size()));
+            }
             CUDA_TRY(cudaMemcpyAsync(d_adj_omega.p, w.data(), sizeof(float) * w.size(), cudaMemcpyHostToDevice, stream));
             CUDA_TRY(cudaStreamSynchronize(stream));
             adj_omega_cache = w;
