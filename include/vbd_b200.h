@@ -231,6 +231,14 @@ int vbd_solver_sync(vbd_solver* s);
  * after spin_limit polls and exits; *timed_out receives 1 if the device recorded the timeout. */
 int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* timed_out);
 
+/* The same for the tile walk (no reference counterpart): launches the walk that steps take with the present
+ * mesh and options, with one tile that publishes none of its results, so that its neighbours' waits
+ * run out after wait_us microseconds (1 to 1,000,000).  *timed_out receives 1 if the device recorded
+ * that; the record stays for the call that reports it, as after a step whose wait gave up.  Positions
+ * and velocities keep their values.  VBD_ERR_STATE where steps do not run as tile walks or no tile reads
+ * from another. */
+int vbd_solver_walk_selftest(vbd_solver* s, int64_t wait_us, int32_t* timed_out);
+
 /* The energy history of VBD_OPT_ENERGY_EVERY (VBDsolver::energyHistory, VBD.h:70; filled at
  * VBD.cpp:93-95): writes up to `capacity` values, oldest first, and sets *count to the number of
  * values appended since the last reset (a count above capacity means the rest were not copied).

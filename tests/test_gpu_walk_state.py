@@ -1,5 +1,7 @@
 """What the walks (csrc/vbd_tile.cuh, csrc/vbd_cluster.cuh) keep between calls: schedules, captured launches,
 packed records and wait states stay right when the calls around them change."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -35,3 +37,52 @@ def test_backward_with_a_longer_schedule_between(gpu_device, resident):
         for a, b in zip(one.backward(W, None, sweeps, 0.9), want):
             np.testing.assert_array_equal(a, b)
     one.close()
+
+
+def give_up(s, wait_us=5000):
+    """One walk of `s` whose waits run out."""
+    out = C.c_int32(0)
+    _capi.call("vbd_solver_walk_selftest", s._h, wait_us, C.byref(out))
+    return out.value
+
+
+# 8 warps with resident and streamed chunks, 16 warps with one and two rounds of a group, VBD_GPU_Solver semantics
+# with 8 and 16 warps
+@pytest.mark.parametrize("mesh,lanes,semantics", [
+    (lambda: meshgen.jittered_block(7, 6, 5, seed=5), 16, 0), (lambda: meshgen.cube(24), 8, 0),
+    (lambda: meshgen.cube(32), 16, 0), (lambda: meshgen.cube(44), 8, 0), (lambda: meshgen.cube(40), 4, 0),
+    (lambda: meshgen.jittered_block(7, 6, 5, seed=5), 8, 1), (lambda: meshgen.cube(26), 8, 1),
+], ids=["block", "cube24", "cube32", "cube44", "cube40", "wrapper block", "wrapper cube26"])
+def test_a_wait_that_runs_out_ends_the_walk(gpu_device, mesh, lanes, semantics):
+    m = mesh()
+    out = []
+    for fail in (False, True):
+        s = build_solver(m, lanes=lanes)
+        s.set_option(_capi.OPT_SEMANTICS, semantics)
+        s.step(1 / 120, 4, G, True, 0.9)
+        if fail:
+            assert give_up(s) == 1
+            with pytest.raises(_capi.VBDError) as e:
+                s.sync()
+            assert e.value.code == 6  # VBD_ERR_TIMEOUT
+        l0 = s.kernel_launches()
+        s.step(1 / 120, 4, G, True, 0.9)
+        s.sync()
+        assert s.kernel_launches() - l0 <= 2  # still the walk
+        out.append((s.get_positions(), s.get_velocities(), np.array(s.status())))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_walk_selftest_refuses_what_is_no_walk(gpu_device):
+    s = build_solver(meshgen.jittered_block(7, 6, 5, seed=5))
+    for wait in (0, 1000001):
+        with pytest.raises(_capi.VBDError) as e:
+            give_up(s, wait)
+        assert e.value.code == 1  # VBD_ERR_INVALID_ARG
+    s.set_option(_capi.OPT_PERSISTENT, 0)
+    with pytest.raises(_capi.VBDError) as e:
+        give_up(s)
+    assert e.value.code == 3  # VBD_ERR_STATE
+    s.close()

@@ -1133,6 +1133,7 @@ struct vbd_solver {
         w.max_own = q.max_own;
         w.max_target = q.max_target;
         w.status = status.p;
+        w.wait_ns = vbd::kTileWaitNs;
         w.omega = omega;
         w.n = N;
         w.nfree = nfree;
@@ -1211,6 +1212,44 @@ struct vbd_solver {
             if (record_energy && k1 > k0 && (k1 - 1) % energy_every == 0) VBD_TRY(emit_energy_append(x0.p));
             k0 = k1;
         } while (k0 < iters);
+        return VBD_OK;
+    }
+
+    // Three iterations of the walk in which the first tile that others read from publishes nothing, so that
+    // their waits run out after wait_us.  The result goes nowhere.
+    int walk_selftest(long long wait_us, int32_t* timed_out) {
+        if (!use_tile()) VBD_FAIL(VBD_ERR_STATE, "with this mesh and these options steps do not run as tile walks");
+        vbd::TileSet& s = walk_tiles();
+        std::vector<vbd::TileGroup> groups = s.plan.groups;
+        bool muted = false;
+        for (const vbd::TileHead& h : s.plan.head) {
+            for (int i = h.group; i < h.group + h.ngroups; ++i) {
+                muted = muted || groups[i].publish > 0;
+                groups[i].publish = 0;
+            }
+            if (muted) break;
+        }
+        if (!muted) VBD_FAIL(VBD_ERR_STATE, "no tile of this mesh reads from another");
+        VBD_TRY(upload_schedule(3, false, 0.0f));
+        VBD_TRY(ensure_tile(s));
+        vbd::DBuf<vbd::TileGroup> list;
+        vbd::DBuf<float4> x;
+        VBD_TRY(list.alloc(groups.size()));
+        VBD_TRY(x.alloc(N));
+        CUDA_TRY(cudaMemcpyAsync(list.p, groups.data(), sizeof(vbd::TileGroup) * groups.size(), cudaMemcpyHostToDevice, stream));
+        CUDA_TRY(cudaMemcpyAsync(x.p, x0.p, sizeof(float4) * (size_t)N, cudaMemcpyDeviceToDevice, stream));
+        vbd::TileParams w;
+        VBD_TRY(tile_params(s, 0, 3, 3600.0f, d_omega.p, false, 1, &w));
+        w.groups = list.p;
+        w.wait_ns = 1000ull * (unsigned long long)wait_us;
+        w.x0 = x.p;
+        w.pp = pp.p;
+        VBD_TRY(tile_launch(s, s.wrapper ? vbd::pick_tile_wrapper(s.plan.warps) : vbd::pick_tile<vbd::kTileForward>(s.plan, false),
+                            w, 1));
+        unsigned long long t = 0;
+        CUDA_TRY(cudaMemcpyAsync(&t, status.p + vbd::ST_WALK_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost, stream));
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        *timed_out = t ? 1 : 0;
         return VBD_OK;
     }
 
@@ -2224,6 +2263,14 @@ int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* time
     CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
     *timed_out = t ? 1 : 0;
     return VBD_OK;
+}
+
+int vbd_solver_walk_selftest(vbd_solver* s, int64_t wait_us, int32_t* timed_out) {
+    vbd::clear_error();
+    VBD_TRY(need_ready(s));
+    if (!timed_out || wait_us < 1 || wait_us > 1000000) VBD_FAIL(VBD_ERR_INVALID_ARG, "need timed_out and wait_us in 1..1000000");
+    DeviceScope scope(s->device);
+    return s->walk_selftest(wait_us, timed_out);
 }
 
 int vbd_solver_energy(vbd_solver* s, int32_t kind, float h, double* out) {

@@ -54,6 +54,7 @@ struct TileParams {
     unsigned long long* arrived;
     unsigned long long arrived_target;  // *arrived once every CTA of this launch has started
     unsigned long long* status;
+    unsigned long long wait_ns; // after which a wait gives up (kTileWaitNs)
     const float* omega;         // Chebyshev weight of each iteration (1 = no blend)
     unsigned tag;               // iteration k publishes tag + k; unused by any earlier launch
     int n, nfree, ncol, k0, k1; // iterations [k0, k1) of the schedule
@@ -113,20 +114,22 @@ __device__ __forceinline__ float4 word_load(const float4* p) {
                        __uint_as_float((unsigned)(b >> 32)));
 }
 
-// Gives up a wait: another wait already gave up, or this one has lasted kTileWaitNs with every CTA of
+// Gives up a wait: another wait already gave up, or this one has lasted wait_ns with every CTA of
 // the launch running (a CTA that cannot start while another program's kernel holds its SM is
-// waited for up to kTileStartNs).
+// waited for up to kTileStartNs).  The walk then sweeps on to the end of the iteration with what it has, so
+// that no thread leaves a barrier, a shuffle or a copy that the others wait for.
 constexpr unsigned long long kTileWaitNs = 2000000000ull;
 constexpr unsigned long long kTileStartNs = 60000000000ull;
+constexpr unsigned long long kTileDrainNs = 20000000ull;  // for the copies under way of a walk that gave up
 struct TileClock {
     unsigned long long first = 0, last = 0;
 };
 __device__ __noinline__ bool tile_give_up(unsigned long long* status, unsigned long long* arrived,
-                                          unsigned long long target, TileClock& c) {
+                                          unsigned long long target, unsigned long long wait_ns, TileClock& c) {
     if (*reinterpret_cast<volatile unsigned long long*>(status + ST_WALK_TIMEOUT) != 0ull) return true;
     const unsigned long long now = global_ns();
     if (c.first == 0) c.first = c.last = now;
-    if (now - c.last <= kTileWaitNs) return false;
+    if (now - c.last <= wait_ns) return false;
     if (*reinterpret_cast<volatile unsigned long long*>(arrived) < target && now - c.first <= kTileStartNs) {
         c.last = now;
         return false;
@@ -144,7 +147,7 @@ __device__ __forceinline__ bool tile_spin(const TileParams& p, const float4* w, 
             *dst = make_float4(v.x, v.y, v.z, 0.f);
             return true;
         }
-        if ((i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, clk)) return false;
+        if ((i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, p.wait_ns, clk)) return false;
     }
 }
 // The same with a first look already taken.
@@ -209,15 +212,30 @@ __device__ __forceinline__ bool ring_try(unsigned bar, unsigned parity) {
                  : "memory");
     return ok != 0;
 }
+// The same without a wait of its own.
+__device__ __forceinline__ bool ring_test(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Waits for a slot's chunk; the same answer for the whole warp.  The repeated tries stand in a function of their
+// own: inlined they cost the sweep loop registers (64^3 cube 3.15 ms a step of 50 iterations against 3.26, 128 meshes
+// 1.31 against 1.43, 32^3 1.07 against 1.09, VBD_GPU_Solver semantics 32^3 0.98 against 1.02 for 20).
+__device__ __noinline__ bool ring_wait_again(unsigned bar, unsigned parity, unsigned long long* status,
+                                             unsigned long long* arrived, unsigned long long target,
+                                             unsigned long long wait_ns) {
+    TileClock clk;
+    for (unsigned i = 1;; ++i) {
+        if (ring_try(bar, parity)) return true;
+        if ((i & 255u) == 0u && tile_give_up(status, arrived, target, wait_ns, clk)) return false;
+    }
+}
 __device__ __forceinline__ bool ring_wait_bulk(const TileParams& p, unsigned bar, unsigned parity) {
     bool done = ring_try(bar, parity);
-    if (!done) {
-        TileClock clk;
-        for (unsigned i = 1; !done; ++i) {
-            done = ring_try(bar, parity);
-            if (!done && (i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, clk)) break;
-        }
-    }
+    if (!done) done = ring_wait_again(bar, parity, p.status, p.arrived, p.arrived_target, p.wait_ns);
     return __all_sync(0xffffffffu, done);
 }
 // Waits until at most `pending` of the newest commit groups are outstanding.
@@ -913,7 +931,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
     };
-    bool ok = true;
+    bool ok = true;  // of this thread, not of its warp: no shuffle or vote may depend on it
     // Chunk i is commit group i.  W = 8: a group's chunks (at most p.max_rounds) have all landed before the
     // barrier that precedes its sweep, and its slots are refilled after its results are out.  W = 16: a
     // chunk is waited for when it is swept and refilled right after.
@@ -987,9 +1005,12 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
                         else tile_contrib(r0, r0.ids(), xi, xs, acc2);
                     }
                 } else {
-                    for (; rounds > 0 && ok; --rounds) {
+                    for (; rounds > 0; --rounds) {
                         const int used = ring.slot;
-                        ok = ring_wait_bulk(p, bar + 8u * used, parity);
+                        if (!ring_wait_bulk(p, bar + 8u * used, parity)) {  // the whole warp; nothing to read there
+                            ok = false;
+                            break;
+                        }
                         ring.slot = next_slot(used);
                         if (ring.slot == 0) parity ^= 1u;
                         const TilePair rec = chunk_at(used);
@@ -1135,8 +1156,9 @@ __global__ void __launch_bounds__(W * 32, 1) k_tile_walk(TileParams p) {
     // no copy outlives the walk (one that gave up has bulk copies under way; the waits are bounded)
     ring_wait_for<0>();
     if (!LAT && !ok) {
+        const unsigned long long t0 = global_ns();
         for (int i = 0; i < p.ring; ++i) {
-            for (int n = 0; n < 100000 && !ring_try(bar + 8u * ring.slot, parity); ++n) __nanosleep(100);
+            while (!ring_test(bar + 8u * ring.slot, parity) && global_ns() - t0 < kTileDrainNs) __nanosleep(100);
             ring.slot = next_slot(ring.slot);
             if (ring.slot == 0) parity ^= 1u;
         }
