@@ -222,8 +222,11 @@ int vbd_solver_backward(vbd_solver* s, const float* dl_dx, const float* dl_dv, i
                         float adjoint_rho, float* dl_dx0, float* dl_dv0, float* dl_dmu, float* dl_dlambda);
 
 /* Waits for all work queued on the handle's stream and reports sticky device errors, and
- * VBD_ERR_TIMEOUT if a grid barrier of the persistent kernel gave up since the last sync.  No
- * reference counterpart: the reference's calls are synchronous. */
+ * VBD_ERR_TIMEOUT if a bounded wait of a tile or cluster walk or a grid barrier of the persistent kernel
+ * gave up since the last report.  Every call that waits for a result reports that too, once: the reads of
+ * positions, velocities, inertia, energies, energy history and status, vbd_solver_record,
+ * vbd_solver_backward and vbd_solver_autotune.  What the steps since then computed is not to be used.
+ * No reference counterpart: the reference's calls are synchronous. */
 int vbd_solver_sync(vbd_solver* s);
 
 /* Failure-detection self-test (no reference counterpart): launches the persistent kernel with one barrier arrival missing and
@@ -305,10 +308,10 @@ int vbd_solver_status(vbd_solver* s, int64_t* singular_skips, int32_t* nonfinite
  *                        L2 after each colour (factored records, 4, 8 or 16 lanes for every colour,
  *                        VBD_OPT_GRAPH on, no kernel timing, the handle's stream not capturing, the
  *                        tile's vertices within shared memory).  Same results as the graph; reads
- *                        back as 0; VBD_ERR_TIMEOUT from vbd_solver_sync if a bounded wait gave up;
+ *                        back as 0; VBD_ERR_TIMEOUT (vbd_solver_sync) if a bounded wait gave up;
  *                        1 = run each step / solve as one cooperative launch that walks the colours
  *                        with a grid barrier after each one (bounded wait: a barrier that gives up
- *                        makes the next vbd_solver_sync return VBD_ERR_TIMEOUT);
+ *                        makes the next call that reports it return VBD_ERR_TIMEOUT);
  *                        2 = run each sub-step / solve as ONE thread-block cluster whose CTAs hold a
  *                        tile of the mesh each (its records too where they fit) and send their
  *                        borders' new positions to each other through distributed shared memory.  For

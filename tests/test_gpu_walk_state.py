@@ -86,3 +86,47 @@ def test_walk_selftest_refuses_what_is_no_walk(gpu_device):
         give_up(s)
     assert e.value.code == 3  # VBD_ERR_STATE
     s.close()
+
+
+@pytest.mark.parametrize("call", [
+    lambda s: s.get_positions(), lambda s: s.get_velocities(), lambda s: s.get_inertia(), lambda s: s.energy(0, 1 / 60),
+    lambda s: s.energy(2, 1 / 60), lambda s: s.energy_history(), lambda s: s.status(), lambda s: s.status(True),
+    lambda s: s.sync(), lambda s: s.record(2), lambda s: s.backward(np.ones((s.num_verts, 3)), None, 5, 0.9),
+    lambda s: s.autotune(1 / 60, 2, 1),
+], ids=["positions", "velocities", "inertia", "energy", "residual", "history", "status", "status reset", "sync", "record",
+        "backward", "autotune"])
+def test_a_wait_that_ran_out_is_reported_once(gpu_device, call):
+    """By the first call that waits for a result; the steps after the report are right again."""
+    m = meshgen.jittered_block(7, 6, 5, seed=5)
+    s = build_solver(m)
+    s.set_option(_capi.OPT_ENERGY_EVERY, 2)
+    s.record(2)
+    s.step(1 / 60, 4, G, True, 0.9)
+    x = s.get_positions()
+    assert give_up(s) == 1
+    with pytest.raises(_capi.VBDError) as e:
+        call(s)
+    assert e.value.code == 6  # VBD_ERR_TIMEOUT
+    s.sync()
+    np.testing.assert_array_equal(s.get_positions(), x)
+    s.step(1 / 60, 4, G, True, 0.9)
+    fresh = build_solver(m)
+    for _ in range(2):
+        fresh.step(1 / 60, 4, G, True, 0.9)
+    np.testing.assert_array_equal(s.get_positions(), fresh.get_positions())
+    s.close()
+    fresh.close()
+
+
+def test_a_new_mesh_starts_without_the_last_ones_report(gpu_device):
+    from vbd_tetmesh_b200 import color_vertices, mesh_mass, precompute_tets
+
+    m = meshgen.jittered_block(7, 6, 5, seed=5)
+    s = build_solver(m)
+    assert give_up(s) == 1
+    _, offs, verts = color_vertices(m.num_verts, m.tets)
+    dminv, v0 = precompute_tets(m.rest, m.tets)
+    s.init_from_cpu(m.x, mesh_mass(m.rest, m.tets, m.density)[0], m.fixed, m.tets, offs, verts, dminv, v0, m.mu, m.lam)
+    s.step(1 / 60, 4, G, True, 0.9)
+    assert np.isfinite(s.get_positions()).all()
+    s.close()

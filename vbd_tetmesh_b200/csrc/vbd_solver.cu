@@ -225,6 +225,7 @@ struct vbd_solver {
     vbd::DBuf<int> inc_vertex;                      // internal vertex of each incidence
     vbd::DBuf<float> stage, mat_stage;
     vbd::DBuf<unsigned long long> status;
+    unsigned* wait_flag = nullptr;  // host memory: set by a kernel whose wait gave up (vbd::ST_HOST)
     vbd::DBuf<double> partials, scalar;
     // defaults: 64-thread blocks, programmatic dependent launch and graphs; lanes, layout and
     // record prefetch are chosen at init from the mesh (below) until their options are set
@@ -338,7 +339,22 @@ struct vbd_solver {
     ~vbd_solver() {
         drop_graphs();
         for (cudaEvent_t e : ev_pool) cudaEventDestroy(e);
+        if (wait_flag) cudaFreeHost(wait_flag);
         if (own_stream && stream) cudaStreamDestroy(stream);
+    }
+
+    // Waits for the work queued so far, and reports a wait of a walk or a grid barrier that gave up since the
+    // last report: positions, velocities and gradients computed since then are not to be used.
+    int finish() {
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        if (!*reinterpret_cast<volatile unsigned*>(wait_flag)) return VBD_OK;
+        unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
+        CUDA_TRY(cudaMemcpyAsync(t, status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost, stream));
+        CUDA_TRY(cudaMemsetAsync(status.p + vbd::ST_TIMEOUT, 0, sizeof(t), stream));
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        *wait_flag = 0;
+        if (t[0]) VBD_FAIL(VBD_ERR_TIMEOUT, "a grid barrier of the persistent kernel gave up waiting");
+        VBD_FAIL(VBD_ERR_TIMEOUT, "a wait of the cluster or tile walk gave up");
     }
 
     // Folds the recorded event pairs into the running totals (synchronises on the last one).
@@ -1493,8 +1509,7 @@ struct vbd_solver {
         vbd::k_gather3<<<vbd::nblk(N, 256), 256, 0, stream>>>(src, perm.p, stage.p, N);
         VBD_TRY(check_launch());
         CUDA_TRY(cudaMemcpyAsync(dst, stage.p, sizeof(float) * 3 * (size_t)N, cudaMemcpyDefault, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        return VBD_OK;
+        return finish();
     }
 
     // Captured graphs bake in buffer addresses: every (re)allocation or release of the streamed
@@ -1553,8 +1568,7 @@ struct vbd_solver {
         vbd::k_sum_partials<<<1, 1024, 0, stream>>>(partials.p, (int)blocks, scalar.p);
         VBD_TRY(check_launch());
         CUDA_TRY(cudaMemcpyAsync(out, scalar.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        return VBD_OK;
+        return finish();
     }
 };
 
@@ -1607,8 +1621,13 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
     }
     s->sm_count = prop.multiProcessorCount;
     s->smem_optin = (int)prop.sharedMemPerBlockOptin;
-    VBD_TRY(s->status.alloc(vbd::ST_SLOTS));
-    CUDA_TRY(cudaMemsetAsync(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS, s->stream));
+    VBD_TRY(s->status.alloc(vbd::ST_HOST + 1));
+    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&s->wait_flag), sizeof(unsigned), cudaHostAllocMapped));
+    *s->wait_flag = 0;
+    void* flag = nullptr;
+    CUDA_TRY(cudaHostGetDevicePointer(&flag, s->wait_flag, 0));
+    const unsigned long long st[vbd::ST_HOST + 1] = {0, 0, 0, 0, reinterpret_cast<unsigned long long>(flag)};
+    CUDA_TRY(cudaMemcpyAsync(s->status.p, st, sizeof(st), cudaMemcpyHostToDevice, s->stream));
     VBD_TRY(s->scalar.alloc(1));
     *out = s.release();
     return VBD_OK;
@@ -1669,6 +1688,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
 
     DeviceScope scope(s->device);
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    *s->wait_flag = 0;  // of the previous mesh
     s->ready = false;
     s->drop_graphs();
     s->irec.release();
@@ -2105,7 +2125,7 @@ int vbd_solver_energy_history(vbd_solver* s, double* energies, int32_t capacity,
     int n = 0;
     if (s->ecount.p) {
         CUDA_TRY(cudaMemcpyAsync(&n, s->ecount.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaStreamSynchronize(s->stream));
+        VBD_TRY(s->finish());
     }
     const int avail = (int)std::min<long long>(n, (long long)s->ehist.n);
     const int copy = std::min(avail, capacity);
@@ -2129,6 +2149,7 @@ int vbd_solver_record(vbd_solver* s, int32_t checkpoint_every) {
     if (checkpoint_every > 0 && s->semantics)
         VBD_FAIL(VBD_ERR_STATE, "the adjoint differentiates the VBDsolver semantics; set VBD_OPT_SEMANTICS to 0");
     DeviceScope scope(s->device);
+    if (checkpoint_every > 0) VBD_TRY(s->finish());  // of a state to start from
     s->tape.clear();
     // a new recording reuses the last one's buffers; stopping gives them back
     if (checkpoint_every == 0) s->ckpt_pool.clear();
@@ -2225,25 +2246,15 @@ int vbd_solver_backward(vbd_solver* s, const float* dl_dx, const float* dl_dv, i
     }
     for (int k = 0; k < 6; ++k)
         CUDA_TRY(cudaMemcpyAsync(live[k], s->adj_save.p + (size_t)k * N, b4, cudaMemcpyDeviceToDevice, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    return rc;
+    const int waits = s->finish();
+    return rc ? rc : waits;
 }
 
 int vbd_solver_sync(vbd_solver* s) {
     vbd::clear_error();
     if (!s) VBD_FAIL(VBD_ERR_INVALID_ARG, "null solver handle");
     DeviceScope scope(s->device);
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    if (s->status.p) {
-        unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
-        CUDA_TRY(cudaMemcpy(t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
-        if (t[0] || t[1]) {
-            CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
-            if (t[0]) VBD_FAIL(VBD_ERR_TIMEOUT, "a grid barrier of the persistent kernel gave up waiting");
-            VBD_FAIL(VBD_ERR_TIMEOUT, "a wait of the cluster or tile walk gave up");
-        }
-    }
-    return VBD_OK;
+    return s->finish();
 }
 
 int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* timed_out) {
@@ -2261,6 +2272,7 @@ int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* time
     unsigned long long t = 0;
     CUDA_TRY(cudaMemcpy(&t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
     CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
+    *s->wait_flag = 0;
     *timed_out = t ? 1 : 0;
     return VBD_OK;
 }
@@ -2316,6 +2328,7 @@ int vbd_solver_status(vbd_solver* s, int64_t* singular_skips, int32_t* nonfinite
     vbd::clear_error();
     VBD_TRY(need_ready(s));
     DeviceScope scope(s->device);
+    const int waits = s->finish();
     unsigned long long h[vbd::ST_SLOTS];
     CUDA_TRY(cudaMemcpyAsync(h, s->status.p, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -2325,7 +2338,7 @@ int vbd_solver_status(vbd_solver* s, int64_t* singular_skips, int32_t* nonfinite
         CUDA_TRY(cudaMemsetAsync(s->status.p, 0, sizeof(h), s->stream));
         CUDA_TRY(cudaStreamSynchronize(s->stream));
     }
-    return VBD_OK;
+    return waits;
 }
 
 int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
@@ -2522,7 +2535,7 @@ int vbd_solver_autotune(vbd_solver* s, float dt, int32_t iterations, int32_t rep
         CUDA_TRY(cudaMemcpyAsync(save.p + (size_t)k * s->N, bufs[k], b4, cudaMemcpyDeviceToDevice, s->stream));
     unsigned long long st[vbd::ST_SLOTS];
     CUDA_TRY(cudaMemcpyAsync(st, s->status.p, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    VBD_TRY(s->finish());
     const int saved_timing = s->timing;
     const int saved_energy = s->energy_every;
     s->timing = 0;

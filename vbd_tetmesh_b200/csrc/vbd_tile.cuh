@@ -134,7 +134,7 @@ __device__ __noinline__ bool tile_give_up(unsigned long long* status, unsigned l
         c.last = now;
         return false;
     }
-    atomicOr(reinterpret_cast<unsigned int*>(status + ST_WALK_TIMEOUT), 1u);
+    note_timeout(status, ST_WALK_TIMEOUT);
     return true;
 }
 
