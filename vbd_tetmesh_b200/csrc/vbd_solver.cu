@@ -848,14 +848,14 @@ struct vbd_solver {
     }
 
     // A sub-step (predict and finish) or a solve as one cluster launch: the tile walk of one cluster where it
-    // fits (and VBD_OPT_CLUSTER_RESIDENT allows it), else vbd::k_cluster_walk.
+    // fits, its memory can be had and VBD_OPT_CLUSTER_RESIDENT allows it, else vbd::k_cluster_walk.
     int launch_cluster(int iters, float dtsr, bool accel, float rho, bool predict, bool finish, bool from_inertia,
                        float h, const float* hg) {
         const char* why = nullptr;
         if (!cluster_fit(&why)) VBD_FAIL(VBD_ERR_INVALID_ARG, "%s", why);
         VBD_TRY(upload_schedule(iters, accel, rho));
         const int L = lanes < 4 ? 4 : lanes;
-        if (cluster_resident && cluster_tiles(L, false))
+        if (cluster_resident && cluster_tiles(L, false) && tile_room(cset))
             return launch_tile(cset, iters, dtsr, accel, rho, from_inertia, h, predict ? hg : nullptr, false);
         void (*fn)(vbd::PersistParams) = nullptr;
         switch (L) {
@@ -957,7 +957,7 @@ struct vbd_solver {
         return tile_fits(walk_tiles(), 1) && tile_room(walk_tiles());
     }
     // Whether the device has (or just gave) the memory of a set's records and words; without it the per-colour
-    // launches run.
+    // launches run, or the cluster walk with whole-mesh copies.
     bool tile_room(vbd::TileSet& s) {
         if (!s.no_room && ensure_tile(s) == VBD_ERR_ALLOC) {
             vbd::clear_error();
@@ -1424,7 +1424,7 @@ struct vbd_solver {
         void (*walk)(vbd::AdjWalkParams) = nullptr;
         vbd::TileSet* tile = nullptr;
         if (!adj_alternate) {
-            const bool walk_tiles = adj_walk() && cluster_resident && cluster_tiles(lanes < 4 ? 4 : lanes, true);
+            const bool walk_tiles = adj_walk() && cluster_resident && cluster_tiles(lanes < 4 ? 4 : lanes, true) && tile_room(cset);
             if (walk_tiles) {
                 tile = &cset;
             } else if (use_tile()) {
@@ -2385,7 +2385,7 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
             s->persistent_set = true;
             s->tile_walk = 0;
             if (value == 2 && s->ready && s->cluster_resident && s->cluster_tiles(s->lanes < 4 ? 4 : s->lanes, false)) {
-                VBD_TRY(s->ensure_tile(s->cset));
+                (void)s->tile_room(s->cset);
                 CUDA_TRY(cudaStreamSynchronize(s->stream));
             }
             return VBD_OK;
