@@ -130,3 +130,133 @@ def test_a_new_mesh_starts_without_the_last_ones_report(gpu_device):
     s.step(1 / 60, 4, G, True, 0.9)
     assert np.isfinite(s.get_positions()).all()
     s.close()
+
+
+def on_stream(m, lanes=8, ctas=0):
+    """A solver with the cluster walk on a torch stream, after one step."""
+    import torch
+
+    st = torch.cuda.Stream()
+    s = build_solver(m, lanes=lanes, layout=4, stream=st.cuda_stream)
+    s.set_option(_capi.OPT_CLUSTER_CTAS, ctas)
+    s.set_option(_capi.OPT_PERSISTENT, 2)
+    s.step(1 / 60, 9, G, True, 0.9)
+    s.sync()
+    return s, st
+
+
+def capture_step(s, st):
+    import torch
+
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        s.step(1 / 60, 9, G, True, 0.9)
+    return g
+
+
+def replay(g, s, st):
+    import torch
+
+    with torch.cuda.stream(st):
+        g.replay()
+    s.sync()
+    return s.get_positions()
+
+
+def plain(m, what):
+    """Positions after each of the steps `what` names by their (lanes, material factor), one launch per colour."""
+    s = build_solver(m, layout=4)
+    s.set_option(_capi.OPT_PERSISTENT, 0)
+    out = []
+    for lanes, factor in what:
+        s.set_option(_capi.OPT_LANES, lanes)
+        s.set_materials(m.mu * np.float32(factor), m.lam * np.float32(factor))
+        s.step(1 / 60, 9, G, True, 0.9)
+        out.append(s.get_positions())
+    s.close()
+    return out
+
+
+def test_captured_cluster_step_follows_new_materials(gpu_device):
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2)
+    s, st = on_stream(m)
+    g = capture_step(s, st)
+    want = plain(m, [(8, 1), (8, 1), (8, 3), (8, 5), (8, 5)])
+    np.testing.assert_array_equal(replay(g, s, st), want[1])
+    s.set_materials(m.mu * np.float32(3), m.lam * np.float32(3))
+    np.testing.assert_array_equal(replay(g, s, st), want[2])
+    # a step captured right after new materials and never launched leaves them to be packed
+    s.set_materials(m.mu * np.float32(5), m.lam * np.float32(5))
+    unused = capture_step(s, st)
+    s.step(1 / 60, 9, G, True, 0.9)
+    np.testing.assert_array_equal(s.get_positions(), want[3])
+    np.testing.assert_array_equal(replay(unused, s, st), want[4])
+    del g, unused
+    s.close()
+
+
+def test_captured_cluster_step_keeps_its_records_beside_other_shapes(gpu_device):
+    """Other lane and CTA counts afterwards, and the first again: what the captured step reads stays in place, and
+    follows new materials."""
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2)
+    s, st = on_stream(m)
+    g8 = capture_step(s, st)
+    s.set_option(_capi.OPT_LANES, 16)
+    want = plain(m, [(8, 1), (16, 1), (8, 1), (16, 1), (16, 2), (8, 2), (16, 2), (8, 2), (8, 2)])
+    s.step(1 / 60, 9, G, True, 0.9)
+    np.testing.assert_array_equal(s.get_positions(), want[1])
+    np.testing.assert_array_equal(replay(g8, s, st), want[2])
+    g16 = capture_step(s, st)
+    np.testing.assert_array_equal(replay(g16, s, st), want[3])
+    s.set_option(_capi.OPT_CLUSTER_CTAS, 5)
+    s.set_materials(m.mu * np.float32(2), m.lam * np.float32(2))
+    s.step(1 / 60, 9, G, True, 0.9)
+    np.testing.assert_array_equal(s.get_positions(), want[4])
+    np.testing.assert_array_equal(replay(g8, s, st), want[5])
+    np.testing.assert_array_equal(replay(g16, s, st), want[6])
+    s.set_option(_capi.OPT_LANES, 8)
+    s.set_option(_capi.OPT_CLUSTER_CTAS, 0)
+    s.step(1 / 60, 9, G, True, 0.9)
+    np.testing.assert_array_equal(s.get_positions(), want[7])
+    np.testing.assert_array_equal(replay(g8, s, st), want[8])
+    del g8, g16
+    s.close()
+
+
+def test_backward_beside_captured_cluster_steps(gpu_device):
+    """The library's own captured adjoint launches follow the sets that come and go."""
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2, E=2e4)
+    W = np.random.default_rng(3).normal(size=(m.num_verts, 3))
+    s, st = on_stream(m)
+    keep = []
+    for lanes in (8, 16, 8, 4, 16, 8):
+        s.set_option(_capi.OPT_LANES, lanes)
+        s.set_positions(m.x)
+        s.set_velocities(m.v)
+        s.record(2)
+        for _ in range(3):
+            s.step(1 / 60, 9, G, True, 0.9)
+        got = s.backward(W, None, 12, 0.9)
+        s.record(0)
+        if lanes == 8:
+            keep.append(capture_step(s, st))
+        ref = build_solver(m, lanes=lanes, layout=4)
+        ref.set_option(_capi.OPT_PERSISTENT, 0)
+        ref.record(2)
+        for _ in range(3):
+            ref.step(1 / 60, 9, G, True, 0.9)
+        for a, b in zip(got, ref.backward(W, None, 12, 0.9)):
+            np.testing.assert_array_equal(a, b)
+        ref.close()
+    del keep
+    s.close()
+
+
+def test_cluster_step_captured_after_another_shape_was_set(gpu_device):
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2)
+    s, st = on_stream(m)
+    s.set_option(_capi.OPT_LANES, 4)
+    g = capture_step(s, st)
+    np.testing.assert_array_equal(replay(g, s, st), plain(m, [(8, 1), (4, 1)])[1])
+    del g
+    s.close()

@@ -157,6 +157,7 @@ struct TileSet {
     unsigned tag = 1;                // next unused word tag
     int stride = 1;                  // of the exchanged words
     bool no_room = false;            // its memory could not be had
+    bool captured = false;           // launches that the caller captured read this set: it is never laid out again
     // cluster form: the forward and adjoint launches checked to fit the device, and the answers
     const void* checked[2] = {nullptr, nullptr};
     bool resident[2] = {false, false};
@@ -322,7 +323,10 @@ struct vbd_solver {
     vbd::TileSet tset;   // one tile per SM, exchanging words through L2
     vbd::TileSet aset;   // tset's tiles as the adjoint sweeps them, where tset has 16 warps or would not stay resident
     vbd::TileSet wset;   // tset's tiles for VBD_GPU_Solver semantics
-    vbd::TileSet cset;   // one tile per CTA of a cluster, its plan merged from tset's tiles
+    // one tile per CTA of a cluster, its plan merged from tset's tiles; and the sets for other lanes or CTA counts
+    // that launches captured by the caller read
+    std::unique_ptr<vbd::TileSet> cset{new vbd::TileSet()};
+    std::vector<std::unique_ptr<vbd::TileSet>> held;
     int tile_walk = 0;
     bool persistent_set = false;
     std::vector<int32_t> batch_mesh;  // mesh of each vertex, set by vbd_solver_init_batch for its init
@@ -855,8 +859,8 @@ struct vbd_solver {
         if (!cluster_fit(&why)) VBD_FAIL(VBD_ERR_INVALID_ARG, "%s", why);
         VBD_TRY(upload_schedule(iters, accel, rho));
         const int L = lanes < 4 ? 4 : lanes;
-        if (cluster_resident && cluster_tiles(L, false) && tile_room(cset))
-            return launch_tile(cset, iters, dtsr, accel, rho, from_inertia, h, predict ? hg : nullptr, false);
+        if (cluster_resident && cluster_tiles(L, false) && cluster_ready())
+            return launch_tile(*cset, iters, dtsr, accel, rho, from_inertia, h, predict ? hg : nullptr, false);
         void (*fn)(vbd::PersistParams) = nullptr;
         switch (L) {
             case 4: fn = vbd::pick_cluster<4>(layout); break;
@@ -932,18 +936,20 @@ struct vbd_solver {
             vbd::tile_groups(&s.plan, L, w, h_inc_off.data());
         }
     }
+    // Whether the caller is capturing the stream (or that cannot be asked).
+    bool capturing() const {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+        (void)cudaGetLastError();
+        return true;
+    }
     // Whether steps and solves run as tile walks.  Under a caller's stream capture they do not: each
     // launch needs tags of its own, which a replayed launch would repeat.
     bool use_tile() {
         if (!tile_walk || tset.plan.P == 0 || timing || !use_graph || persistent || ninc == 0) return false;
         // VBD_GPU_Solver semantics read the tet records, with lanes of their own
         if (!semantics && (!colour_lanes.empty() || layout < 3 || (lanes != 4 && lanes != 8 && lanes != 16))) return false;
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
-        }
-        if (cs != cudaStreamCaptureStatusNone) return false;
+        if (capturing()) return false;
         if (semantics) {
             if (wset.plan.P == 0) {
                 vbd::TilePlan q = tset.plan;
@@ -990,34 +996,69 @@ struct vbd_solver {
     bool cluster_tiles(int L, bool adjoint) {
         if (tset.plan.P == 0 || C > vbd::kTileMaxColours || layout < 3) return false;
         const int P = std::min({16, tset.plan.P, cluster_ctas_opt > 0 ? cluster_ctas_opt : std::max(1, nfree / vbd::kClusterTileMin)});
-        if (cset.plan.P != P || cset.sums != L) {
-            vbd::TilePlan q;
-            vbd::tile_merge(tset.plan, P, cstart, &q);
-            cset.reset(std::move(q));
-            cset.cluster = true;
-            group_tiles(cset, L, 8, 3);
-        }
+        if ((cset->plan.P != P || cset->sums != L) && !cluster_plan(P, L)) return false;
+        vbd::TileSet& s = *cset;
         const int which = adjoint ? 1 : 0, vectors = adjoint ? 3 : 2;
-        if (!tile_fits(cset, vectors)) return false;
-        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<vbd::kTileAdjoint>(cset.plan, true)
-                                                              : vbd::pick_tile<vbd::kTileForward>(cset.plan, true));
-        if (cset.checked[which] != f) {
-            cset.checked[which] = f;
-            cset.resident[which] = false;
-            const size_t smem = vbd::tile_smem(8, tile_ring_chunks(cset, vectors), cset.chunk_bytes(), cset.plan, C, vectors, true);
+        if (!tile_fits(s, vectors)) return false;
+        const void* f = reinterpret_cast<const void*>(adjoint ? vbd::pick_tile<vbd::kTileAdjoint>(s.plan, true)
+                                                              : vbd::pick_tile<vbd::kTileForward>(s.plan, true));
+        if (s.checked[which] != f) {
+            s.checked[which] = f;
+            s.resident[which] = false;
+            const size_t smem = vbd::tile_smem(8, tile_ring_chunks(s, vectors), s.chunk_bytes(), s.plan, C, vectors, true);
             if (allow_shared(f, true) == cudaSuccess) {
                 cudaLaunchConfig_t cfg = {};
                 cudaLaunchAttribute attr[1];
                 cluster_config(&cfg, attr, P, 256, smem);
                 int clusters = 0;
-                cset.resident[which] = cudaOccupancyMaxActiveClusters(&clusters, f, &cfg) == cudaSuccess && clusters >= 1;
+                s.resident[which] = cudaOccupancyMaxActiveClusters(&clusters, f, &cfg) == cudaSuccess && clusters >= 1;
             }
             (void)cudaGetLastError();
         }
-        return cset.resident[which];
+        return s.resident[which];
+    }
+    // Makes cset the set of P tiles and L lanes.  One that a caller's captured launches read is put by, and is
+    // taken back when it is wanted again.
+    bool cluster_plan(int P, int L) {
+        if (capturing()) return false;
+        if (cset->captured) {
+            held.push_back(std::move(cset));
+            cset.reset(new vbd::TileSet());
+        }
+        for (auto& h : held)
+            if (h->plan.P == P && h->sums == L) {
+                drop_graphs();  // the adjoint's captured launches hold the addresses of the set that goes
+                std::swap(cset, h);
+                std::swap(h, held.back());
+                held.pop_back();
+                return true;
+            }
+        vbd::TilePlan q;
+        vbd::tile_merge(tset.plan, P, cstart, &q);
+        cset->reset(std::move(q));
+        cset->cluster = true;
+        group_tiles(*cset, L, 8, 3);
+        return true;
+    }
+    // Whether cset is on the device, packed from the present records.  While the caller captures the stream
+    // nothing can be packed (a pack that is only captured packs nothing now, and memory cannot be had): a
+    // set that needs it is not used, and one that is used keeps its place and is packed with every new material.
+    bool cluster_ready() {
+        vbd::TileSet& s = *cset;
+        if (!capturing()) return tile_room(s);
+        if (s.dirty || s.layout != layout || s.lanes != s.plan.lanes || s.warps != s.plan.warps) return false;
+        return s.captured = true;
+    }
+    // Readies the cluster's tiles when an option or a mesh calls for them, so that the next step may be one that
+    // the caller captures.
+    int prepare_cluster() {
+        const char* why = nullptr;
+        if (!ready || persistent != 2 || !cluster_resident || capturing() || !cluster_fit(&why)) return VBD_OK;
+        if (cluster_tiles(lanes < 4 ? 4 : lanes, false) && tile_room(*cset)) CUDA_TRY(cudaStreamSynchronize(stream));
+        return VBD_OK;
     }
     // The automatic CTA count of VBD_OPT_CLUSTER_CTAS.
-    int cluster_auto(int L) { return cluster_resident && cluster_tiles(L, false) ? cset.plan.P : cluster_auto_ctas(L); }
+    int cluster_auto(int L) { return cluster_resident && cluster_tiles(L, false) ? cset->plan.P : cluster_auto_ctas(L); }
     void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int ctas, int threads, size_t smem) const {
         cfg->gridDim = dim3(ctas);
         cfg->blockDim = dim3(threads);
@@ -1424,9 +1465,9 @@ struct vbd_solver {
         void (*walk)(vbd::AdjWalkParams) = nullptr;
         vbd::TileSet* tile = nullptr;
         if (!adj_alternate) {
-            const bool walk_tiles = adj_walk() && cluster_resident && cluster_tiles(lanes < 4 ? 4 : lanes, true) && tile_room(cset);
+            const bool walk_tiles = adj_walk() && cluster_resident && cluster_tiles(lanes < 4 ? 4 : lanes, true) && cluster_ready();
             if (walk_tiles) {
-                tile = &cset;
+                tile = cset.get();
             } else if (use_tile()) {
                 tile = &adjoint_tiles();
                 if (!tile_fits(*tile, 2) || !tile_room(*tile)) tile = nullptr;
@@ -1515,7 +1556,8 @@ struct vbd_solver {
     // Captured graphs bake in buffer addresses: every (re)allocation or release of the streamed
     // record copies invalidates them.
     int repack_stream() {
-        tset.dirty = aset.dirty = cset.dirty = wset.dirty = true;
+        tset.dirty = aset.dirty = cset->dirty = wset.dirty = true;
+        for (auto& h : held) h->dirty = true;
         if (layout != 1 && irec.p) {
             drop_graphs();
             irec.release();
@@ -1560,6 +1602,12 @@ struct vbd_solver {
                     rec.p, inc_tet.p, inc_vertex.p, crec.p, cmat.p, (int)ninc);
                 VBD_TRY(check_launch());
             }
+        }
+        // what the caller's captured launches read, as they read the records themselves
+        if (layout >= 3) {
+            for (auto& h : held) VBD_TRY(ensure_tile(*h));
+            if (cset->captured) VBD_TRY(ensure_tile(*cset));
+            else if (persistent == 2 && cset->lanes) (void)tile_room(*cset);
         }
         return VBD_OK;
     }
@@ -1799,7 +1847,8 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     }
     s->tset.reset(std::move(plan));
     s->aset.reset(vbd::TilePlan());
-    s->cset.reset(vbd::TilePlan());
+    s->cset.reset(new vbd::TileSet());
+    s->held.clear();
     s->wset.reset(vbd::TilePlan());
     s->tile_walk = !s->persistent_set && nfree >= vbd::kTileMinVertices;
 
@@ -1896,7 +1945,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     if (s->use_tile()) VBD_TRY(s->ensure_tile(s->walk_tiles()));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     s->ready = true;
-    return VBD_OK;
+    return s->prepare_cluster();
 }
 
 int vbd_solver_init_batch(vbd_solver* s, int32_t M, const int32_t* voff, const int32_t* toff, const float* positions,
@@ -2351,7 +2400,7 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
                 VBD_FAIL(VBD_ERR_INVALID_ARG, "lanes must be 1, 2, 4, 8, 16 or 32");
             s->lanes = value;
             s->lanes_auto = false;
-            return VBD_OK;
+            return s->prepare_cluster();
         case VBD_OPT_PREFETCH:
             if (value < 0 || value > 3) VBD_FAIL(VBD_ERR_INVALID_ARG, "prefetch must be 0, 1, 2 or 3");
             s->prefetch = value;
@@ -2384,18 +2433,14 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
             s->persistent = value;
             s->persistent_set = true;
             s->tile_walk = 0;
-            if (value == 2 && s->ready && s->cluster_resident && s->cluster_tiles(s->lanes < 4 ? 4 : s->lanes, false)) {
-                (void)s->tile_room(s->cset);
-                CUDA_TRY(cudaStreamSynchronize(s->stream));
-            }
-            return VBD_OK;
+            return s->prepare_cluster();
         case VBD_OPT_CLUSTER_CTAS:
             if (value < 0 || value > 16) VBD_FAIL(VBD_ERR_INVALID_ARG, "cluster CTAs must be 0 (automatic) to 16");
             s->cluster_ctas_opt = value;
-            return VBD_OK;
+            return s->prepare_cluster();
         case VBD_OPT_CLUSTER_RESIDENT:
             s->cluster_resident = value ? 1 : 0;
-            return VBD_OK;
+            return s->prepare_cluster();
         case VBD_OPT_L2_PREFETCH:
             s->l2_prefetch = value ? 1 : 0;
             return VBD_OK;
@@ -2429,7 +2474,7 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
                 VBD_TRY(s->repack_stream());
                 CUDA_TRY(cudaStreamSynchronize(s->stream));
             }
-            return VBD_OK;
+            return s->prepare_cluster();
         case VBD_OPT_GRAPH:
             s->use_graph = value ? 1 : 0;
             return VBD_OK;
@@ -2444,6 +2489,7 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
 int vbd_solver_get_option(vbd_solver* s, int32_t option, int32_t* value) {
     vbd::clear_error();
     if (!s || !value) VBD_FAIL(VBD_ERR_INVALID_ARG, "null argument");
+    DeviceScope scope(s->device);
     switch (option) {
         case VBD_OPT_LANES: *value = s->lanes; return VBD_OK;
         case VBD_OPT_LAYOUT: *value = s->layout; return VBD_OK;
