@@ -89,3 +89,91 @@ for refuse in (False, True):
     s.close()
 same(*out)
 """)
+
+
+# VBDsolver and VBD_GPU_Solver semantics; the first launch of a handle, and one between accepted ones
+@pytest.mark.parametrize("semantics", [0, 1])
+def test_steps_without_the_cooperative_launch(gpu_device, run, semantics):
+    run(f"""
+m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2, E=2e4)
+W = np.random.default_rng(3).normal(size=(m.num_verts, 3))
+out = []
+for refuse in ((), (0, 1, 2, 3), (1, 2)):
+    s = build_solver(m, lanes=8, layout=4)
+    s.set_option(_capi.OPT_SEMANTICS, {semantics})
+    res = []
+    for k in range(4):
+        cooperative_error.value = 720 if k in refuse else 0  # cudaErrorCooperativeLaunchTooLarge
+        s.set_option(_capi.OPT_LANES, 16 if k % 2 else 8)
+        s.set_option(_capi.OPT_ENERGY_EVERY, 4 if k == 2 else 0)
+        s.step(1 / 60, 10, G, True, 0.9, 2)
+        res += [s.get_positions(), s.get_velocities(), s.energy_history()]
+        s.update_inertia_from_cpu(m.x)
+        s.solve_vbd(6, 3600.0, True, 0.9, k % 2)
+        res.append(s.get_positions())
+        if not {semantics}:
+            s.record(2)
+            for _ in range(3):
+                s.step(1 / 60, 5, G, True, 0.9)
+            res += s.backward(W, None, 8, 0.9)
+            s.record(0)
+    out.append(res)
+    s.close()
+same(out[0], out[1])
+same(out[0], out[2])
+""")
+
+
+def test_walks_after_a_refused_launch_wait_as_long_as_before(gpu_device, run):
+    """The count of started CTAs does not run ahead: a wait that runs out ends after its limit, not after the time
+    that a CTA may take to start."""
+    run("""
+import time
+m = meshgen.jittered_block(9, 6, 5, seed=3)
+s = build_solver(m, lanes=8, layout=4)
+s.step(1 / 60, 5, G, True, 0.9)
+cooperative_error.value = 720
+s.step(1 / 60, 5, G, True, 0.9)
+cooperative_error.value = 0
+s.set_option(_capi.OPT_LANES, 16)  # the walk is tried again, on the same lists
+out = ctypes.c_int32(0)
+t = time.perf_counter()
+_capi.call("vbd_solver_walk_selftest", s._h, 5000, ctypes.byref(out))
+assert out.value == 1 and time.perf_counter() - t < 5.0
+""")
+
+
+def test_a_stream_of_fewer_sms(gpu_device):
+    """On a green context's stream the walk takes as many tiles as that context has SMs."""
+    import numpy as np
+    import torch
+
+    from vbd_tetmesh_b200 import _capi, build_solver, meshgen
+
+    driver = pytest.importorskip("cuda.bindings.driver")
+    torch.zeros(1, device="cuda")  # the primary context
+
+    def ok(r):
+        assert r[0] == driver.CUresult.CUDA_SUCCESS, r[0]
+        return r[1:] if len(r) > 2 else r[1] if len(r) == 2 else None
+
+    sms = ok(driver.cuDeviceGetDevResource(0, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups, _, _ = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, 16))
+    assert groups[0].sm.smCount < sms.sm.smCount
+    desc = ok(driver.cuDevResourceGenerateDesc(groups, 1))
+    ctx = ok(driver.cuGreenCtxCreate(desc, 0, driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(ctx, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    m = meshgen.jittered_block(20, 12, 11, seed=3)  # more than 16 tiles on the whole device
+    out = []
+    for st in (None, int(stream)):
+        s = build_solver(m, lanes=8, layout=4, stream=st)
+        l0 = s.kernel_launches()
+        s.step(1 / 60, 10, (0.0, -9.8, 0.0), True, 0.9)
+        s.sync()
+        assert s.kernel_launches() - l0 == 1
+        out.append((s.get_positions(), s.get_velocities()))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    ok(driver.cuStreamDestroy(stream))
+    ok(driver.cuGreenCtxDestroy(ctx))

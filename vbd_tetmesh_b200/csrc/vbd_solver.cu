@@ -1,5 +1,6 @@
 // Solver handle of libvbd_b200: device state, launch sequencing, CUDA-graph replay and the
 // solver half of the C ABI declared in include/vbd_b200.h.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -135,6 +136,10 @@ static void (*pick_tile_wrapper(int warps))(TileParams) {
     return warps == 8 ? &k_tile_walk<16, kTileWrapper, 8> : &k_tile_walk<16, kTileWrapper, 16>;
 }
 
+// What launch_tile and tile_launch return where the device refuses a cooperative launch of as many CTAs
+// (nothing of the walk has run then).
+constexpr int kWalkRefused = -1;
+
 // A tile plan on the device.
 struct TileSet {
     TilePlan plan;
@@ -156,7 +161,7 @@ struct TileSet {
     unsigned long long started = 0;  // CTAs of all launches so far
     unsigned tag = 1;                // next unused word tag
     int stride = 1;                  // of the exchanged words
-    bool no_room = false;            // its memory could not be had
+    bool no_room = false;            // its memory could not be had, or its launch was refused
     bool captured = false;           // launches that the caller captured read this set: it is never laid out again
     // cluster form: the forward and adjoint launches checked to fit the device, and the answers
     const void* checked[2] = {nullptr, nullptr};
@@ -557,10 +562,12 @@ struct vbd_solver {
     }
 
     int emit_substep(float h, float dtsr, const float* hg, int iters, bool accel, float rho,
-                     bool record_energy = false) {
-        vbd::k_predict<<<vbd::nblk(N, 256), 256, 0, stream>>>(x0.p, v.p, xprev.p, y.p, nfree, N, h, hg[0], hg[1],
-                                                              hg[2]);
-        VBD_TRY(check_launch());
+                     bool record_energy = false, bool predicted = false) {
+        if (!predicted) {
+            vbd::k_predict<<<vbd::nblk(N, 256), 256, 0, stream>>>(x0.p, v.p, xprev.p, y.p, nfree, N, h, hg[0], hg[1],
+                                                                  hg[2]);
+            VBD_TRY(check_launch());
+        }
         if (semantics) {
             // main.cpp's GPU loop: solveVBD starts every substep from the inertial target
             // (VBD_GPU_Wrapper.cu:334)
@@ -962,8 +969,8 @@ struct vbd_solver {
         }
         return tile_fits(walk_tiles(), 1) && tile_room(walk_tiles());
     }
-    // Whether the device has (or just gave) the memory of a set's records and words; without it the per-colour
-    // launches run, or the cluster walk with whole-mesh copies.
+    // Whether the device has (or just gave) the memory of a set's records and words, and has not refused its
+    // launch; else the per-colour launches run, or the cluster walk with whole-mesh copies.
     bool tile_room(vbd::TileSet& s) {
         if (!s.no_room && ensure_tile(s) == VBD_ERR_ALLOC) {
             vbd::clear_error();
@@ -1174,9 +1181,8 @@ struct vbd_solver {
             w.words = s.words;
             w.word_stride = s.stride;
             w.arrived = reinterpret_cast<unsigned long long*>(s.words + s.nwords - 1);
-            w.arrived_target = (s.started += (unsigned)q.P);
+            w.arrived_target = s.started + (unsigned)q.P;
             w.tag = s.tag - (unsigned)k0;
-            s.tag += (unsigned)(k1 - k0);
         }
         w.chunk = s.chunk;
         w.head = reinterpret_cast<const vbd::TileHead*>(s.ints(S::HEAD));
@@ -1212,7 +1218,7 @@ struct vbd_solver {
         return VBD_OK;
     }
 
-    int tile_launch(const vbd::TileSet& s, void (*fn)(vbd::TileParams), vbd::TileParams& w, int vectors) {
+    int tile_launch(vbd::TileSet& s, void (*fn)(vbd::TileParams), vbd::TileParams& w, int vectors) {
         const size_t smem = vbd::tile_smem(s.plan.warps, w.ring_chunks, s.chunk_bytes(), s.plan, C, vectors, s.cluster);
         CUDA_TRY(allow_shared(reinterpret_cast<const void*>(fn), s.cluster));
         if (s.cluster) {
@@ -1223,13 +1229,22 @@ struct vbd_solver {
             return check_launch();
         }
         void* args[] = {&w};
-        CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(s.plan.P), dim3(32 * s.plan.warps), args,
-                                             smem, stream));
+        const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(s.plan.P),
+                                                          dim3(32 * s.plan.warps), args, smem, stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            (void)cudaGetLastError();
+            s.no_room = true;
+            return vbd::kWalkRefused;
+        }
+        CUDA_TRY(e);
+        s.started += (unsigned)s.plan.P;
+        s.tag += (unsigned)(w.k1 - w.k0);
         return check_launch();
     }
 
     // A sub-step (hg given: predictor and velocity update) or a solve as tile walks: one launch, or one
-    // per energy evaluation with an energy history (emit_iterations' schedule).
+    // per energy evaluation with an energy history (emit_iterations' schedule).  kWalkRefused: nothing has run but,
+    // with VBD_GPU_Solver semantics, the predictor.
     int launch_tile(vbd::TileSet& s, int iters, float dtsr, bool accel, float rho, bool from_inertia, float h,
                     const float* hg, bool record_energy) {
         VBD_TRY(upload_schedule(iters, accel, rho));
@@ -1301,8 +1316,10 @@ struct vbd_solver {
         w.wait_ns = 1000ull * (unsigned long long)wait_us;
         w.x0 = x.p;
         w.pp = pp.p;
-        VBD_TRY(tile_launch(s, s.wrapper ? vbd::pick_tile_wrapper(s.plan.warps) : vbd::pick_tile<vbd::kTileForward>(s.plan, false),
-                            w, 1));
+        const int rc = tile_launch(
+            s, s.wrapper ? vbd::pick_tile_wrapper(s.plan.warps) : vbd::pick_tile<vbd::kTileForward>(s.plan, false), w, 1);
+        if (rc == vbd::kWalkRefused) VBD_FAIL(VBD_ERR_STATE, "the device refuses the walk's launch");
+        VBD_TRY(rc);
         unsigned long long t = 0;
         CUDA_TRY(cudaMemcpyAsync(&t, status.p + vbd::ST_WALK_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1346,7 +1363,10 @@ struct vbd_solver {
         key.rho = t.rho;
         if (persistent && !timing)
             return launch_walk(t.iters, t.dtsr, t.accel != 0, t.rho, true, true, false, t.h, t.hg);
-        if (use_tile()) return launch_tile(tset, t.iters, t.dtsr, t.accel != 0, t.rho, false, t.h, t.hg, false);
+        if (use_tile()) {
+            const int rc = launch_tile(tset, t.iters, t.dtsr, t.accel != 0, t.rho, false, t.h, t.hg, false);
+            if (rc != vbd::kWalkRefused) return rc;
+        }
         return run(key, [&] { return emit_substep(t.h, t.dtsr, t.hg, t.iters, t.accel != 0, t.rho); });
     }
 
@@ -1482,15 +1502,17 @@ struct vbd_solver {
             key.block = ca_ctas;
         }
         // a launch that exchanges words needs tags of its own each time: no graph
-        if (tile && !tile->cluster) {
-            VBD_TRY(emit_adjoint_substep(t, X, sweeps, rho, nullptr, tile));
-        } else {
+        int rc = vbd::kWalkRefused;
+        if (tile && !tile->cluster) rc = emit_adjoint_substep(t, X, sweeps, rho, nullptr, tile);
+        if (rc == vbd::kWalkRefused) {
+            if (tile && !tile->cluster) tile = nullptr;
             if (tile) {
                 key.walk = 3;
                 key.block = tile->plan.P;
             }
-            VBD_TRY(run(key, [&] { return emit_adjoint_substep(t, X, sweeps, rho, walk, tile); }));
+            rc = run(key, [&] { return emit_adjoint_substep(t, X, sweeps, rho, walk, tile); });
         }
+        VBD_TRY(rc);
         float omega = 1.0f;
         for (int it = 1; it <= sweeps && rho > 0.0f; ++it) {
             omega = vbd::omega_of(it, rho, omega);
@@ -1633,6 +1655,25 @@ struct DeviceScope {
     }
 };
 
+// The SMs that launches on `stream` may use: fewer than the device's where the stream belongs to a green context.
+int stream_sms(cudaStream_t stream, int device_sms) {
+    void *of_stream = nullptr, *resource = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetGreenCtx", &of_stream, 12040, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess ||
+        cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &resource, 12040, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
+        return device_sms;
+    }
+    CUgreenCtx ctx = nullptr;
+    CUdevResource r{};
+    if (reinterpret_cast<decltype(&cuStreamGetGreenCtx)>(of_stream)(stream, &ctx) != CUDA_SUCCESS || !ctx ||
+        reinterpret_cast<decltype(&cuGreenCtxGetDevResource)>(resource)(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return device_sms;
+    return std::max(1, std::min<int>(device_sms, (int)r.sm.smCount));
+}
+
 int need_ready(vbd_solver* s) {
     if (!s) VBD_FAIL(VBD_ERR_INVALID_ARG, "null solver handle");
     if (!s->ready) VBD_FAIL(VBD_ERR_STATE, "solver has no mesh: call vbd_solver_init first");
@@ -1667,7 +1708,7 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
         CUDA_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
         s->own_stream = true;
     }
-    s->sm_count = prop.multiProcessorCount;
+    s->sm_count = stream_sms(s->stream, prop.multiProcessorCount);
     s->smem_optin = (int)prop.sharedMemPerBlockOptin;
     VBD_TRY(s->status.alloc(vbd::ST_HOST + 1));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&s->wait_flag), sizeof(unsigned), cudaHostAllocMapped));
@@ -2104,9 +2145,11 @@ int vbd_solver_solve(vbd_solver* s, int32_t iterations, float dt_sqr_reciprocal,
     if (s->persistent && !s->timing)
         return s->launch_walk(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, false, false,
                               init_mode == VBD_INIT_FROM_INERTIA, 1.0f, nullptr);
-    if (s->use_tile())
-        return s->launch_tile(s->walk_tiles(), iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode == VBD_INIT_FROM_INERTIA,
-                              1.0f, nullptr, false);
+    if (s->use_tile()) {
+        const int rc = s->launch_tile(s->walk_tiles(), iterations, dt_sqr_reciprocal, use_acceleration != 0, rho,
+                                      init_mode == VBD_INIT_FROM_INERTIA, 1.0f, nullptr, false);
+        if (rc != vbd::kWalkRefused) return rc;
+    }
     return s->run(key, [&] { return s->emit_solve(iterations, dt_sqr_reciprocal, use_acceleration != 0, rho, init_mode); });
 }
 
@@ -2151,14 +2194,19 @@ int vbd_solver_step(vbd_solver* s, float dt, int32_t substeps, int32_t iteration
     for (int k = 0; k < substeps; ++k) {
         // the persistent kernel evaluates no energies: with an energy history the step runs as
         // separate launches
-        if (s->persistent && !s->timing && nenergy == 0)
-            VBD_TRY(s->launch_walk(iterations, dtsr, use_acceleration != 0, rho, true, true, false, h, hg));
-        else if (s->use_tile())
-            VBD_TRY(s->launch_tile(s->walk_tiles(), iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0));
-        else
-            VBD_TRY(s->run(key, [&] {
-                return s->emit_substep(h, dtsr, hg, iterations, use_acceleration != 0, rho, nenergy > 0);
-            }));
+        int rc = vbd::kWalkRefused;
+        bool predicted = false;
+        if (s->persistent && !s->timing && nenergy == 0) {
+            rc = s->launch_walk(iterations, dtsr, use_acceleration != 0, rho, true, true, false, h, hg);
+        } else if (s->use_tile()) {
+            rc = s->launch_tile(s->walk_tiles(), iterations, dtsr, use_acceleration != 0, rho, false, h, hg, nenergy > 0);
+            predicted = s->semantics != 0;
+        }
+        const auto emit = [&] {
+            return s->emit_substep(h, dtsr, hg, iterations, use_acceleration != 0, rho, nenergy > 0, predicted);
+        };
+        if (rc == vbd::kWalkRefused) rc = predicted ? emit() : s->run(key, emit);
+        VBD_TRY(rc);
         VBD_TRY(s->record_substep(h, dtsr, hg, iterations, use_acceleration != 0, rho));
     }
     s->ehist_queued += nenergy;
