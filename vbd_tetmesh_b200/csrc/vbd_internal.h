@@ -5,8 +5,8 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdint>
+#include <exception>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -41,22 +41,32 @@ constexpr double kFactoredDegenerate = 1e-3;
 constexpr double kFactoredLossFraction = 1e-3;
 
 // fn(worker, item) for every item in [0, items), workers in [0, kMaxWorkers), over several host threads
-// when the work is large (a set-up loop of milliseconds).  Fewer threads where none can be made.
+// when the work is large (a set-up loop of milliseconds).  Fewer threads where none can be made.  An exception
+// of fn reaches the caller once every worker has ended (one of them, where several throw).
 constexpr int kMaxWorkers = 16;
 template <class Fn> void each_item(int items, bool large, Fn fn) {
     const int workers =
         large ? (int)std::max(1u, std::min((unsigned)kMaxWorkers, std::thread::hardware_concurrency())) : 1;
     std::atomic<int> next{0};
+    std::atomic<bool> failed{false};
+    std::exception_ptr error;
     auto run = [&](int w) {
-        for (int i; (i = next.fetch_add(1)) < items;) fn(w, i);
+        try {
+            for (int i; (i = next.fetch_add(1)) < items;) fn(w, i);
+        } catch (...) {
+            if (!failed.exchange(true)) error = std::current_exception();
+            next = items;
+        }
     };
     std::vector<std::thread> ts;
     try {
+        ts.reserve(workers);
         for (int w = 1; w < workers && w < items; ++w) ts.emplace_back(run, w);
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {
     }
     run(0);
     for (auto& t : ts) t.join();
+    if (error) std::rethrow_exception(error);
 }
 
 // The same over ranges [b, e) of n elements.
