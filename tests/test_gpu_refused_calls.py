@@ -18,6 +18,8 @@ sys.path.insert(0, {root!r})
 from vbd_tetmesh_b200 import _capi, build_solver, meshgen
 fake = ctypes.CDLL({fake!r})
 malloc_limit = ctypes.c_size_t.in_dll(fake, "fake_malloc_limit")
+memory = ctypes.c_size_t.in_dll(fake, "fake_memory")
+memory_limit = ctypes.c_size_t.in_dll(fake, "fake_memory_limit")
 cooperative_error = ctypes.c_int.in_dll(fake, "fake_cooperative_error")
 G = (0.0, -9.8, 0.0)
 NONE = 2**64 - 1
@@ -177,3 +179,43 @@ def test_a_stream_of_fewer_sms(gpu_device):
         np.testing.assert_array_equal(a, b)
     ok(driver.cuStreamDestroy(stream))
     ok(driver.cuGreenCtxDestroy(ctx))
+
+
+def test_recording_buffers_give_way(gpu_device, run):
+    """Buffers kept from a long recording are no reason to refuse another recording or its backward pass, and a new
+    mesh and the end of recording give them back."""
+    run("""
+from vbd_tetmesh_b200 import color_vertices, mesh_mass, precompute_tets
+m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2, E=2e4)
+W = np.random.default_rng(3).normal(size=(m.num_verts, 3))
+def recorded(s, every, steps):
+    s.set_positions(m.x)
+    s.set_velocities(m.v)
+    s.record(every)
+    for _ in range(steps):
+        s.step(1 / 60, 5, G, True, 0.9)
+    return s.backward(W, None, 8, 0.9)
+s = build_solver(m, lanes=8, layout=4)
+want = recorded(s, 16, 20)
+s.close()
+s = build_solver(m, lanes=8, layout=4)
+s.step(1 / 60, 5, G, True, 0.9)
+before = memory.value
+s.record(1)
+for _ in range(60):
+    s.step(1 / 60, 5, G, True, 0.9)
+memory_limit.value = memory.value  # what the long recording took is all there is
+same(want, recorded(s, 16, 20))
+memory_limit.value = NONE
+s.record(0)
+kept = memory.value
+s.record(1)
+for _ in range(60):
+    s.step(1 / 60, 5, G, True, 0.9)
+s.record(1)
+_, offs, verts = color_vertices(m.num_verts, m.tets)
+dminv, v0 = precompute_tets(m.rest, m.tets)
+s.init_from_cpu(m.x, mesh_mass(m.rest, m.tets, m.density)[0], m.fixed, m.tets, offs, verts, dminv, v0, m.mu, m.lam)
+assert memory.value <= kept + 4 * 32 * m.num_verts, (memory.value, kept)
+s.close()
+""")

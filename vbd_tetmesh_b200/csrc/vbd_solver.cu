@@ -314,8 +314,19 @@ struct vbd_solver {
             ckpts.push_back(std::move(ckpt_pool.back()));
             ckpt_pool.pop_back();
         }
-        if (ckpts.back()->n != 2 * (size_t)N) VBD_TRY(ckpts.back()->alloc(2 * (size_t)N));
+        if (ckpts.back()->n != 2 * (size_t)N) VBD_TRY(tape_alloc(*ckpts.back(), 2 * (size_t)N));
         return snapshot(*ckpts.back());
+    }
+    // Memory of a recording or a backward pass; buffers kept from earlier recordings give way where there is none left.
+    template <class T> int tape_alloc(vbd::DBuf<T>& b, size_t n) {
+        int rc = b.alloc(n);
+        if (rc == VBD_ERR_ALLOC && !ckpt_pool.empty()) {
+            vbd::clear_error();
+            (void)cudaGetLastError();
+            ckpt_pool.clear();
+            rc = b.alloc(n);
+        }
+        return rc;
     }
     vbd::DBuf<float4> adj_lam, adj_lam2, adj_lpp, adj_G, adj_ax, adj_av, adj_seg, adj_save;
     // converged positions of the recorded sub-steps of the newest segment, kept as the forward runs
@@ -1778,6 +1789,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     DeviceScope scope(s->device);
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     *s->wait_flag = 0;  // of the previous mesh
+    s->ckpt_pool.clear();
     s->ready = false;
     s->drop_graphs();
     s->irec.release();
@@ -2248,7 +2260,7 @@ int vbd_solver_record(vbd_solver* s, int32_t checkpoint_every) {
     DeviceScope scope(s->device);
     if (checkpoint_every > 0) VBD_TRY(s->finish());  // of a state to start from
     s->tape.clear();
-    // a new recording reuses the last one's buffers; stopping gives them back
+    // a new recording reuses the last one's buffers; stopping, and a new mesh, give them back
     if (checkpoint_every == 0) s->ckpt_pool.clear();
     else for (auto& c : s->ckpts) s->ckpt_pool.push_back(std::move(c));
     s->ckpts.clear();
@@ -2256,7 +2268,7 @@ int vbd_solver_record(vbd_solver* s, int32_t checkpoint_every) {
     if (checkpoint_every > 0) {
         if (s->live_seg.n != (size_t)checkpoint_every * s->N) {
             s->drop_graphs();
-            VBD_TRY(s->live_seg.alloc((size_t)checkpoint_every * s->N));
+            VBD_TRY(s->tape_alloc(s->live_seg, (size_t)checkpoint_every * s->N));
         }
         VBD_TRY(s->add_ckpt());
         CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -2279,17 +2291,17 @@ int vbd_solver_backward(vbd_solver* s, const float* dl_dx, const float* dl_dv, i
     for (auto* b : {&s->adj_lam, &s->adj_lam2, &s->adj_lpp, &s->adj_G, &s->adj_ax, &s->adj_av})
         if (b->n != (size_t)N) {
             s->drop_graphs();
-            VBD_TRY(b->alloc(N));
+            VBD_TRY(s->tape_alloc(*b, N));
         }
     if (s->adj_seg.n != (size_t)K * N) {
         s->drop_graphs();
-        VBD_TRY(s->adj_seg.alloc((size_t)K * N));
+        VBD_TRY(s->tape_alloc(s->adj_seg, (size_t)K * N));
     }
-    if (s->adj_save.n != 6 * (size_t)N) VBD_TRY(s->adj_save.alloc(6 * (size_t)N));
+    if (s->adj_save.n != 6 * (size_t)N) VBD_TRY(s->tape_alloc(s->adj_save, 6 * (size_t)N));
     if (s->adj_gmu.n != (size_t)std::max(T, 1)) {
         s->drop_graphs();
-        VBD_TRY(s->adj_gmu.alloc(std::max(T, 1)));
-        VBD_TRY(s->adj_glam.alloc(std::max(T, 1)));
+        VBD_TRY(s->tape_alloc(s->adj_gmu, std::max(T, 1)));
+        VBD_TRY(s->tape_alloc(s->adj_glam, std::max(T, 1)));
     }
     // keep the caller's state; the recompute overwrites it
     float4* live[6] = {s->x0.p, s->x1.p, s->pp.p, s->y.p, s->v.p, s->xprev.p};
