@@ -219,3 +219,32 @@ s.init_from_cpu(m.x, mesh_mass(m.rest, m.tets, m.density)[0], m.fixed, m.tets, o
 assert memory.value <= kept + 4 * 32 * m.num_verts, (memory.value, kept)
 s.close()
 """)
+
+
+def test_options_give_unused_walk_memory_back(gpu_device, run):
+    run("""
+m = meshgen.jittered_block(20, 12, 11, seed=3, per_tet_sigma=0.2)
+def steps(s):
+    s.set_positions(m.x)
+    s.set_velocities(m.v)
+    s.step(1 / 60, 5, G, True, 0.9)
+    return s.get_positions(), s.get_velocities()
+s = build_solver(m, lanes=8, layout=4)
+made = memory.value
+s.set_option(_capi.OPT_PERSISTENT, 0)
+base = memory.value
+assert base < made - 44 * 4 * m.num_tets * 0.8, (base, made)  # the records, less those of pinned vertices
+graph = steps(s)
+s.close()
+s = build_solver(m, lanes=8, layout=4)
+s.set_option(_capi.OPT_SEMANTICS, 1)  # the other semantics' set instead of, not beside, the one made at init
+assert memory.value - base < 2.2 * (made - base), (memory.value, base, made)
+wrapper = steps(s)
+s.set_option(_capi.OPT_SEMANTICS, 0)
+same(steps(s), graph)
+both = memory.value
+s.set_option(_capi.OPT_SEMANTICS, 1)  # both have run: kept
+assert memory.value == both
+same(steps(s), wrapper)
+s.close()
+""")

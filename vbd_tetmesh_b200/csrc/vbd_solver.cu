@@ -1090,6 +1090,14 @@ struct vbd_solver {
         cfg->numAttrs = 1;
     }
 
+    // Gives the memory of a set that no step will use back; it is made again if one does.
+    void give_back(vbd::TileSet& s) {
+        if (!s.mem.p || capturing()) return;
+        s.mem.release();
+        s.lanes = s.warps = 0;
+        s.dirty = true;
+    }
+
     // The plan's lists and the record chunks on the device, made when first needed for the current lanes, layout
     // and materials.
     int ensure_tile(vbd::TileSet& s) {
@@ -2493,6 +2501,7 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
             s->persistent = value;
             s->persistent_set = true;
             s->tile_walk = 0;
+            for (auto* t : {&s->tset, &s->aset, &s->wset}) s->give_back(*t);
             return s->prepare_cluster();
         case VBD_OPT_CLUSTER_CTAS:
             if (value < 0 || value > 16) VBD_FAIL(VBD_ERR_INVALID_ARG, "cluster CTAs must be 0 (automatic) to 16");
@@ -2511,6 +2520,7 @@ int vbd_solver_set_option(vbd_solver* s, int32_t option, int32_t value) {
             if (value && s->ckpt_every > 0)
                 VBD_FAIL(VBD_ERR_STATE, "recording for the adjoint is on; the adjoint needs the VBDsolver semantics");
             s->semantics = value;
+            if (value && s->tset.started == 0) s->give_back(s->tset);  // made at init, and no step has run it
             if (value && s->ready && s->use_tile()) {
                 VBD_TRY(s->ensure_tile(s->wset));
                 CUDA_TRY(cudaStreamSynchronize(s->stream));
