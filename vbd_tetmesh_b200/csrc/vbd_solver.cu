@@ -120,10 +120,11 @@ template <int L> static void (*pick_cluster_adjoint(int layout))(AdjWalkParams) 
 // The tile walk runs lanes / 2 threads per vertex; it reads its own record chunks, packed from the
 // factored records of either layout.  With `cluster` the tiles are the CTAs of one cluster.
 template <TileKind KIND, int W, bool CL> static void (*pick_tile_form(int lanes, bool stack))(TileParams) {
-    if (stack)
-        return lanes == 8    ? &k_tile_walk<4, KIND, W, CL, true>
-               : lanes == 16 ? &k_tile_walk<8, KIND, W, CL, true>
-                             : &k_tile_walk<16, KIND, W, CL, true>;
+    if constexpr (W == 8)  // group_tiles stacks for 8 warps only
+        if (stack)
+            return lanes == 8    ? &k_tile_walk<4, KIND, W, CL, true>
+                   : lanes == 16 ? &k_tile_walk<8, KIND, W, CL, true>
+                                 : &k_tile_walk<16, KIND, W, CL, true>;
     if (CL && lanes == 32) return &k_tile_walk<16, KIND, 8, true>;
     return lanes == 4 ? &k_tile_walk<2, KIND, W, CL> : lanes == 8 ? &k_tile_walk<4, KIND, W, CL> : &k_tile_walk<8, KIND, W, CL>;
 }
