@@ -260,3 +260,43 @@ def test_cluster_step_captured_after_another_shape_was_set(gpu_device):
     np.testing.assert_array_equal(replay(g, s, st), plain(m, [(8, 1), (4, 1)])[1])
     del g
     s.close()
+
+
+@pytest.mark.parametrize("semantics", [0, 1])
+@pytest.mark.parametrize("warm_up", [True, False])
+def test_default_step_and_solve_captured_by_the_caller(gpu_device, semantics, warm_up):
+    """The walk that a default step takes cannot be captured; the per-colour launches are captured in its place,
+    whether or not a step has run before."""
+    import torch
+
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2)
+    out = []
+    for captured in (True, False):
+        st = torch.cuda.Stream()
+        s = build_solver(m, lanes=8, layout=4, stream=st.cuda_stream)
+        s.set_option(_capi.OPT_SEMANTICS, semantics)
+        if not captured:
+            s.set_option(_capi.OPT_PERSISTENT, 0)
+        if warm_up:
+            s.step(1 / 60, 9, G, True, 0.9)
+        s.sync()
+
+        def steps():
+            s.step(1 / 60, 9, G, True, 0.9, 2)
+            s.solve_vbd(7, 3600.0, True, 0.9, 0)
+
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=st):
+                steps()
+            for _ in range(2):
+                x = replay(g, s, st)
+            del g
+        else:
+            steps()
+            steps()
+            x = s.get_positions()
+        out.append((x, s.get_velocities()))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)

@@ -1546,6 +1546,8 @@ struct vbd_solver {
         vbd::GraphEntry* hit = nullptr;
         for (auto& g : graphs)
             if (g.key == key) hit = &g;
+        // the caller is capturing the stream: the launches go straight into that capture
+        if (!hit && capturing()) return emit();
         if (!hit) {
             vbd::GraphEntry e;
             e.key = key;
