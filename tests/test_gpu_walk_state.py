@@ -300,3 +300,64 @@ def test_default_step_and_solve_captured_by_the_caller(gpu_device, semantics, wa
         s.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_changing_schedules_are_queued_without_waiting(gpu_device):
+    """A step with another schedule than the one before returns while that one is still at work, as with the same
+    schedule: schedules used before, and a new one."""
+    import torch
+
+    st = torch.cuda.Stream()
+    s = build_solver(meshgen.cube(32), stream=st.cuda_stream)
+    for n, accel, rho in ((2000, True, 0.9), (20, False, 0.9), (25, True, 0.95)):
+        s.step(1 / 120, n, G, accel, rho)
+    s.sync()
+    for n, accel, rho in ((20, False, 0.9), (25, True, 0.95), (30, True, 0.8)):
+        s.step(1 / 120, 2000, G, True, 0.9)  # about 5 ms
+        before = torch.cuda.Event()
+        before.record(st)
+        s.step(1 / 120, n, G, accel, rho)
+        assert not before.query()
+        s.sync()
+    s.close()
+
+
+@pytest.mark.parametrize("persistent", [None, 1, 2])
+def test_many_schedules_equal_the_graph(gpu_device, persistent):
+    """More schedules than are kept, prefixes of one another, with and without blending, in turn."""
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2)
+    shapes = [(n, accel, rho) for n in (3, 12, 7) for accel, rho in ((True, 0.9), (True, 0.95), (False, 0.0), (True, 0.5))]
+    order = np.random.default_rng(1).integers(0, len(shapes), 40)
+    out = []
+    for p in (persistent, 0):
+        s = build_solver(m, lanes=8, layout=4)
+        if p is not None:
+            s.set_option(_capi.OPT_PERSISTENT, p)
+        for k in order:
+            n, accel, rho = shapes[k]
+            s.step(1 / 60, n, G, accel, rho)
+        out.append((s.get_positions(), s.get_velocities()))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("persistent", [1, 2])
+def test_captured_step_keeps_its_schedule(gpu_device, persistent):
+    m = meshgen.jittered_block(9, 6, 5, seed=3, per_tet_sigma=0.2)
+    s, st = on_stream(m)
+    s.set_option(_capi.OPT_PERSISTENT, persistent)
+    s.step(1 / 60, 9, G, True, 0.9)
+    g = capture_step(s, st)
+    ref = build_solver(m, lanes=8, layout=4)
+    ref.set_option(_capi.OPT_PERSISTENT, 0)
+    for _ in range(2):
+        ref.step(1 / 60, 9, G, True, 0.9)
+    for k in range(10):
+        for t in (s, ref):
+            t.step(1 / 60, 9, G, True, 0.5 + 0.04 * k)
+    ref.step(1 / 60, 9, G, True, 0.9)
+    np.testing.assert_array_equal(replay(g, s, st), ref.get_positions())
+    del g
+    s.close()
+    ref.close()

@@ -294,9 +294,16 @@ struct vbd_solver {
     std::vector<float> adj_omega_cache;
     long long spin_limit = 1LL << 22;               // barrier polls before a persistent launch gives up
     vbd::DBuf<int> d_cstart;
-    vbd::DBuf<float> d_omega;
+    // Chebyshev schedules on the device, the last used last: a step with another schedule than the step before
+    // uploads nothing and waits for nothing
+    struct Schedule {
+        std::vector<float> w;
+        vbd::DBuf<float> d;
+        bool captured = false;  // launches that the caller captured read it: it is never overwritten
+    };
+    std::vector<std::unique_ptr<Schedule>> schedules;
+    const float* omega_at = nullptr;  // of the last upload_schedule
     vbd::DBuf<vbd::GridBarrier> barrier;
-    std::vector<float> omega_cache;
     int adj_alternate = 0;  // adjoint sweeps alternate the colour order (symmetric Gauss-Seidel pairs)
     // adjoint tape: sub-steps taken since vbd_solver_record, (x, v) every ckpt_every sub-steps
     struct TapeStep {
@@ -621,7 +628,7 @@ struct vbd_solver {
         return w;
     }
 
-    // The colour starts and the Chebyshev schedule on the device, for the single-launch walks.
+    // The colour starts and the Chebyshev schedule (omega_at) on the device, for the single-launch walks.
     int upload_schedule(int iters, bool accel, float rho) {
         if (d_cstart.n != cstart.size()) {
             VBD_TRY(d_cstart.alloc(cstart.size()));
@@ -629,12 +636,33 @@ struct vbd_solver {
             CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));  // landed before any kernel of `stream`
         }
         std::vector<float> w = omega_schedule(iters, accel, rho);
-        if (w != omega_cache) {
-            if (d_omega.n < w.size()) VBD_TRY(d_omega.alloc(w.size()));
-            CUDA_TRY(cudaMemcpyAsync(d_omega.p, w.data(), sizeof(float) * w.size(), cudaMemcpyHostToDevice, stream));
-            CUDA_TRY(cudaStreamSynchronize(stream));
-            omega_cache = w;
+        const bool captured = persistent && capturing();
+        size_t at = schedules.size();
+        while (at > 0 && !(schedules[at - 1]->w.size() >= w.size() && std::equal(w.begin(), w.end(), schedules[at - 1]->w.begin())))
+            --at;
+        std::unique_ptr<Schedule> s;
+        if (at > 0) {  // it, or one that starts with it
+            s = std::move(schedules[at - 1]);
+            schedules.erase(schedules.begin() + (at - 1));
+        } else {
+            if (captured) VBD_FAIL(VBD_ERR_STATE, "run a step with these iterations and weights before capturing one");
+            if (schedules.size() >= 8)
+                for (auto i = schedules.begin(); i != schedules.end() && !s; ++i)
+                    if (!(*i)->captured) {
+                        s = std::move(*i);
+                        schedules.erase(i);
+                        break;
+                    }
+            if (!s) s.reset(new Schedule());
+            s->w.clear();
+            if (s->d.n < w.size()) VBD_TRY(s->d.alloc(std::max<size_t>(w.size(), 64)));
+            // pageable memory: read before the call returns
+            CUDA_TRY(cudaMemcpyAsync(s->d.p, w.data(), sizeof(float) * w.size(), cudaMemcpyHostToDevice, stream));
+            s->w = std::move(w);
         }
+        s->captured = s->captured || captured;
+        omega_at = s->d.p;
+        schedules.push_back(std::move(s));
         return VBD_OK;
     }
 
@@ -649,7 +677,7 @@ struct vbd_solver {
         w.v = v.p;
         w.xprev = xprev.p;
         w.cstart = d_cstart.p;
-        w.omega = d_omega.p;
+        w.omega = omega_at;
         w.ncol = C;
         w.iters = iters;
         w.nfree = nfree;
@@ -1282,7 +1310,7 @@ struct vbd_solver {
             // both position buffers in shared memory where that leaves the rings their depth
             const int two = s.cluster || (accel && (tile_resident(s, 2) || (!tile_resident(s, 1) && tile_ring(s, 2) >= vbd::kTileTwoRing)));
             vbd::TileParams w;
-            VBD_TRY(tile_params(s, k0, k1, dtsr, d_omega.p, accel, 1 + two, &w));
+            VBD_TRY(tile_params(s, k0, k1, dtsr, omega_at, accel, 1 + two, &w));
             w.two = two;
             w.x0 = x0.p;
             w.x1 = x1.p;
@@ -1331,7 +1359,7 @@ struct vbd_solver {
         CUDA_TRY(cudaMemcpyAsync(list.p, groups.data(), sizeof(vbd::TileGroup) * groups.size(), cudaMemcpyHostToDevice, stream));
         CUDA_TRY(cudaMemcpyAsync(x.p, x0.p, sizeof(float4) * (size_t)N, cudaMemcpyDeviceToDevice, stream));
         vbd::TileParams w;
-        VBD_TRY(tile_params(s, 0, 3, 3600.0f, d_omega.p, false, 1, &w));
+        VBD_TRY(tile_params(s, 0, 3, 3600.0f, omega_at, false, 1, &w));
         w.groups = list.p;
         w.wait_ns = 1000ull * (unsigned long long)wait_us;
         w.x0 = x.p;
@@ -2004,6 +2032,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     s->ninc = ninc;
     s->cstart = cstart;
     s->d_cstart.release();
+    s->schedules.clear();
     s->have_materials = tet_mu != nullptr;
     VBD_TRY(s->repack_stream());
     if (s->use_tile()) VBD_TRY(s->ensure_tile(s->walk_tiles()));
