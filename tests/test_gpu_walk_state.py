@@ -118,6 +118,19 @@ def test_a_wait_that_ran_out_is_reported_once(gpu_device, call):
     fresh.close()
 
 
+def test_the_barrier_selftest_leaves_a_walks_report(gpu_device):
+    s = build_solver(meshgen.jittered_block(7, 6, 5, seed=5))
+    assert give_up(s) == 1
+    out = C.c_int32(0)
+    _capi.call("vbd_solver_barrier_selftest", s._h, 2000, C.byref(out))
+    assert out.value == 1
+    with pytest.raises(_capi.VBDError) as e:
+        s.get_positions()
+    assert e.value.code == 6  # VBD_ERR_TIMEOUT
+    s.sync()
+    s.close()
+
+
 def test_a_new_mesh_starts_without_the_last_ones_report(gpu_device):
     from vbd_tetmesh_b200 import color_vertices, mesh_mass, precompute_tets
 

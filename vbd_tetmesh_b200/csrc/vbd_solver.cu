@@ -2418,11 +2418,11 @@ int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* time
     s->spin_limit = saved;
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    unsigned long long t = 0;
-    CUDA_TRY(cudaMemcpy(&t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
-    *s->wait_flag = 0;
-    *timed_out = t ? 1 : 0;
+    unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
+    CUDA_TRY(cudaMemcpy(t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t[0]), s->stream));
+    if (!t[1]) *s->wait_flag = 0;  // a walk's record stays for the call that reports it
+    *timed_out = t[0] ? 1 : 0;
     return VBD_OK;
 }
 
