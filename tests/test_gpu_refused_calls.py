@@ -145,6 +145,46 @@ assert out.value == 1 and time.perf_counter() - t < 5.0
 """)
 
 
+# about 4,300 and 7,300 free vertices a tile: the vertex data, ids and two chunks per warp fit in an SM's shared memory
+# up to about 6,000
+@pytest.mark.parametrize("n,walks", [(40, True), (48, False)])
+def test_tiles_larger_than_shared_memory(gpu_device, n, walks):
+    """A mesh with too many vertices per SM takes the per-colour launches (here on a stream of 16 SMs)."""
+    import numpy as np
+    import torch
+
+    from vbd_tetmesh_b200 import _capi, build_solver, meshgen
+
+    driver = pytest.importorskip("cuda.bindings.driver")
+    torch.zeros(1, device="cuda")  # the primary context
+
+    def ok(r):
+        assert r[0] == driver.CUresult.CUDA_SUCCESS, r[0]
+        return r[1:] if len(r) > 2 else r[1] if len(r) == 2 else None
+
+    sms = ok(driver.cuDeviceGetDevResource(0, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups, _, _ = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, 16))
+    desc = ok(driver.cuDevResourceGenerateDesc(groups, 1))
+    ctx = ok(driver.cuGreenCtxCreate(desc, 0, driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(ctx, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    m = meshgen.cube(n)
+    out = []
+    for persistent in (None, 0):
+        s = build_solver(m, lanes=8, layout=4, stream=int(stream))
+        if persistent is not None:
+            s.set_option(_capi.OPT_PERSISTENT, persistent)
+        l0 = s.kernel_launches()
+        s.step(1 / 120, 3, (0.0, -9.8, 0.0), True, 0.9)
+        s.sync()
+        assert (s.kernel_launches() - l0 == 1) == (walks and persistent is None)
+        out.append((s.get_positions(), s.get_velocities()))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    ok(driver.cuStreamDestroy(stream))
+    ok(driver.cuGreenCtxDestroy(ctx))
+
+
 def test_a_stream_of_fewer_sms(gpu_device):
     """On a green context's stream the walk takes as many tiles as that context has SMs."""
     import numpy as np
