@@ -126,6 +126,33 @@ same(out[0], out[2])
 """)
 
 
+def test_a_wait_that_ran_out_is_reported_without_mapped_host_memory(gpu_device, run):
+    run("""
+m = meshgen.jittered_block(9, 6, 5, seed=3)
+register_error = ctypes.c_int.in_dll(fake, "fake_register_error")
+xs = []
+for refuse in (0, 2, 801):  # accepted, cudaErrorMemoryAllocation, cudaErrorNotSupported
+    register_error.value = refuse
+    s = build_solver(m, lanes=8, layout=4)
+    s.step(1 / 60, 5, G, True, 0.9)
+    s.sync()
+    out = ctypes.c_int32(0)
+    _capi.call("vbd_solver_walk_selftest", s._h, 5000, ctypes.byref(out))
+    assert out.value == 1
+    try:
+        s.get_velocities()
+        raise SystemExit("not reported")
+    except _capi.VBDError as e:
+        assert e.code == 6  # VBD_ERR_TIMEOUT
+    s.sync()
+    s.step(1 / 60, 5, G, True, 0.9)
+    xs.append([s.get_positions(), s.get_velocities()])
+    s.close()
+same(xs[0], xs[1])
+same(xs[0], xs[2])
+""")
+
+
 def test_walks_after_a_refused_launch_wait_as_long_as_before(gpu_device, run):
     """The count of started CTAs does not run ahead: a wait that runs out ends after its limit, not after the time
     that a CTA may take to start."""

@@ -31,12 +31,12 @@ static_assert(sizeof(TetRec) == 64, "TetRec must be 64 bytes");
 
 // ST_TIMEOUT: a grid barrier of the persistent kernel gave up; ST_WALK_TIMEOUT: an mbarrier wait
 // of a cluster walk gave up.
-// ST_HOST (after the slots that are reset) holds the address of a word in host memory, set with either of them:
-// the host sees after any synchronisation, without a copy, that a wait gave up.
+// ST_HOST (after the slots that are reset) holds the address of a word in host memory (or 0), set with either of
+// them: the host sees after any synchronisation, without a copy, that a wait gave up.
 enum StatusSlot { ST_SINGULAR = 0, ST_NONFINITE = 1, ST_TIMEOUT = 2, ST_WALK_TIMEOUT = 3, ST_SLOTS = 4, ST_HOST = 4 };
 __device__ __forceinline__ void note_timeout(unsigned long long* status, int slot) {
     atomicOr(reinterpret_cast<unsigned int*>(status + slot), 1u);
-    *reinterpret_cast<volatile unsigned int*>(status[ST_HOST]) = 1u;
+    if (status[ST_HOST]) *reinterpret_cast<volatile unsigned int*>(status[ST_HOST]) = 1u;
 }
 
 struct SweepParams {

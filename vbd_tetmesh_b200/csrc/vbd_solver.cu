@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <vector>
@@ -232,7 +233,10 @@ struct vbd_solver {
     vbd::DBuf<int> inc_vertex;                      // internal vertex of each incidence
     vbd::DBuf<float> stage, mat_stage;
     vbd::DBuf<unsigned long long> status;
-    unsigned* wait_flag = nullptr;  // host memory: set by a kernel whose wait gave up (vbd::ST_HOST)
+    // A page of host memory whose first word a kernel sets where its wait gave up (vbd::ST_HOST).  It is registered:
+    // that takes 0.45 ms, cudaHostAlloc 3 ms and more a handle.
+    unsigned* wait_flag = nullptr;
+    bool wait_mapped = false;  // else (it could not be registered) the record itself is read
     vbd::DBuf<double> partials, scalar;
     // defaults: 64-thread blocks, programmatic dependent launch and graphs; lanes, layout and
     // record prefetch are chosen at init from the mesh (below) until their options are set
@@ -367,7 +371,8 @@ struct vbd_solver {
     ~vbd_solver() {
         drop_graphs();
         for (cudaEvent_t e : ev_pool) cudaEventDestroy(e);
-        if (wait_flag) cudaFreeHost(wait_flag);
+        if (wait_mapped) cudaHostUnregister(wait_flag);
+        std::free(wait_flag);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
 
@@ -375,9 +380,13 @@ struct vbd_solver {
     // last report: positions, velocities and gradients computed since then are not to be used.
     int finish() {
         CUDA_TRY(cudaStreamSynchronize(stream));
-        if (!*reinterpret_cast<volatile unsigned*>(wait_flag)) return VBD_OK;
+        if (wait_mapped && !*reinterpret_cast<volatile unsigned*>(wait_flag)) return VBD_OK;
         unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
         CUDA_TRY(cudaMemcpyAsync(t, status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost, stream));
+        if (!wait_mapped) {
+            CUDA_TRY(cudaStreamSynchronize(stream));
+            if (!t[0] && !t[1]) return VBD_OK;
+        }
         CUDA_TRY(cudaMemsetAsync(status.p + vbd::ST_TIMEOUT, 0, sizeof(t), stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
         *wait_flag = 0;
@@ -1744,11 +1753,14 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
         VBD_FAIL(VBD_ERR_NO_DEVICE, "no CUDA device available");
     }
     if (device < 0 || device >= count) VBD_FAIL(VBD_ERR_NO_DEVICE, "device %d out of range (%d devices)", device, count);
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10 || prop.minor != 0)
-        VBD_FAIL(VBD_ERR_NO_DEVICE, "device %d is sm_%d%d; this library is built for sm_100a only", device,
-                 prop.major, prop.minor);
+    // single attributes: cudaGetDeviceProperties takes 2.5 ms
+    int major = 0, minor = 0, sms = 0, smem = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    CUDA_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    CUDA_TRY(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    if (major != 10 || minor != 0)
+        VBD_FAIL(VBD_ERR_NO_DEVICE, "device %d is sm_%d%d; this library is built for sm_100a only", device, major, minor);
     DeviceScope scope(device);
     std::unique_ptr<vbd_solver> s(new vbd_solver());
     s->device = device;
@@ -1758,13 +1770,17 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
         CUDA_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
         s->own_stream = true;
     }
-    s->sm_count = stream_sms(s->stream, prop.multiProcessorCount);
-    s->smem_optin = (int)prop.sharedMemPerBlockOptin;
+    s->sm_count = stream_sms(s->stream, sms);
+    s->smem_optin = smem;
     VBD_TRY(s->status.alloc(vbd::ST_HOST + 1));
-    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&s->wait_flag), sizeof(unsigned), cudaHostAllocMapped));
+    constexpr size_t kPage = 4096;
+    s->wait_flag = static_cast<unsigned*>(std::aligned_alloc(kPage, kPage));
+    if (!s->wait_flag) VBD_FAIL(VBD_ERR_ALLOC, "no host memory for a handle");
     *s->wait_flag = 0;
     void* flag = nullptr;
-    CUDA_TRY(cudaHostGetDevicePointer(&flag, s->wait_flag, 0));
+    s->wait_mapped = cudaHostRegister(s->wait_flag, kPage, cudaHostRegisterMapped) == cudaSuccess;
+    if (s->wait_mapped) CUDA_TRY(cudaHostGetDevicePointer(&flag, s->wait_flag, 0));
+    else (void)cudaGetLastError();
     const unsigned long long st[vbd::ST_HOST + 1] = {0, 0, 0, 0, reinterpret_cast<unsigned long long>(flag)};
     CUDA_TRY(cudaMemcpyAsync(s->status.p, st, sizeof(st), cudaMemcpyHostToDevice, s->stream));
     VBD_TRY(s->scalar.alloc(1));
