@@ -17,7 +17,6 @@ size_t fake_malloc_limit = ~(size_t)0;  // cudaMalloc of as many bytes or more f
 size_t fake_memory = 0;                 // bytes in use
 size_t fake_memory_limit = ~(size_t)0;  // cudaMalloc beyond it fails
 int fake_cooperative_error = 0;         // cudaLaunchCooperativeKernel returns this where it is not 0
-int fake_register_error = 0;            // cudaHostRegister returns this where it is not 0
 
 int cudaMalloc(void** p, size_t n) {
     static auto real = reinterpret_cast<int (*)(void**, size_t)>(runtime("cudaMalloc"));
@@ -37,12 +36,6 @@ int cudaFree(void* p) {
         sizes.erase(it);
     }
     return real(p);
-}
-
-int cudaHostRegister(void* p, size_t n, unsigned flags) {
-    if (fake_register_error) return fake_register_error;
-    static auto real = reinterpret_cast<int (*)(void*, size_t, unsigned)>(runtime("cudaHostRegister"));
-    return real(p, n, flags);
 }
 
 struct Dim {

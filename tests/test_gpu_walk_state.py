@@ -118,6 +118,18 @@ def test_a_wait_that_ran_out_is_reported_once(gpu_device, call):
     fresh.close()
 
 
+def test_a_wait_of_full_length_is_reported_between_reads(gpu_device):
+    """The record is not read after every step: a wait that gave up lasts longer than the time between two looks."""
+    s = build_solver(meshgen.jittered_block(7, 6, 5, seed=5))
+    s.get_positions()  # looks
+    assert give_up(s, 400000) == 1
+    with pytest.raises(_capi.VBDError) as e:
+        s.get_positions()
+    assert e.value.code == 6  # VBD_ERR_TIMEOUT
+    s.get_positions()
+    s.close()
+
+
 def test_the_barrier_selftest_leaves_a_walks_report(gpu_device):
     s = build_solver(meshgen.jittered_block(7, 6, 5, seed=5))
     assert give_up(s) == 1

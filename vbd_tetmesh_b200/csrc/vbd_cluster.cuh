@@ -114,7 +114,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigne
         }
     }
     done = __all_sync(0xffffffffu, done);
-    if (!done) note_timeout(status, ST_WALK_TIMEOUT);
+    if (!done) atomicOr(reinterpret_cast<unsigned int*>(status + ST_WALK_TIMEOUT), 1u);
     return done;
 }
 

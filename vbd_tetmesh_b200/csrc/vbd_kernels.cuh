@@ -29,15 +29,9 @@ struct __align__(16) TetRec {
 };
 static_assert(sizeof(TetRec) == 64, "TetRec must be 64 bytes");
 
-// ST_TIMEOUT: a grid barrier of the persistent kernel gave up; ST_WALK_TIMEOUT: an mbarrier wait
-// of a cluster walk gave up.
-// ST_HOST (after the slots that are reset) holds the address of a word in host memory (or 0), set with either of
-// them: the host sees after any synchronisation, without a copy, that a wait gave up.
-enum StatusSlot { ST_SINGULAR = 0, ST_NONFINITE = 1, ST_TIMEOUT = 2, ST_WALK_TIMEOUT = 3, ST_SLOTS = 4, ST_HOST = 4 };
-__device__ __forceinline__ void note_timeout(unsigned long long* status, int slot) {
-    atomicOr(reinterpret_cast<unsigned int*>(status + slot), 1u);
-    if (status[ST_HOST]) *reinterpret_cast<volatile unsigned int*>(status[ST_HOST]) = 1u;
-}
+// ST_TIMEOUT: a grid barrier of the persistent kernel gave up; ST_WALK_TIMEOUT: a wait of a cluster or tile
+// walk gave up.
+enum StatusSlot { ST_SINGULAR = 0, ST_NONFINITE = 1, ST_TIMEOUT = 2, ST_WALK_TIMEOUT = 3, ST_SLOTS = 4 };
 
 struct SweepParams {
     float4* x;                 // positions being swept in place (Gauss-Seidel)
@@ -1041,7 +1035,7 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier* bar, int expected, lon
             while (ld_acquire_gpu(&bar->gen) == gen) {
                 if (++polls > spin_limit) {
                     ok = 0;
-                    note_timeout(status, ST_TIMEOUT);
+                    atomicOr(reinterpret_cast<unsigned int*>(status + ST_TIMEOUT), 1u);
                     break;
                 }
                 __nanosleep(32);

@@ -4,8 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
-#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <vector>
@@ -233,10 +233,7 @@ struct vbd_solver {
     vbd::DBuf<int> inc_vertex;                      // internal vertex of each incidence
     vbd::DBuf<float> stage, mat_stage;
     vbd::DBuf<unsigned long long> status;
-    // A page of host memory whose first word a kernel sets where its wait gave up (vbd::ST_HOST).  It is registered:
-    // that takes 0.45 ms, cudaHostAlloc 3 ms and more a handle.
-    unsigned* wait_flag = nullptr;
-    bool wait_mapped = false;  // else (it could not be registered) the record itself is read
+    std::chrono::steady_clock::time_point looked_at{};  // when finish() last read the record of waits that gave up
     vbd::DBuf<double> partials, scalar;
     // defaults: 64-thread blocks, programmatic dependent launch and graphs; lanes, layout and
     // record prefetch are chosen at init from the mesh (below) until their options are set
@@ -371,25 +368,27 @@ struct vbd_solver {
     ~vbd_solver() {
         drop_graphs();
         for (cudaEvent_t e : ev_pool) cudaEventDestroy(e);
-        if (wait_mapped) cudaHostUnregister(wait_flag);
-        std::free(wait_flag);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
 
     // Waits for the work queued so far, and reports a wait of a walk or a grid barrier that gave up since the
-    // last report: positions, velocities and gradients computed since then are not to be used.
+    // last report: positions, velocities and gradients computed since then are not to be used.  The record is read
+    // where kLookAfter has passed since it was last read with the stream drained: a wait that gave up since then
+    // lasted longer (1 s in a cluster, 2 s for words, 2^22 loads from L2 at a barrier).  A read takes 10 us, which
+    // the reads after each 240 us step would pay twice; a word in pinned host memory that the kernel sets took
+    // 0.5 to 10 ms a handle.
+    static constexpr std::chrono::milliseconds kLookAfter{250};
     int finish() {
         CUDA_TRY(cudaStreamSynchronize(stream));
-        if (wait_mapped && !*reinterpret_cast<volatile unsigned*>(wait_flag)) return VBD_OK;
+        const auto now = std::chrono::steady_clock::now();
+        if (now - looked_at < kLookAfter) return VBD_OK;
         unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
         CUDA_TRY(cudaMemcpyAsync(t, status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost, stream));
-        if (!wait_mapped) {
-            CUDA_TRY(cudaStreamSynchronize(stream));
-            if (!t[0] && !t[1]) return VBD_OK;
-        }
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        looked_at = now;
+        if (!t[0] && !t[1]) return VBD_OK;
         CUDA_TRY(cudaMemsetAsync(status.p + vbd::ST_TIMEOUT, 0, sizeof(t), stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
-        *wait_flag = 0;
         if (t[0]) VBD_FAIL(VBD_ERR_TIMEOUT, "a grid barrier of the persistent kernel gave up waiting");
         VBD_FAIL(VBD_ERR_TIMEOUT, "a wait of the cluster or tile walk gave up");
     }
@@ -1304,7 +1303,7 @@ struct vbd_solver {
     // with VBD_GPU_Solver semantics, the predictor.
     int launch_tile(vbd::TileSet& s, int iters, float dtsr, bool accel, float rho, bool from_inertia, float h,
                     const float* hg, bool record_energy) {
-        VBD_TRY(upload_schedule(iters, accel, rho));
+        if (!s.cluster) VBD_TRY(upload_schedule(iters, accel, rho));  // launch_cluster has
         VBD_TRY(ensure_tile(s));
         if (s.wrapper && hg) {
             // every vertex starts from its inertial target, which a tile's ghosts need before the walk
@@ -1367,6 +1366,7 @@ struct vbd_solver {
         VBD_TRY(x.alloc(N));
         CUDA_TRY(cudaMemcpyAsync(list.p, groups.data(), sizeof(vbd::TileGroup) * groups.size(), cudaMemcpyHostToDevice, stream));
         CUDA_TRY(cudaMemcpyAsync(x.p, x0.p, sizeof(float4) * (size_t)N, cudaMemcpyDeviceToDevice, stream));
+        if (std::chrono::microseconds(wait_us) <= kLookAfter) looked_at = {};  // shorter than a real wait that gives up
         vbd::TileParams w;
         VBD_TRY(tile_params(s, 0, 3, 3600.0f, omega_at, false, 1, &w));
         w.groups = list.p;
@@ -1772,17 +1772,8 @@ int vbd_solver_create(vbd_solver** out, int device, void* cuda_stream) {
     }
     s->sm_count = stream_sms(s->stream, sms);
     s->smem_optin = smem;
-    VBD_TRY(s->status.alloc(vbd::ST_HOST + 1));
-    constexpr size_t kPage = 4096;
-    s->wait_flag = static_cast<unsigned*>(std::aligned_alloc(kPage, kPage));
-    if (!s->wait_flag) VBD_FAIL(VBD_ERR_ALLOC, "no host memory for a handle");
-    *s->wait_flag = 0;
-    void* flag = nullptr;
-    s->wait_mapped = cudaHostRegister(s->wait_flag, kPage, cudaHostRegisterMapped) == cudaSuccess;
-    if (s->wait_mapped) CUDA_TRY(cudaHostGetDevicePointer(&flag, s->wait_flag, 0));
-    else (void)cudaGetLastError();
-    const unsigned long long st[vbd::ST_HOST + 1] = {0, 0, 0, 0, reinterpret_cast<unsigned long long>(flag)};
-    CUDA_TRY(cudaMemcpyAsync(s->status.p, st, sizeof(st), cudaMemcpyHostToDevice, s->stream));
+    VBD_TRY(s->status.alloc(vbd::ST_SLOTS));
+    CUDA_TRY(cudaMemsetAsync(s->status.p, 0, sizeof(unsigned long long) * vbd::ST_SLOTS, s->stream));
     VBD_TRY(s->scalar.alloc(1));
     *out = s.release();
     return VBD_OK;
@@ -1843,7 +1834,6 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
 
     DeviceScope scope(s->device);
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    *s->wait_flag = 0;  // of the previous mesh
     s->ckpt_pool.clear();
     s->ready = false;
     s->drop_graphs();
@@ -2053,6 +2043,7 @@ int vbd_solver_init(vbd_solver* s, int32_t N, int32_t T, const float* positions,
     VBD_TRY(s->repack_stream());
     if (s->use_tile()) VBD_TRY(s->ensure_tile(s->walk_tiles()));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    s->looked_at = std::chrono::steady_clock::now();  // the record was cleared above
     s->ready = true;
     return s->prepare_cluster();
 }
@@ -2434,11 +2425,10 @@ int vbd_solver_barrier_selftest(vbd_solver* s, int64_t spin_limit, int32_t* time
     s->spin_limit = saved;
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    unsigned long long t[2] = {0, 0};  // ST_TIMEOUT, ST_WALK_TIMEOUT
-    CUDA_TRY(cudaMemcpy(t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t[0]), s->stream));
-    if (!t[1]) *s->wait_flag = 0;  // a walk's record stays for the call that reports it
-    *timed_out = t[0] ? 1 : 0;
+    unsigned long long t = 0;
+    CUDA_TRY(cudaMemcpy(&t, s->status.p + vbd::ST_TIMEOUT, sizeof(t), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemsetAsync(s->status.p + vbd::ST_TIMEOUT, 0, sizeof(t), s->stream));
+    *timed_out = t ? 1 : 0;
     return VBD_OK;
 }
 

@@ -1,5 +1,6 @@
-// The tile walk: all iterations of a sub-step (or of its adjoint solve) in ONE cooperative launch, for
-// meshes too large for one cluster's shared memory.
+// The tile walk: all iterations of a sub-step (or of its adjoint solve) in ONE launch: a cooperative one, the
+// default from kTileMinVertices free vertices until a tile no longer fits in an SM's shared memory, or one cluster
+// (VBD_OPT_PERSISTENT 2).
 //
 // Per-colour launches pay a kernel boundary per colour (2.3 us and up) and start each colour's
 // record stream only then.  Here the free vertices are cut into one spatial tile per CTA (one CTA per
@@ -24,8 +25,8 @@
 // What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
 // one SM to another's poll, 885 on average) plus one vertex's chain per colour (about 1,000 cycles from
 // the barrier to its publication): 1.3 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by
-// issue and the chunk stream: 64^3 cube 3.34 against 4.17 ms a step of 400 colours, 4.0 TB/s of DRAM
-// reads.  VBD_GPU_Solver semantics: 425-vertex beam 2.6 against 4.6 us a colour, 32^3 cube 6.6 against 9.6.
+// issue and the chunk stream: 64^3 cube 3.10 against 4.17 ms a step of 400 colours, 4.2 TB/s of DRAM
+// traffic.  VBD_GPU_Solver semantics: 425-vertex beam 2.6 against 4.6 us a colour, 32^3 cube 6.6 against 9.6.
 // Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
 // records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds
 // the sums of lanes t and t + L/2 (group_reduce's first addition), so a vertex takes L/2 threads:
@@ -134,7 +135,7 @@ __device__ __noinline__ bool tile_give_up(unsigned long long* status, unsigned l
         c.last = now;
         return false;
     }
-    note_timeout(status, ST_WALK_TIMEOUT);
+    atomicOr(reinterpret_cast<unsigned int*>(status + ST_WALK_TIMEOUT), 1u);
     return true;
 }
 
