@@ -160,6 +160,8 @@ struct TileSet {
     enum { HEAD, GROUPS, WCOL, WSTREAM, TABLE, LID, GHOST, VTILE, VLOCAL, TARGET_OFF, TARGET, COUNT };
     size_t at[COUNT + 1] = {};
     const int* ints(int which) const { return lists + at[which]; }
+    // after the words: the count of started CTAs, the limit of a wait
+    unsigned long long* arrived() const { return reinterpret_cast<unsigned long long*>(words + nwords - 1); }
     unsigned long long started = 0;  // CTAs of all launches so far
     unsigned tag = 1;                // next unused word tag
     int stride = 1;                  // of the exchanged words
@@ -1135,6 +1137,13 @@ struct vbd_solver {
         s.dirty = true;
     }
 
+    // After how many nanoseconds a wait of the set's walks gives up.
+    int set_wait_limit(vbd::TileSet& s, unsigned long long ns) {
+        CUDA_TRY(cudaMemcpyAsync(s.arrived() + 1, &ns, sizeof(ns), cudaMemcpyHostToDevice, stream));
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        return VBD_OK;
+    }
+
     // The plan's lists and the record chunks on the device, made when first needed for the current lanes, layout
     // and materials.
     int ensure_tile(vbd::TileSet& s) {
@@ -1173,7 +1182,10 @@ struct vbd_solver {
             s.chunk = s.words + s.nwords;
             s.lists = reinterpret_cast<int*>(s.chunk + nchunk);
             CUDA_TRY(cudaMemcpyAsync(s.lists, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, stream));
-            if (s.nwords) CUDA_TRY(cudaMemsetAsync(s.words, 0, sizeof(float4) * s.nwords, stream));
+            if (s.nwords) {
+                CUDA_TRY(cudaMemsetAsync(s.words, 0, sizeof(float4) * s.nwords, stream));
+                VBD_TRY(set_wait_limit(s, vbd::kTileWaitNs));
+            }
             s.started = 0;
             s.tag = 1;
             CUDA_TRY(cudaStreamSynchronize(stream));  // the host lists may change after this
@@ -1236,7 +1248,7 @@ struct vbd_solver {
             }
             w.words = s.words;
             w.word_stride = s.stride;
-            w.arrived = reinterpret_cast<unsigned long long*>(s.words + s.nwords - 1);
+            w.arrived = s.arrived();
             w.arrived_target = s.started + (unsigned)q.P;
             w.tag = s.tag - (unsigned)k0;
         }
@@ -1252,7 +1264,6 @@ struct vbd_solver {
         w.max_own = q.max_own;
         w.max_target = q.max_target;
         w.status = status.p;
-        w.wait_ns = vbd::kTileWaitNs;
         w.omega = omega;
         w.n = N;
         w.nfree = nfree;
@@ -1370,11 +1381,12 @@ struct vbd_solver {
         vbd::TileParams w;
         VBD_TRY(tile_params(s, 0, 3, 3600.0f, omega_at, false, 1, &w));
         w.groups = list.p;
-        w.wait_ns = 1000ull * (unsigned long long)wait_us;
         w.x0 = x.p;
         w.pp = pp.p;
+        VBD_TRY(set_wait_limit(s, 1000ull * (unsigned long long)wait_us));
         const int rc = tile_launch(
             s, s.wrapper ? vbd::pick_tile_wrapper(s.plan.warps) : vbd::pick_tile<vbd::kTileForward>(s.plan, false), w, 1);
+        VBD_TRY(set_wait_limit(s, vbd::kTileWaitNs));
         if (rc == vbd::kWalkRefused) VBD_FAIL(VBD_ERR_STATE, "the device refuses the walk's launch");
         VBD_TRY(rc);
         unsigned long long t = 0;

@@ -25,7 +25,7 @@
 // What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
 // one SM to another's poll, 885 on average) plus one vertex's chain per colour (about 1,000 cycles from
 // the barrier to its publication): 1.3 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by
-// issue and the chunk stream: 64^3 cube 3.10 against 4.17 ms a step of 400 colours, 4.2 TB/s of DRAM
+// issue and the chunk stream: 64^3 cube 3.15 against 4.17 ms a step of 400 colours, 4.2 TB/s of DRAM
 // traffic.  VBD_GPU_Solver semantics: 425-vertex beam 2.6 against 4.6 us a colour, 32^3 cube 6.6 against 9.6.
 // Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
 // records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds
@@ -52,10 +52,9 @@ struct TileParams {
     const int2* wstream;        // [P][warps]
     float4* words;              // exchanged words: [parity][n] x~, then [parity][n] blended, word_stride apart
     int word_stride;
-    unsigned long long* arrived;
+    unsigned long long* arrived;        // and after it the nanoseconds after which a wait gives up (kTileWaitNs)
     unsigned long long arrived_target;  // *arrived once every CTA of this launch has started
     unsigned long long* status;
-    unsigned long long wait_ns; // after which a wait gives up (kTileWaitNs)
     const float* omega;         // Chebyshev weight of each iteration (1 = no blend)
     unsigned tag;               // iteration k publishes tag + k; unused by any earlier launch
     int n, nfree, ncol, k0, k1; // iterations [k0, k1) of the schedule
@@ -115,7 +114,7 @@ __device__ __forceinline__ float4 word_load(const float4* p) {
                        __uint_as_float((unsigned)(b >> 32)));
 }
 
-// Gives up a wait: another wait already gave up, or this one has lasted wait_ns with every CTA of
+// Gives up a wait: another wait already gave up, or this one has lasted arrived[1] nanoseconds with every CTA of
 // the launch running (a CTA that cannot start while another program's kernel holds its SM is
 // waited for up to kTileStartNs).  The walk then sweeps on to the end of the iteration with what it has, so
 // that no thread leaves a barrier, a shuffle or a copy that the others wait for.
@@ -126,11 +125,11 @@ struct TileClock {
     unsigned long long first = 0, last = 0;
 };
 __device__ __noinline__ bool tile_give_up(unsigned long long* status, unsigned long long* arrived,
-                                          unsigned long long target, unsigned long long wait_ns, TileClock& c) {
+                                          unsigned long long target, TileClock& c) {
     if (*reinterpret_cast<volatile unsigned long long*>(status + ST_WALK_TIMEOUT) != 0ull) return true;
     const unsigned long long now = global_ns();
     if (c.first == 0) c.first = c.last = now;
-    if (now - c.last <= wait_ns) return false;
+    if (now - c.last <= arrived[1]) return false;
     if (*reinterpret_cast<volatile unsigned long long*>(arrived) < target && now - c.first <= kTileStartNs) {
         c.last = now;
         return false;
@@ -148,7 +147,7 @@ __device__ __forceinline__ bool tile_spin(const TileParams& p, const float4* w, 
             *dst = make_float4(v.x, v.y, v.z, 0.f);
             return true;
         }
-        if ((i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, p.wait_ns, clk)) return false;
+        if ((i & 255u) == 0u && tile_give_up(p.status, p.arrived, p.arrived_target, clk)) return false;
     }
 }
 // The same with a first look already taken.
@@ -226,17 +225,16 @@ __device__ __forceinline__ bool ring_test(unsigned bar, unsigned parity) {
 // own: inlined they cost the sweep loop registers (64^3 cube 3.15 ms a step of 50 iterations against 3.26, 128 meshes
 // 1.31 against 1.43, 32^3 1.07 against 1.09, VBD_GPU_Solver semantics 32^3 0.98 against 1.02 for 20).
 __device__ __noinline__ bool ring_wait_again(unsigned bar, unsigned parity, unsigned long long* status,
-                                             unsigned long long* arrived, unsigned long long target,
-                                             unsigned long long wait_ns) {
+                                             unsigned long long* arrived, unsigned long long target) {
     TileClock clk;
     for (unsigned i = 1;; ++i) {
         if (ring_try(bar, parity)) return true;
-        if ((i & 255u) == 0u && tile_give_up(status, arrived, target, wait_ns, clk)) return false;
+        if ((i & 255u) == 0u && tile_give_up(status, arrived, target, clk)) return false;
     }
 }
 __device__ __forceinline__ bool ring_wait_bulk(const TileParams& p, unsigned bar, unsigned parity) {
     bool done = ring_try(bar, parity);
-    if (!done) done = ring_wait_again(bar, parity, p.status, p.arrived, p.arrived_target, p.wait_ns);
+    if (!done) done = ring_wait_again(bar, parity, p.status, p.arrived, p.arrived_target);
     return __all_sync(0xffffffffu, done);
 }
 // Waits until at most `pending` of the newest commit groups are outstanding.
