@@ -13,9 +13,10 @@ E = 1e6 Pa, nu = 0.4, density 1000, bottom face pinned, seeded initial velocitie
 * e2e: the same metric through the C ABI with host buffers: each step uploads positions and
   velocities from pinned host memory, steps, and reads both back.
 * roofline: the colour sweeps (a tile walk runs a step's 400 in one launch; else 400 of its 402
-  launches): the algorithmic bytes of one (60 B per incident tet + 96 B per swept vertex) over the
-  timed region's CUDA-event time per sweep; a second pass with an event pair around every sweep launched on its own is reported
-  beside it as "isolated".
+  launches): the bytes of one over the timed region's CUDA-event time per sweep.  A tile walk is charged
+  what it moves (44 B per incident tet + 48 B per swept vertex), per-colour launches the algorithmic
+  60 B per incident tet + 96 B per swept vertex.  A second pass with an event pair around every sweep
+  launched on its own is reported beside it as "isolated".
 * cpu_baseline (rank 0, N = 1): the reference's own CPU sources (oracle/_ref, compiled against the
   Eigen-API subset) on all host cores, one cube iteration per sample; the oracle's reference-cost
   restatement (literal 12x12 element Hessian, energy every 10 iterations) when they are not built.
@@ -395,6 +396,14 @@ def bench_wrapper(mesh, local, stream):
     return out
 
 
+def walk_bytes(mesh):
+    """Bytes that one iteration of a tile walk moves between an SM and L2 or HBM: 44 B per incidence of a free
+    vertex, and per free vertex its inertial target and pre-sweep position in, the pre-sweep position out.
+    Neighbours come from shared memory; the border's exchanged words are not counted."""
+    free = mesh.fixed == 0
+    return 44.0 * int(free[mesh.tets].sum()) + 48.0 * int(free.sum())
+
+
 def bench_batched(args, rank, world, local, stream, dist, barrier):
     """The batched configuration: args.batch_meshes jittered blocks (dims U{4..24}^3, E log-uniform
     [1e4, 1e6], nu U[0.2, 0.45], one face pinned), dt 1/60, 20 iterations, Chebyshev 0.9.  One solver
@@ -477,10 +486,14 @@ def bench_batched(args, rank, world, local, stream, dist, barrier):
     allm = meshgen.concat(meshes)
     peak, peak_kind = measured_peaks()
     step_s = ms_b / K * 1e-3
+    tile = 0 < launches_b < sw_launches  # the steps ran as tile walks
+    iso_bytes = sw_bytes
+    if tile:
+        sw_bytes = iters * sum(walk_bytes(m) for m in sub)
     achieved = sw_bytes / step_s / 1e9 if sw_bytes else None
     roofline = {
         "bound": "hbm",
-        "kernel": "vbd::k_tile_walk (all colour sweeps of a step)" if 0 < launches_b < sw_launches
+        "kernel": "vbd::k_tile_walk (all colour sweeps of a step)" if tile
                   else "vbd::k_sweep (colour sweeps of all meshes, one launch per colour)",
         "achieved": achieved,
         "peak": peak,
@@ -491,10 +504,11 @@ def bench_batched(args, rank, world, local, stream, dist, barrier):
         "alg_bytes_per_vertex_iteration": sw_bytes / (b.num_verts * iters) if sw_bytes else None,
         "sweep_launches_per_step": int(sw_launches),
         "launch_us_in_timed_region": (ms_b / K * 1e3 / sw_launches) if sw_launches else None,
-        "how": "this rank's algorithmic sweep bytes of one step (60 B per incidence + 96 B per swept vertex) over "
-               "the timed region's device time per step; predictor and velocity kernels are charged to the sweeps",
+        "how": ("the bytes this rank's walk moves in one step (44 B per incidence + 48 B per swept vertex)" if tile else
+                "this rank's algorithmic sweep bytes of one step (60 B per incidence + 96 B per swept vertex)")
+               + " over the timed region's device time per step; predictor and velocity update are charged to the sweeps",
         "isolated": {
-            "achieved": sw_bytes / (sw_ms * 1e-3) / 1e9 if sw_ms else None,
+            "achieved": iso_bytes / (sw_ms * 1e-3) / 1e9 if sw_ms else None,
             "launch_us": sw_ms * 1e3 / sw_launches if sw_launches else None,
             "how": "one CUDA event pair around every sweep launched on its own (no graph, no PDL overlap)",
         },
@@ -644,6 +658,7 @@ def bench_adjoint(local, stream, autotune=True):
     adj_sweep = 68.0 * inc_free + 128.0 * nfree
     alg = recomputed * st["iterations"] * fwd_iter + st["steps"] * st["adjoint_iterations"] * adj_sweep
     peak, peak_kind = measured_peaks()
+    resident = walks or persistent == 2  # the walks keep these records in shared memory and read them once a launch
     return {
         "workload": "32x8x8 beam x 6 tets (2,673 vertices, 12,288 tets), per-tet log-normal mu/lambda (sigma 0.2), "
                     "30 steps x 30 iterations, Chebyshev 0.95, checkpoint every 10 steps, loss on 25 tip vertices",
@@ -658,14 +673,14 @@ def bench_adjoint(local, stream, autotune=True):
         "accuracy": "checked in tests/test_gpu_adjoint.py: <= 1e-3 relative vs the FP64 implicit adjoint",
         "roofline": {
             "bound": "latency: 2,673 vertices give under 1% of the GPU's resident threads work",
-            "achieved": alg / tb / 1e9,
+            "achieved": None if resident else alg / tb / 1e9,
             "peak": peak,
             "peak_source": peak_kind,
             "unit": "GB/s",
-            "frac": alg / tb / 1e9 / peak,
+            "frac": None if resident else alg / tb / 1e9 / peak,
             "alg_bytes_backward": alg,
             "how": "algorithmic bytes of the backward (recomputed forward sweeps + adjoint sweeps) over its wall "
-                   "time around the C-ABI call (uploads and read-backs included)",
+                   "time around the C-ABI call (uploads and read-backs included); none for a walk, which does not move them",
         },
     }
 
@@ -863,17 +878,20 @@ def main():
     # one event pair around every sweep launched on its own (no graph, no PDL overlap), is reported
     # beside it as "isolated".
     achieved = iso_achieved = launch_us = None
+    tile = 0 < launches < sweep_launches  # the steps ran as tile walks: one launch each
+    iso_bytes = sweep_bytes
+    if tile:
+        sweep_bytes = walk_bytes(mesh) * iters * args.steps
     if sweep_launches and sweep_ms > 0:
         bytes_per_launch = sweep_bytes / sweep_launches
         launch_us = ms_max * 1e3 / sweep_launches
         achieved = bytes_per_launch / (launch_us * 1e-6) / 1e9
-        iso_achieved = sweep_bytes / (sweep_ms * 1e-3) / 1e9
-    # DRAM traffic per launch: the ncu-measured traffic / algorithmic-bytes ratio of the sweep
-    # kernel (profiles/sweep_cube64_dram.txt) times this run's algorithmic bytes per launch
+        iso_achieved = iso_bytes / (sweep_ms * 1e-3) / 1e9
+    # DRAM traffic per sweep: the ncu-measured ratio of DRAM bytes to the bytes charged to the kernel
+    # (profiles/) times this run's bytes per sweep
     traffic = None
-    prof = os.path.join(ROOT, "profiles", "sweep_cube64_dram.txt")
-    tile = 0 < launches < sweep_launches  # the steps ran as tile walks: one launch each
-    if os.path.exists(prof) and sweep_launches and not tile:
+    prof = os.path.join(ROOT, "profiles", "tile_walk_cube64.md" if tile else "sweep_cube64_dram.txt")
+    if os.path.exists(prof) and sweep_launches:
         for line in open(prof):
             if line.startswith("dram_traffic_over_algorithmic"):
                 traffic = float(line.split("=")[1].split()[0]) * sweep_bytes / sweep_launches
