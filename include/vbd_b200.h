@@ -306,9 +306,11 @@ int vbd_solver_status(vbd_solver* s, int64_t* singular_skips, int32_t* nonfinite
  *                        instead where these apply: one cooperative launch, the free vertices cut into
  *                        one spatial tile per SM that exchanges its border with its neighbours through
  *                        L2 after each colour (factored records, 4, 8 or 16 lanes for every colour,
- *                        VBD_OPT_GRAPH on, no kernel timing, the handle's stream not capturing, the
- *                        tile's vertices within shared memory).  Same results as the graph; reads
- *                        back as 0; VBD_ERR_TIMEOUT (vbd_solver_sync) if a bounded wait gave up;
+ *                        VBD_OPT_GRAPH on, no kernel timing, the handle's stream not capturing, a
+ *                        tile's vertices within shared memory, the launch accepted by the device).  On 148
+ *                        SMs a grid of 525,000 free vertices fits, one of 607,000 does not.  Same results
+ *                        as the graph; reads back as 0; VBD_ERR_TIMEOUT (vbd_solver_sync) if a bounded
+ *                        wait gave up;
  *                        1 = run each step / solve as one cooperative launch that walks the colours
  *                        with a grid barrier after each one (bounded wait: a barrier that gives up
  *                        makes the next call that reports it return VBD_ERR_TIMEOUT);

@@ -19,8 +19,8 @@ constexpr int kTileMaxRing = 6;             // chunks a warp's ring holds at mos
 constexpr int kTileMaxLocal = 65535;        // local vertex ids are 16 bits
 // A mesh gets a plan from this many free vertices.  Microseconds per colour of a step, tile walk against
 // captured graph (cubes of n^3 cells, one B200): n = 6 (294 free vertices) 1.29 / 2.33, 12 1.51 / 2.50, 16
-// 1.51 / 2.57, 24 1.84 / 3.31, 32 2.73 / 3.53, 48 4.57 / 5.5, 64 8.07 / 10.2.  Below it a few vertices per
-// tile would only exchange words.
+// 1.51 / 2.57, 24 1.84 / 3.31, 32 2.73 / 3.53, 48 4.57 / 5.5, 64 7.9 / 10.2.  Smaller meshes were not
+// measured: the line lies below the smallest that was, not where the gain ends.
 constexpr int kTileMinVertices = 256;
 // Free vertices per tile at least, up to one tile per SM.  32, 64 and 128 measured 0.81, 0.81 and 0.86 ms a
 // step on the 12^3 to 16^3 cubes: a colour lasts one exchange and one vertex's chain either way.
