@@ -25,7 +25,7 @@
 // What bounds it (one B200): small tiles by one exchange through L2 (a word takes 480 to 1,050 cycles from
 // one SM to another's poll, 885 on average) plus one vertex's chain per colour (about 1,000 cycles from
 // the barrier to its publication): 1.3 to 1.8 us a colour against 2.3 to 3.3 us a launch.  Large tiles by
-// issue and the chunk stream: 64^3 cube 3.15 against 4.17 ms a step of 400 colours, 4.2 TB/s of DRAM
+// issue and the chunk stream: 64^3 cube 3.15 against 4.17 ms a step of 400 colours, 4.1 TB/s of DRAM
 // traffic.  VBD_GPU_Solver semantics: 425-vertex beam 2.6 against 4.6 us a colour, 32^3 cube 6.6 against 9.6.
 // Same bits as the per-colour launches at the same lane count L: the partial sum of lane l takes
 // records l, l + L, ... in order, and lanes are added in the order of group_reduce.  A thread holds
@@ -222,8 +222,9 @@ __device__ __forceinline__ bool ring_test(unsigned bar, unsigned parity) {
     return ok != 0;
 }
 // Waits for a slot's chunk; the same answer for the whole warp.  The repeated tries stand in a function of their
-// own: inlined they cost the sweep loop registers (64^3 cube 3.15 ms a step of 50 iterations against 3.26, 128 meshes
-// 1.31 against 1.43, 32^3 1.07 against 1.09, VBD_GPU_Solver semantics 32^3 0.98 against 1.02 for 20).
+// own: inlined they cost the sweep loop registers (a step of 50 iterations of the 64^3 cube 2.98 ms against 3.17 with 4
+// lanes, 3.10 against 3.27 with 8; 128 meshes 1.36 against 1.44, 32^3 1.12 against 1.14, VBD_GPU_Solver semantics 32^3
+// 2.56 against 2.66).
 __device__ __noinline__ bool ring_wait_again(unsigned bar, unsigned parity, unsigned long long* status,
                                              unsigned long long* arrived, unsigned long long target) {
     TileClock clk;
